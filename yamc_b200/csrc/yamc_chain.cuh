@@ -25,9 +25,6 @@
 #ifndef YAMC_WIDE_THREADS
 #define YAMC_WIDE_THREADS 384  // threads of the wide streamed variant (up to 170 registers each)
 #endif
-#ifndef YAMC_KSPACE_UNROLL
-#define YAMC_KSPACE_UNROLL 1  // streamed k entries handled per loop iteration
-#endif
 
 namespace yamc {
 
@@ -92,7 +89,7 @@ struct Slot { double x, y, z, q, iq, dhs; int type, pad; };
 constexpr int kMaxSpecies = 8;
 constexpr int kCPT = 8;   // atoms each worker thread tests per filter round
 constexpr int kBlk = 32;  // atoms per bounding box of the pair filter (one warp's candidates per round and c)
-constexpr int kQueueMax = 4096;  // pair-queue chunk (items); a round's pairs are consumed in chunks
+constexpr int kQueueMax = 2560;  // pair-queue chunk (items); a round's pairs are consumed in chunks
 constexpr int kWin = 256; // random-stream window held in shared memory
 constexpr int kCtl = 32;  // threads of the control warp
 constexpr int kChainMaxThreads = 256;  // one CTA per SM, up to 255 registers per thread
@@ -245,6 +242,7 @@ struct Cand {
 struct ChainShared {
     Cand cand[4];         // the move being evaluated (cand[icur]) and up to three prepared next moves
     int icur;             // buffer of the move being evaluated
+    int imoved;           // buffer of the move just decided (its commit)
     int spec[3];          // buffers of the candidates: after an overlap / after a draw / accepted same molecule
     int abort, accepted, overlap, last_mol, spec_ok;
     long long cursor;     // stream position after the last completed move
@@ -316,6 +314,12 @@ template <> __device__ __forceinline__ double2 cvt2<double2>(double2 v) { return
 template <> __device__ __forceinline__ float2 cvt2<float2>(double2 v) { return make_float2((float)v.x, (float)v.y); }
 template <class R2> __device__ __forceinline__ R2 cvt2(float2 v);  // (FP32 rho copies: the mixed form only)
 template <> __device__ __forceinline__ float2 cvt2<float2>(float2 v) { return v; }
+// a product rounded on its own (never fused into a following sum)
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+// a or b as values (a conditional over array elements selects their addresses, which would keep
+// the array in local memory)
+template <class T> __device__ __forceinline__ T pick(bool c, T a, T b) { return c ? a : b; }
 __device__ __forceinline__ double2 to_d2(double2 v) { return v; }
 __device__ __forceinline__ double2 to_d2(float2 v) { return make_double2((double)v.x, (double)v.y); }
 
@@ -341,6 +345,7 @@ struct Acc {
     __device__ __forceinline__ void add_plain(int i, double x) { v[i] += x; }
     __device__ __forceinline__ void flag(int i) { v[i] = 1.0; }
     __device__ __forceinline__ double get(int i) const { return v[i]; }
+    __device__ __forceinline__ double kpart(int i) const { return v[i]; }
 };
 template <int N>
 struct Acc<true, N> {
@@ -362,9 +367,8 @@ struct Acc<true, N> {
     __device__ __forceinline__ void add_plain(int i, float x) { s[i] += x; }
     __device__ __forceinline__ void flag(int i) { d[i] = 1.0; }
     __device__ __forceinline__ double get(int i) const { return d[i] + ((double)s[i] + (double)c[i]); }
-    // the FP32 part alone, and its clearing (the k-space sums are reduced before the real space)
+    // the FP32 part alone (the k-space sums are reduced before the real space)
     __device__ __forceinline__ double kpart(int i) const { return (double)s[i] + (double)c[i]; }
-    __device__ __forceinline__ void clear_kpart(int i) { s[i] = 0.f; c[i] = 0.f; }
 };
 
 template <int NT, int EPT, bool MX = false>
@@ -387,13 +391,16 @@ struct EntryRegs {
 template <int NT, int EPT, bool MX = false>
 using RegsOf = EntryRegs<NT, (EPT > 0 ? EPT : 1), MX>;
 
-// The per-move phase tables of the molecule's slots, T[slot][axis][m] = (cos, sin)(2 pi m u),
-// and tmask: the LJ types the moving molecule carries.
+// The per-move phase tables of the molecule's slots, T[axis][m][slot] = (cos, sin)(2 pi m u): an
+// entry's thread forms one address per axis and reaches every slot at a fixed offset from it.  A
+// row holds kTabRow slots, one more than the molecule's at most 2 kMaxA, so the rows of consecutive
+// m fall into different banks (9 x 8 B or 9 x 16 B apart) for the lanes of a warp, which take
+// consecutive kz.
+constexpr int kTabRow = 2 * kMaxA + 1;
 template <bool MX>
 struct PhaseTabs {
     const typename Prec<MX>::R2 *T;
     int KM;
-    int tmask;
 };
 
 // Phase tables of slots [s0, s1) of move m, by the workers.  The FP32 form reduces 2 k u
@@ -415,79 +422,142 @@ __device__ __forceinline__ void build_tables(typename Prec<MX>::R2 *tab, const S
             sincospi(2.0 * (double)k * u, &s, &c);
         }
         if (k == 0) { s = R(0); c = R(1); }
-        tab[(sl * 3 + d) * KM + k] = mk2(c, s);
+        tab[(d * KM + k) * kTabRow + sl] = mk2(c, s);
     }
 }
+
+// What the k-space sweep reads of the moving molecule, in registers: read from the slots once per
+// pass.  (Read per entry they cost a shared load, an FP64 compare and an FP64-to-FP32 conversion
+// per atom and entry: the sweep's stores keep the compiler from hoisting them.)
+// `simple`: three charged atoms with LJ on the first only (rigid 3-site water): the sweep then
+// holds one LJ row per entry instead of one per LJ type, and runs without branches on the atoms.
+template <bool MX>
+struct MolK {
+    using R = typename Prec<MX>::R;
+    R q[kMaxA], iq[kMaxA];
+    int type[kMaxA];  // LJ type (0 = none)
+    int na, cmask;    // atoms; bit a: atom a is charged
+    int tmask;        // bit t: the molecule carries LJ type t + 1
+    bool simple;
+    __device__ __forceinline__ explicit MolK(const Slot *slots, int n) : na(n), cmask(0), tmask(0) {
+#pragma unroll
+        for (int a = 0; a < kMaxA; ++a) {
+            q[a] = R(0); iq[a] = R(0); type[a] = 0;
+            if (a < n) {
+                q[a] = (R)slots[a].q; iq[a] = (R)slots[a].iq; type[a] = slots[a].type;
+                if (slots[a].q != 0.0) cmask |= 1 << a;
+                if (type[a] > 0) tmask |= 1 << (type[a] - 1);
+            }
+        }
+        simple = n == 3 && cmask == 7 && type[0] > 0 && type[1] == 0 && type[2] == 0;
+    }
+};
+
+// q (cos, sin)(2 pi (x kx + y ky + z kz)) of one slot (entry_phase's arithmetic) from the slot's
+// elements X, Y, Z of the entry's three table rows
+template <class R, class R2>
+__device__ __forceinline__ void slot_phase(R2 X, R2 Y, R2 Z, bool yneg, bool zneg, R q, R &c, R &s) {
+    const R cx = X.x, sx = X.y, cy = Y.x, sy = yneg ? -Y.y : Y.y, cz = Z.x, sz = zneg ? -Z.y : Z.y;
+    const R qcc = q * cx * cy, qss = q * sx * sy, qsc = q * sx * cy, qcs = q * cx * sy;
+    const R qc = qcc - qss, qs = qsc + qcs;
+    const R c1 = qc * cz, s1 = qs * sz, s2 = qs * cz, c2 = qc * sz;
+    c = c1 - s1;
+    s = s2 + c2;
+}
+
+// one entry's three table rows and signs
+template <bool MX>
+struct EntryRows {
+    const typename Prec<MX>::R2 *tx, *ty, *tz;
+    bool yneg, zneg;
+    __device__ __forceinline__ EntryRows(const PhaseTabs<MX> &pt, int kx, int ky, int kz)
+        : tx(pt.T + kx * kTabRow), ty(pt.T + (pt.KM + (ky < 0 ? -ky : ky)) * kTabRow),
+          tz(pt.T + (2 * pt.KM + (kz < 0 ? -kz : kz)) * kTabRow), yneg(ky < 0), zneg(kz < 0) {}
+};
 
 // Molecule phase sums of one entry over slots [s0, s0+na) -- RhoSquared_addAtom per atom:
 // Coulomb phase q (cos, sin), LJ phase = Coulomb phase * (1/q) (the unit phase when q == 0),
 // accumulated per LJ type in atom order.  ph/phl keep the per-atom phases for the forces.
 template <int NT, bool MX>
-__device__ __forceinline__ void mol_phase_sum(const PhaseTabs<MX> &pt, const Slot *slots, int s0, int na, int kx, int ky,
-                                              int kz, typename Prec<MX>::R2 (&out)[1 + NT],
+__device__ __forceinline__ void mol_phase_sum(const EntryRows<MX> &er, const MolK<MX> &mk, int s0,
+                                              typename Prec<MX>::R2 (&out)[1 + NT],
                                               typename Prec<MX>::R2 (&ph)[kMaxA], typename Prec<MX>::R2 (&phl)[kMaxA]) {
     using R = typename Prec<MX>::R;
     using R2 = typename Prec<MX>::R2;
-    const int KM = pt.KM;
 #pragma unroll
     for (int t = 0; t <= NT; ++t) out[t] = mk2(R(0), R(0));
 #pragma unroll
     for (int a = 0; a < kMaxA; ++a) {
         ph[a] = mk2(R(0), R(0));
         phl[a] = mk2(R(0), R(0));
-        if (a < na) {
-            const Slot &sl = slots[s0 + a];
-            const R2 *T = pt.T + (size_t)(s0 + a) * 3 * KM;
-            const R q = (R)sl.q;
+        if (a < mk.na) {
+            const R2 X = er.tx[s0 + a], Y = er.ty[s0 + a], Z = er.tz[s0 + a];
+            const bool charged = (mk.cmask >> a) & 1;
             R c = 0, s = 0;
-            if (sl.q != 0.0) {
-                entry_phase<R, R2>(T, T + KM, T + 2 * KM, kx, ky, kz, q, c, s);
+            if (charged) {
+                slot_phase<R, R2>(X, Y, Z, er.yneg, er.zneg, mk.q[a], c, s);
                 out[0].x = out[0].x + c; out[0].y = out[0].y + s;
             }
             ph[a] = mk2(c, s);
-            if (sl.type > 0) {
-                R cl, sl2;
-                if (sl.q != 0.0) { const R iq = (R)sl.iq; cl = c * iq; sl2 = s * iq; }
-                else entry_phase<R, R2>(T, T + KM, T + 2 * KM, kx, ky, kz, R(1), cl, sl2);
+            if (mk.type[a] > 0) {
+                R cl, sl;
+                if (charged) { cl = c * mk.iq[a]; sl = s * mk.iq[a]; }
+                else slot_phase<R, R2>(X, Y, Z, er.yneg, er.zneg, R(1), cl, sl);
 #pragma unroll
-                for (int t = 0; t < NT; ++t)
-                    if (t == sl.type - 1) { out[1 + t].x = out[1 + t].x + cl; out[1 + t].y = out[1 + t].y + sl2; }
-                phl[a] = mk2(cl, sl2);
+                for (int t = 0; t < NT; ++t) {  // (selects of values: an indexed or conditional store would put out in local memory)
+                    const bool hit = t == mk.type[a] - 1;
+                    out[1 + t].x = pick<R>(hit, out[1 + t].x + cl, out[1 + t].x);
+                    out[1 + t].y = pick<R>(hit, out[1 + t].y + sl, out[1 + t].y);
+                }
+                phl[a] = mk2(cl, sl);
             }
         }
     }
 }
 
-// k-space force on the molecule's atoms from one entry: 4 pi beta (C sin - S cos) k per atom,
-// Coulomb with the q-weighted phase, plus the dispersion terms of the atom's LJ type against
-// every type's structure factor (ForceKSpace.f90:59-302).
+// element (t0, t) of an entry's beta_LJ row set, t0 known at run time (selects of values)
+template <int NT, class R>
+__device__ __forceinline__ R beta_lj_of(const R (&bl)[NPair<NT>::value], int t0, int t) {
+    R b = bl[pair_idx<NT>(0, t)];
+#pragma unroll
+    for (int u = 1; u < NT; ++u) {
+        b = pick<R>(t0 == u, bl[pair_idx<NT>(u, t)], b);
+    }
+    return b;
+}
+
+// k-space force on one atom from one entry: 4 pi beta (C sin - S cos) k, Coulomb with the
+// q-weighted phase (ForceKSpace.f90:59-302); w also holds the dispersion terms where there are any
+template <class R, class AccT>
+__device__ __forceinline__ void add_force(int a, R w, int kx, int ky, int kz, AccT &acc) {
+    acc.add_plain(RV_F + 3 * a, w * (R)kx);
+    acc.add_plain(RV_F + 3 * a + 1, w * (R)ky);
+    acc.add_plain(RV_F + 3 * a + 2, w * (R)kz);
+}
+
+// k-space force on the molecule's atoms from one entry, plus the dispersion terms of the atom's
+// LJ type against every type's structure factor.
 template <int NT, bool MX, class AccT>
-__device__ __forceinline__ void entry_forces(const Slot *slots, int s0, int na, int kx, int ky, int kz,
+__device__ __forceinline__ void entry_forces(const MolK<MX> &mk, int kx, int ky, int kz,
                                              typename Prec<MX>::R beta,
                                              const typename Prec<MX>::R (&bl)[NPair<NT>::value],
                                              const typename Prec<MX>::R2 (&C)[1 + NT],
                                              const typename Prec<MX>::R2 (&ph)[kMaxA],
-                                             const typename Prec<MX>::R2 (&phl)[kMaxA], AccT &acc, int f0 = RV_F) {
+                                             const typename Prec<MX>::R2 (&phl)[kMaxA], AccT &acc) {
     using R = typename Prec<MX>::R;
     const R fourpi = (R)kFourPi;
 #pragma unroll
     for (int a = 0; a < kMaxA; ++a) {
-        if (a < na) {
-            const int ta = slots[s0 + a].type;
-            R w = fourpi * ((C[0].x * ph[a].y - C[0].y * ph[a].x) * beta);
-            if (ta > 0) {
+        if (a < mk.na) {
+            R w = mul_rn(fourpi, (C[0].x * ph[a].y - C[0].y * ph[a].x) * beta);
+            if (mk.type[a] > 0) {
 #pragma unroll
                 for (int t = 0; t < NT; ++t) {
-                    R b = R(0);
-#pragma unroll
-                    for (int u = 0; u < NT; ++u)
-                        if (u == ta - 1) b = bl[pair_idx<NT>(u, t)];
+                    const R b = beta_lj_of<NT, R>(bl, mk.type[a] - 1, t);
                     w += fourpi * ((C[1 + t].x * phl[a].y - C[1 + t].y * phl[a].x) * b);
                 }
             }
-            acc.add_plain(f0 + 3 * a, w * (R)kx);
-            acc.add_plain(f0 + 3 * a + 1, w * (R)ky);
-            acc.add_plain(f0 + 3 * a + 2, w * (R)kz);
+            add_force(a, w, kx, ky, kz, acc);
         }
     }
 }
@@ -495,23 +565,24 @@ __device__ __forceinline__ void entry_forces(const Slot *slots, int s0, int na, 
 // One signed entry of a pass: the molecule's phase sums at the old positions (into mold) and/or
 // the new ones, the delta (into dl), dU_k Coulomb + LJ against rho, and the k-space forces.
 template <int NT, int KIND, bool FORCES, bool MX, class AccT, class RhoT>
-__device__ __forceinline__ void kspace_entry(const PhaseTabs<MX> &pt, const Slot *slots, int na, int kx,
+__device__ __forceinline__ void kspace_entry(const PhaseTabs<MX> &pt, const MolK<MX> &mk, int kx,
                                              int ky, int kz, typename Prec<MX>::R beta,
                                              const typename Prec<MX>::R (&bl)[NPair<NT>::value],
                                              const RhoT (&rho)[1 + NT], typename Prec<MX>::R2 (&mold)[1 + NT],
                                              typename Prec<MX>::R2 (&dl)[1 + NT], AccT &acc) {
     using R = typename Prec<MX>::R;
     using R2 = typename Prec<MX>::R2;
+    const EntryRows<MX> er(pt, kx, ky, kz);
     R2 ph[kMaxA], phl[kMaxA];
     R2 C[1 + NT];
 #pragma unroll
     for (int t = 0; t <= NT; ++t) C[t] = cvt2<R2>(rho[t]);
-    if constexpr (KIND != PASS_NEW) mol_phase_sum<NT, MX>(pt, slots, na, na, kx, ky, kz, mold, ph, phl);
+    if constexpr (KIND != PASS_NEW) mol_phase_sum<NT, MX>(er, mk, mk.na, mold, ph, phl);
     if constexpr (KIND == PASS_OLD) {
-        if constexpr (FORCES) entry_forces<NT, MX>(slots, na, na, kx, ky, kz, beta, bl, C, ph, phl, acc);
+        if constexpr (FORCES) entry_forces<NT, MX>(mk, kx, ky, kz, beta, bl, C, ph, phl, acc);
     } else {
         R2 mnew[1 + NT];
-        mol_phase_sum<NT, MX>(pt, slots, 0, na, kx, ky, kz, mnew, ph, phl);
+        mol_phase_sum<NT, MX>(er, mk, 0, mnew, ph, phl);
 #pragma unroll
         for (int t = 0; t <= NT; ++t) dl[t] = mk2(mnew[t].x - mold[t].x, mnew[t].y - mold[t].y);
         {   // EwaldSumKSpace_calc_dU_coulomb (EwaldSumKSpace.f90:528-620)
@@ -528,9 +599,9 @@ __device__ __forceinline__ void kspace_entry(const PhaseTabs<MX> &pt, const Slot
             const R tc = (C1.x + C1.x) + D1.x, ts = (C1.y + C1.y) + D1.y;
 #pragma unroll
             for (int t2 = 0; t2 < NT; ++t2) {
-                if (!((pt.tmask >> t2) & 1)) continue;
                 const R2 D2 = dl[1 + t2];
-                dul += (tc * D2.x + ts * D2.y) * bl[pair_idx<NT>(t1, t2)];
+                const R u = dul + (tc * D2.x + ts * D2.y) * bl[pair_idx<NT>(t1, t2)];
+                dul = pick<R>((mk.tmask >> t2) & 1, u, dul);
             }
         }
         acc.add(RV_DUL, dul);
@@ -538,110 +609,220 @@ __device__ __forceinline__ void kspace_entry(const PhaseTabs<MX> &pt, const Slot
             R2 Cn[1 + NT];
 #pragma unroll
             for (int t = 0; t <= NT; ++t) Cn[t] = mk2(C[t].x + dl[t].x, C[t].y + dl[t].y);
-            entry_forces<NT, MX>(slots, 0, na, kx, ky, kz, beta, bl, Cn, ph, phl, acc);
+            entry_forces<NT, MX>(mk, kx, ky, kz, beta, bl, Cn, ph, phl, acc);
         }
     }
 }
 
-// The k-space sweep of one pass over the worker's entries (kspace_entry per entry).
-// Registers layout: k, beta, beta_LJ and rho stay in registers (R); the old phase sums are R.mold
-// (or read from mold_in when given), the delta R.dl.  Streamed layout: every entry is read from
-// memory (L2-resident), the next entry's loads in flight while the current one computes; the old
-// sums come from mold_in (PASS_NEW, PASS_BOTH's are computed), the delta goes to the chain's
-// scratch.  PASS_OLD stores its phase sums to mold_out (registers layout: when mold_store).
-template <int NT, int EPT, int KIND, bool FORCES, bool MX, class AccT>
+// The same entry for a `simple` molecule (MolK): the same terms in the same order, with the one LJ
+// row (type t0 + 1) that its delta has; mold / dl: row 0 Coulomb, row 1 that LJ row; b[t]: beta_LJ
+// of the pair (t0, t).
+template <int NT, int KIND, bool FORCES, bool MX, class AccT, class RhoT>
+__device__ __forceinline__ void kspace_entry_simple(const PhaseTabs<MX> &pt, const MolK<MX> &mk, int kx, int ky, int kz,
+                                                    typename Prec<MX>::R beta, const typename Prec<MX>::R (&b)[NT],
+                                                    const RhoT (&rho)[1 + NT], typename Prec<MX>::R2 &mold0,
+                                                    typename Prec<MX>::R2 &mold1, typename Prec<MX>::R2 &dl0,
+                                                    typename Prec<MX>::R2 &dl1, AccT &acc) {
+    using R = typename Prec<MX>::R;
+    using R2 = typename Prec<MX>::R2;
+    constexpr int NA = 3;
+    const EntryRows<MX> er(pt, kx, ky, kz);
+    const int t0 = mk.type[0] - 1;
+    const R fourpi = (R)kFourPi;
+    R2 C[1 + NT];
+#pragma unroll
+    for (int t = 0; t <= NT; ++t) C[t] = cvt2<R2>(rho[t]);
+    R2 ph[NA], phl;
+    auto phases = [&](int s0, R2 &sum0, R2 &sum1) {
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            R c, s;
+            slot_phase<R, R2>(er.tx[s0 + a], er.ty[s0 + a], er.tz[s0 + a], er.yneg, er.zneg, mk.q[a], c, s);
+            sum0 = a == 0 ? mk2(c, s) : mk2(sum0.x + c, sum0.y + s);
+            ph[a] = mk2(c, s);
+        }
+        phl = mk2(mul_rn(ph[0].x, mk.iq[0]), mul_rn(ph[0].y, mk.iq[0]));
+        sum1 = phl;
+    };
+    auto forces = [&](const R2 (&F)[1 + NT]) {
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            R w = mul_rn(fourpi, (F[0].x * ph[a].y - F[0].y * ph[a].x) * beta);
+            if (a == 0) {
+#pragma unroll
+                for (int t = 0; t < NT; ++t) w += fourpi * ((F[1 + t].x * phl.y - F[1 + t].y * phl.x) * b[t]);
+            }
+            add_force(a, w, kx, ky, kz, acc);
+        }
+    };
+    if constexpr (KIND != PASS_NEW) phases(NA, mold0, mold1);
+    if constexpr (KIND == PASS_OLD) {
+        if constexpr (FORCES) forces(C);
+    } else {
+        R2 n0, n1;
+        phases(0, n0, n1);
+        dl0 = mk2(n0.x - mold0.x, n0.y - mold0.y);
+        dl1 = mk2(n1.x - mold1.x, n1.y - mold1.y);
+        acc.add(RV_DUC, (((C[0].x + C[0].x) + dl0.x) * dl0.x + ((C[0].y + C[0].y) + dl0.y) * dl0.y) * beta);
+        R dul = R(0);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const R dx = t == t0 ? dl1.x : R(0), dy = t == t0 ? dl1.y : R(0);
+            const R tc = (C[1 + t].x + C[1 + t].x) + dx, ts = (C[1 + t].y + C[1 + t].y) + dy;
+            dul += (tc * dl1.x + ts * dl1.y) * b[t];
+        }
+        acc.add(RV_DUL, dul);
+        if constexpr (KIND == PASS_NEW && FORCES) {
+            R2 Cn[1 + NT];
+            Cn[0] = mk2(C[0].x + dl0.x, C[0].y + dl0.y);
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+                Cn[1 + t] = mk2(C[1 + t].x + (t == t0 ? dl1.x : R(0)), C[1 + t].y + (t == t0 ? dl1.y : R(0)));
+            forces(Cn);
+        }
+    }
+}
+
+// The k-space sweep of one pass over the worker's entries.  Registers layout: k, beta, beta_LJ and
+// rho stay in registers (R), the old phase sums are R.mold and the delta R.dl; all EPT entries run
+// without a branch between them, so their dependency chains interleave (an entry past the last has
+// k = 0 and zero beta, beta_LJ and rho: it adds exact zeros).  Streamed layout: every entry is read
+// from memory (L2-resident), the next entry's loads in flight while the current one computes; the
+// old sums go to the chain's scratch in PASS_OLD and come from there in PASS_NEW, the delta goes to
+// the scratch.  SIMPLE: only rows 0 and 1 + t0 of mold and dl exist (in registers: rows 0 and 1).
+template <int NT, int EPT, int KIND, bool FORCES, bool MX, bool SIMPLE, class AccT>
 __device__ __forceinline__ void kspace_sweep(const DevSys &D, RegsOf<NT, EPT, MX> &R, const PhaseTabs<MX> &pt,
-                                             const Slot *slots, int na, int e0, int estep,
-                                             const typename Prec<MX>::R2 *mold_in, typename Prec<MX>::R2 *mold_out,
-                                             bool mold_store, AccT &acc) {
+                                             const MolK<MX> &mk, int e0, int estep, typename Prec<MX>::R2 *mold_g,
+                                             AccT &acc) {
     using Rt = typename Prec<MX>::R;
     using R2 = typename Prec<MX>::R2;
     const int S = D.S;
-    R2 *dl_g = scratch_buf<MX>(D.scratch, 1, 1 + NT, S);
+    const int t0 = SIMPLE ? mk.type[0] - 1 : 0;
     if constexpr (EPT > 0) {
         static_for<0, EPT>([&](auto kc) {
             constexpr int k = decltype(kc)::value;
-            if (R.e[k] < 0) return;
-            if (KIND == PASS_NEW && mold_in) {
+            if constexpr (SIMPLE) {
+                Rt b[NT];
 #pragma unroll
-                for (int t = 0; t <= NT; ++t) R.mold[k][t] = mold_in[(size_t)t * S + R.e[k]];
-            }
-            kspace_entry<NT, KIND, FORCES, MX>(pt, slots, na, R.kx[k], R.ky[k], R.kz[k], R.beta[k], R.bl[k],
-                                               R.rho[k], R.mold[k], R.dl[k], acc);
-            if (KIND == PASS_OLD && mold_store) {
-#pragma unroll
-                for (int t = 0; t <= NT; ++t) mold_out[(size_t)t * S + R.e[k]] = R.mold[k][t];
+                for (int t = 0; t < NT; ++t) b[t] = beta_lj_of<NT, Rt>(R.bl[k], t0, t);
+                kspace_entry_simple<NT, KIND, FORCES, MX>(pt, mk, R.kx[k], R.ky[k], R.kz[k], R.beta[k], b, R.rho[k],
+                                                          R.mold[k][0], R.mold[k][1], R.dl[k][0], R.dl[k][1], acc);
+            } else {
+                kspace_entry<NT, KIND, FORCES, MX>(pt, mk, R.kx[k], R.ky[k], R.kz[k], R.beta[k], R.bl[k],
+                                                   R.rho[k], R.mold[k], R.dl[k], acc);
             }
         });
     } else {
-        // U entries per iteration: their independent dependency chains interleave
-        constexpr int U = YAMC_KSPACE_UNROLL;
         constexpr bool IN_MOLD = KIND == PASS_NEW;   // read the old sums
+        constexpr int NB = SIMPLE ? NT : NPair<NT>::value;  // beta_LJ rows read per entry
+        constexpr int NR = SIMPLE ? 2 : 1 + NT;             // rows of mold and dl
+        R2 *dl_g = scratch_buf<MX>(D.scratch, 1, 1 + NT, S);
         // the mixed form reads FP32 rho (D.rho_f, equal to rho rounded to FP32, which is what its
         // arithmetic takes), FP32 beta tables and FP32 scratch; k comes packed in one word
         using RhoT = std::conditional_t<MX, float2, double2>;
-        int kv_n[U];
-        Rt beta_n[U], bl_n[U][NPair<NT>::value];
-        RhoT rho_n[U][1 + NT];
-        R2 mold_n[U][1 + NT];
+        auto row = [&](int r) { return (SIMPLE && r == 1) ? 1 + t0 : r; };
+        auto brow = [&](int p) { return SIMPLE ? pair_idx<NT>(t0, p) : p; };
+        int kv_n;
+        Rt beta_n, bl_n[NB];
+        RhoT rho_n[1 + NT];
+        R2 mold_n[NR];
         // the loads of the next entry stay in flight until the entry is taken up: no value is
         // converted here
-        auto fetch = [&](int j, int e) {
-            kv_n[j] = D.kpack[YAMC_IX(e, S)];
+        auto fetch = [&](int e) {
+            kv_n = D.kpack[YAMC_IX(e, S)];
             if constexpr (MX) {
-                beta_n[j] = D.ebeta_f[e];
+                beta_n = D.ebeta_f[e];
 #pragma unroll
-                for (int p = 0; p < NPair<NT>::value; ++p) bl_n[j][p] = D.ebetalj_f[(size_t)p * S + e];
+                for (int p = 0; p < NB; ++p) bl_n[p] = D.ebetalj_f[(size_t)brow(p) * S + e];
             } else {
-                beta_n[j] = D.ebeta[e];
+                beta_n = D.ebeta[e];
 #pragma unroll
-                for (int p = 0; p < NPair<NT>::value; ++p) bl_n[j][p] = D.ebetalj[(size_t)p * S + e];
+                for (int p = 0; p < NB; ++p) bl_n[p] = D.ebetalj[(size_t)brow(p) * S + e];
             }
 #pragma unroll
             for (int t = 0; t <= NT; ++t) {
-                if constexpr (MX) rho_n[j][t] = D.rho_f[(size_t)t * S + e];
-                else rho_n[j][t] = D.rho[(size_t)t * S + e];
-                mold_n[j][t] = IN_MOLD ? mold_in[(size_t)t * S + e] : mk2(Rt(0), Rt(0));
+                if constexpr (MX) rho_n[t] = D.rho_f[(size_t)t * S + e];
+                else rho_n[t] = D.rho[(size_t)t * S + e];
+            }
+            if constexpr (IN_MOLD) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r) mold_n[r] = mold_g[(size_t)row(r) * S + e];
             }
         };
-        const int step = U * estep;
+        if (e0 < S) fetch(e0);
+        for (int e = e0; e < S; e += estep) {
+            const int kx = kv_n & 255, ky = ((kv_n >> 8) & 255) - 128, kz = (kv_n >> 16) - 128;
+            const Rt beta = beta_n;
+            Rt bl[NB];
+            RhoT rho[1 + NT];
+            R2 mold[NR], dl[NR];
 #pragma unroll
-        for (int j = 0; j < U; ++j)
-            if (e0 + j * estep < S) fetch(j, e0 + j * estep);
-        for (int e = e0; e < S; e += step) {
-            int kx[U], ky[U], kz[U];
-            Rt beta[U], bl[U][NPair<NT>::value];
-            RhoT rho[U][1 + NT];
-            R2 mold[U][1 + NT], dl[U][1 + NT];
+            for (int p = 0; p < NB; ++p) bl[p] = bl_n[p];
 #pragma unroll
-            for (int j = 0; j < U; ++j) {
-                kx[j] = kv_n[j] & 255; ky[j] = ((kv_n[j] >> 8) & 255) - 128; kz[j] = (kv_n[j] >> 16) - 128;
-                beta[j] = beta_n[j];
+            for (int t = 0; t <= NT; ++t) rho[t] = rho_n[t];
 #pragma unroll
-                for (int p = 0; p < NPair<NT>::value; ++p) bl[j][p] = bl_n[j][p];
+            for (int r = 0; r < NR; ++r) mold[r] = IN_MOLD ? mold_n[r] : mk2(Rt(0), Rt(0));
+            if (e + estep < S) fetch(e + estep);
+            if constexpr (SIMPLE)
+                kspace_entry_simple<NT, KIND, FORCES, MX>(pt, mk, kx, ky, kz, beta, bl, rho, mold[0], mold[1], dl[0],
+                                                          dl[1], acc);
+            else
+                kspace_entry<NT, KIND, FORCES, MX>(pt, mk, kx, ky, kz, beta, bl, rho, mold, dl, acc);
 #pragma unroll
-                for (int t = 0; t <= NT; ++t) { rho[j][t] = rho_n[j][t]; mold[j][t] = mold_n[j][t]; }
-            }
-#pragma unroll
-            for (int j = 0; j < U; ++j)
-                if (e + step + j * estep < S) fetch(j, e + step + j * estep);
-#pragma unroll
-            for (int j = 0; j < U; ++j)
-                if (e + j * estep < S)
-                    kspace_entry<NT, KIND, FORCES, MX>(pt, slots, na, kx[j], ky[j], kz[j], beta[j], bl[j], rho[j],
-                                                       mold[j], dl[j], acc);
-#pragma unroll
-            for (int j = 0; j < U; ++j) {
-                const int ej = e + j * estep;
-                if (ej >= S) continue;
-#pragma unroll
-                for (int t = 0; t <= NT; ++t) {
-                    if (KIND == PASS_OLD) mold_out[(size_t)t * S + ej] = mold[j][t];
-                    else dl_g[(size_t)t * S + ej] = dl[j][t];
-                }
+            for (int r = 0; r < NR; ++r) {
+                if (KIND == PASS_OLD) mold_g[(size_t)row(r) * S + e] = mold[r];
+                else dl_g[(size_t)row(r) * S + e] = dl[r];
             }
         }
     }
+}
+
+// Sums N <= 16 values over the warp: a tree that halves the values each lane holds at every step
+// (15 exchanges for 16 values and one more, against 80 for a butterfly per value; the same pairs
+// are added in the same order, so the sums are the butterfly's bit for bit).  Value i ends in lane
+// 2 i (and 2 i + 1); returns the lane's value.
+template <int N>
+__device__ __forceinline__ double warp_sums(const double (&v)[N]) {
+    static_assert(N <= 16, "at most 16 values");
+    const int lane = threadIdx.x & 31;
+    double a[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) a[i] = i < N ? v[i < N ? i : 0] : 0.0;
+#pragma unroll
+    for (int h = 8; h >= 1; h >>= 1) {
+        const bool up = lane & (2 * h);
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double keep = pick<double>(up, a[i + h], a[i]), give = pick<double>(up, a[i], a[i + h]);
+            a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+        }
+    }
+    return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
+}
+
+// The k-space part of a pass: the sweep over the worker's entries, then its sums (dU_k and, with
+// FORCES, the k-space forces) over the warp into the warp's row of red -- all values of the row
+// that the pass uses, so the real-space part adds to it.
+constexpr int kKV = 2 + 3 * kMaxA;  // k-space values: dU_k Coulomb, dU_k LJ, forces
+template <int NT, int EPT, int KIND, bool FORCES, bool MX, bool SIMPLE>
+__device__ __forceinline__ void kspace_part(const DevSys &D, RegsOf<NT, EPT, MX> &R, const PhaseTabs<MX> &pt,
+                                            const MolK<MX> &mk, int e0, int estep, typename Prec<MX>::R2 *mold_g,
+                                            double *row) {
+    Acc<MX> acc;
+    acc.zero();
+    kspace_sweep<NT, EPT, KIND, FORCES, MX, SIMPLE>(D, R, pt, mk, e0, estep, mold_g, acc);
+    double v[FORCES ? kKV : 2];
+#pragma unroll
+    for (int i = 0; i < (FORCES ? kKV : 2); ++i) v[i] = acc.kpart(i < 2 ? RV_DUC + i : RV_F + i - 2);
+    const double x = warp_sums(v);
+    const int lane = threadIdx.x & 31, i = lane >> 1;
+    if (!(lane & 1) && i < (FORCES ? kKV : 2)) row[i < 2 ? RV_DUC + i : RV_F + i - 2] = x;
+}
+template <int NT, int EPT, int KIND, bool FORCES, bool MX, bool SIMPLE>
+__device__ __noinline__ void kspace_part_call(const DevSys &D, RegsOf<NT, EPT, MX> &R, const PhaseTabs<MX> &pt,
+                                              const Slot *slots, int na, int e0, int estep,
+                                              typename Prec<MX>::R2 *mold_g, double *row) {
+    kspace_part<NT, EPT, KIND, FORCES, MX, SIMPLE>(D, R, pt, MolK<MX>(slots, na), e0, estep, mold_g, row);
 }
 
 // The workers' part of one pass over the molecule's slots: k-space over their entries, real
@@ -655,7 +836,7 @@ __device__ __forceinline__ void worker_pass_body(const DevSys &D, ChainShared &s
                                             int *blist, int *queue,
                                             int *nearbuf,
                                             double *red, const double *lj_s, int nown, int qcap, int e0, int estep,
-                                            long long *prof, typename Prec<MX>::R2 *mold_buf, bool mold_out) {
+                                            long long *prof, typename Prec<MX>::R2 *mold_buf) {
     constexpr int NVMAX = FORCES ? kNVP : RV_F;
     const Cand &m = sh.cand[sh.icur];
     const int na = m.na;
@@ -678,31 +859,24 @@ __device__ __forceinline__ void worker_pass_body(const DevSys &D, ChainShared &s
     build_tables<MX>(tab, m.slot, s_lo, s_hi, KM, wtid, nwork);
     worker_sync(nwork);
     YAMC_WPH(PH_TABLES);
-    int tmask = 0;
-    for (int a = 0; a < na; ++a)
-        if (m.slot[a].type > 0) tmask |= 1 << (m.slot[a].type - 1);
-    const PhaseTabs<MX> pt{tab, KM, tmask};
+    const PhaseTabs<MX> pt{tab, KM};
 
-    Acc<MX> acc;
-    acc.zero();
-    kspace_sweep<NT, EPT, KIND, FORCES, MX>(D, R, pt, m.slot, na, e0, estep, EPT > 0 ? nullptr : mold_buf, mold_buf,
-                                            mold_out, acc);
-    // the mixed form's FP32 k-space sums (dU_k, k-space forces) leave the registers here: reduced
-    // over the warp into its row now, so the real-space phase holds only its own accumulators;
-    // the real-space values are added to the row at the end
+    // k space, out of line when the entries are streamed: each sweep then has the register budget to
+    // itself, and its sums are in the warp's row of red before the real-space part begins
     const int nv = FORCES ? (RV_F + 3 * na) : RV_F;
-    auto kvalue = [&](int v) { return (KIND != PASS_OLD && (v == RV_DUC || v == RV_DUL)) || (FORCES && v >= RV_F && v < nv); };
-    if constexpr (MX) {
-#pragma unroll
-        for (int v = 0; v < NVMAX; ++v) {
-            if (!kvalue(v)) continue;
-            double x = acc.kpart(v);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            if (lane == 0) red[wwarp * kNV + v] = x;
-            acc.clear_kpart(v);
+    {
+        const MolK<MX> mk(m.slot, na);
+        double *row = red + wwarp * kNV;
+        if constexpr (EPT > 0) {
+            if (mk.simple) kspace_part<NT, EPT, KIND, FORCES, MX, true>(D, R, pt, mk, e0, estep, mold_buf, row);
+            else kspace_part<NT, EPT, KIND, FORCES, MX, false>(D, R, pt, mk, e0, estep, mold_buf, row);
+        } else {
+            if (mk.simple) kspace_part_call<NT, EPT, KIND, FORCES, MX, true>(D, R, pt, m.slot, na, e0, estep, mold_buf, row);
+            else kspace_part_call<NT, EPT, KIND, FORCES, MX, false>(D, R, pt, m.slot, na, e0, estep, mold_buf, row);
         }
     }
+    Acc<MX> acc;
+    acc.zero();
     YAMC_WPH(PH_KSPACE);
 
     // bounding spheres of the molecule at its new (slot 0) and old (slot na) positions: an atom
@@ -889,18 +1063,20 @@ __device__ __forceinline__ void worker_pass_body(const DevSys &D, ChainShared &s
         if (!more_rounds) break;
     }
 
-    // per-warp reduction (xor tree) into red[worker warp][value] (the mixed form adds its
-    // k-space part, already there)
+    // the real-space sums over the warp, added to the k-space sums in the warp's row
+    {
+        constexpr int NR = FORCES ? 3 + 3 * kMaxA : 3;
+        double v[NR];
 #pragma unroll
-    for (int v = 0; v < NVMAX; ++v) {
-        if (v < nv) {
-            double x = acc.get(v);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double y = __shfl_xor_sync(0xffffffffu, x, o);
-                x = (v == RV_OVL) ? fmax(x, y) : x + y;
-            }
-            if (lane == 0) red[wwarp * kNV + v] = (MX && kvalue(v)) ? red[wwarp * kNV + v] + x : x;
+        for (int i = 0; i < NR; ++i) v[i] = acc.get(i < 3 ? RV_EW + i : RV_F + i - 3);
+        const double x = warp_sums(v);
+        const bool ovl = __any_sync(0xffffffffu, acc.get(RV_OVL) > 0.0);
+        const int i = lane >> 1, at = i < 3 ? RV_EW + i : RV_F + i - 3;
+        double *row = red + wwarp * kNV;
+        if (!(lane & 1) && i < NR && at < nv) row[at] = i < 3 ? x : row[at] + x;
+        if (lane == 31) {
+            row[RV_OVL] = ovl ? 1.0 : 0.0;
+            if (KIND == PASS_OLD) row[RV_DUC] = row[RV_DUL] = 0.0;
         }
     }
 #undef YAMC_WPH
@@ -916,9 +1092,9 @@ __device__ __noinline__ void worker_pass_call(const DevSys &D, ChainShared &sh, 
                                               int dhs_typed, int grank, int gsize, const int2 *meta_s, const float4 *box_s,
                                             int *blist, int *queue,
                                               int *nearbuf, double *red, const double *lj_s, int nown, int qcap, int e0,
-                                              int estep, long long *prof, typename Prec<MX>::R2 *mold_buf, bool mold_out) {
+                                              int estep, long long *prof, typename Prec<MX>::R2 *mold_buf) {
     worker_pass_body<NT, EPT, KIND, FORCES, MX>(D, sh, R, tab_raw, atom_s, dhs_ts, dhs_g, dhs_typed, grank, gsize, meta_s,
-                                                box_s, blist, queue, nearbuf, red, lj_s, nown, qcap, e0, estep, prof, mold_buf, mold_out);
+                                                box_s, blist, queue, nearbuf, red, lj_s, nown, qcap, e0, estep, prof, mold_buf);
 }
 
 template <int NT, int EPT, int KIND, bool FORCES, bool MX>
@@ -927,15 +1103,15 @@ __device__ __forceinline__ void worker_pass(const DevSys &D, ChainShared &sh, Re
                                             int dhs_typed, int grank, int gsize, const int2 *meta_s, const float4 *box_s,
                                             int *blist, int *queue,
                                             int *nearbuf, double *red, const double *lj_s, int nown, int qcap, int e0,
-                                            int estep, long long *prof, typename Prec<MX>::R2 *mold_buf, bool mold_out) {
+                                            int estep, long long *prof, typename Prec<MX>::R2 *mold_buf) {
     if constexpr (EPT > 0)
         worker_pass_body<NT, EPT, KIND, FORCES, MX>(D, sh, R, tab_raw, atom_s, dhs_ts, dhs_g, dhs_typed, grank, gsize,
                                                     meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, qcap, e0, estep, prof,
-                                                    mold_buf, mold_out);
+                                                    mold_buf);
     else
         worker_pass_call<NT, EPT, KIND, FORCES, MX>(D, sh, R, tab_raw, atom_s, dhs_ts, dhs_g, dhs_typed, grank, gsize,
                                                     meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, qcap, e0, estep, prof,
-                                                    mold_buf, mold_out);
+                                                    mold_buf);
 }
 
 // Control warp, after the workers' per-warp partials: trees over the worker warps, then over the
@@ -1007,8 +1183,12 @@ struct ChooseCtx {
 };
 
 __device__ inline RngReader make_reader(const ChooseCtx &X, const ChainShared &sh, long long cur) {
-    return RngReader{X.run->rng, X.run->rng_off, X.run->n_rng, cur, 0, X.w0, sh.wbase[0], sh.wn[0],
-                     X.w1, sh.wbase[1], sh.wn[1]};
+    // the window that holds cur (the newer one where both do): the draws of a move fit in it, and
+    // one that passes its end reads the stream itself
+    const int b = sh.wnext ^ 1;
+    const unsigned long long k = (unsigned long long)(cur - sh.wbase[b]);
+    const int s = sh.wbase[b] >= 0 && k < (unsigned long long)sh.wn[b] ? b : b ^ 1;
+    return RngReader{X.run->rng, X.run->rng_off, X.run->n_rng, cur, 0, s ? X.w1 : X.w0, sh.wbase[s], sh.wn[s]};
 }
 
 __device__ inline void stage_molecule(const ChooseCtx &X, ChainShared &sh, Cand &C, int imol, int moving,
@@ -1022,9 +1202,17 @@ __device__ inline void stage_molecule(const ChooseCtx &X, ChainShared &sh, Cand 
     else { const int2 mr = D.mol[YAMC_IX(imol - 1, D.M)]; first = mr.x; nam = mr.y; }
     C.imol = imol; C.first = first; C.na = nam;
     double mx = 0, my = 0, mz = 0;
-    int slots[kMaxA];  // staging slots of the molecule's atoms (loaded together)
+    int slots[kMaxA];  // staging slots of the molecule's atoms (loaded together), then their positions
+    double4 pos[kMaxA];
 #pragma unroll
-    for (int a = 0; a < kMaxA; ++a) slots[a] = a < nam ? D.slot[YAMC_IX(first + a, D.N)] : 0;
+    for (int a = 0; a < kMaxA; ++a) slots[a] = a < nam ? ld_table(D.slot + YAMC_IX(first + a, D.N)) : 0;
+    const bool staged = imol - 1 != moving && imol - 1 != sh.last_mol;
+#pragma unroll
+    for (int a = 0; a < kMaxA; ++a)
+        if (staged && a < nam) {
+            const double4 *src = (X.G > 1) ? cluster.map_shared_rank(X.atom_s, (first + a) % X.G) : X.atom_s;
+            pos[a] = src[slots[a]];
+        }
 #pragma unroll
     for (int a = 0; a < kMaxA; ++a) {
         if (a >= nam) break;
@@ -1040,11 +1228,7 @@ __device__ inline void stage_molecule(const ChooseCtx &X, ChainShared &sh, Cand 
         s.pad = slots[a];  // the commit updates the staged copy in this slot of CTA j % G
         if (imol - 1 == moving) { s.x = moving_pos[a].x; s.y = moving_pos[a].y; s.z = moving_pos[a].z; }
         else if (imol - 1 == sh.last_mol) { s.x = sh.lx[a]; s.y = sh.ly[a]; s.z = sh.lz[a]; }
-        else {
-            const double4 *src = (X.G > 1) ? cluster.map_shared_rank(X.atom_s, j % X.G) : X.atom_s;
-            const double4 p = src[slots[a]];
-            s.x = p.x; s.y = p.y; s.z = p.z;
-        }
+        else { s.x = pos[a].x; s.y = pos[a].y; s.z = pos[a].z; }
         C.slot[nam + a] = s;  // old positions
         C.slot[a] = s;        // proposed positions, replaced by propose()
         // dipole of the molecule at the old positions (EwaldSumExternal_calc_mu)
@@ -1087,8 +1271,10 @@ __device__ inline void propose(const DevSys &D, Cand &C, RngReader &rng, const d
 // atoms' per-axis phase tables built in chunks in the scratch region; then the k-space energies
 // (EwaldSumKSpace_calc_coulomb_energy / _calc_LJ_energy, EwaldSumKSpace.f90:389-526) are
 // reduced over the cluster into the engine scalars.
-template <int NT, int EPT, class Regs>
-__device__ __noinline__ void refresh_in_chain(const DevSys &D, Regs &R, double2 *scr, int scr_atoms, int e0, int estep,
+// (the entries of the register layout come back through D.rho: taking the address of the
+// register-held rows would keep them in local memory for the whole launch)
+template <int NT, int EPT>
+__device__ __noinline__ void refresh_in_chain(const DevSys &D, double2 *scr, int scr_atoms, int e0, int estep,
                                               int G, int rank, ChainShared &sh, double *red, double *xch, int xpar,
                                               cg::cluster_group &cluster) {
     const int tid = threadIdx.x, B = blockDim.x;
@@ -1111,9 +1297,7 @@ __device__ __noinline__ void refresh_in_chain(const DevSys &D, Regs &R, double2 
         double2 acc[EB][1 + NT];
 #pragma unroll
         for (int j = 0; j < EB; ++j) {
-            int e;
-            if constexpr (EPT > 0) e = R.e[j];
-            else e = e0 + (b * EB + j) * estep;
+            const int e = e0 + (b * EB + j) * estep;
             ent[j] = (!ctl && e >= 0 && e < S) ? e : -1;
             kv[j] = ent[j] >= 0 ? D.kvec[ent[j]] : make_int4(0, 0, 0, 0);
 #pragma unroll
@@ -1164,9 +1348,8 @@ __device__ __noinline__ void refresh_in_chain(const DevSys &D, Regs &R, double2 
             if (e < 0) continue;
 #pragma unroll
             for (int t = 0; t <= NT; ++t) {
-                if constexpr (EPT > 0) R.rho[j][t] = acc[j][t];
-                else {
-                    D.rho[(size_t)t * S + e] = acc[j][t];
+                D.rho[(size_t)t * S + e] = acc[j][t];
+                if constexpr (EPT <= 0) {
                     D.rho_f[(size_t)t * S + e] = make_float2((float)acc[j][t].x, (float)acc[j][t].y);
                 }
             }
@@ -1234,8 +1417,8 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
 
     // shared memory carve-up (chain_smem_bytes on the host computes the same sizes)
     const int nblk_max = (A.nown_max + kBlk - 1) / kBlk;
-    double2 *tab = reinterpret_cast<double2 *>(smem_raw);                     // [2 kMaxA][3][KM]
-    float4 *box_s = reinterpret_cast<float4 *>(tab + 2 * kMaxA * 3 * KM);     // [nblk_max][2]
+    double2 *tab = reinterpret_cast<double2 *>(smem_raw);                     // [3][KM][kTabRow]
+    float4 *box_s = reinterpret_cast<float4 *>(tab + kTabRow * 3 * KM);       // [nblk_max][2]
     double4 *atom_s = reinterpret_cast<double4 *>(box_s + 2 * nblk_max);      // [nown_max]
     int2 *meta_s = reinterpret_cast<int2 *>(atom_s + A.nown_max);             // [nown_max]
     int *queue = reinterpret_cast<int *>(meta_s + A.nown_max);                // [qcap]
@@ -1370,7 +1553,7 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
             const int na0 = sh.cand[sh.icur].na;
             // old forces for force-biased moves (movemc Steps 3-4)
             if constexpr (SPLIT) if (biased) {
-                if (!ctl) worker_pass<NT, EPT, PASS_OLD, true, MX>(D, sh, R, tab, atom_s, dhs_ts, D.dhs, D.dhs_typed, rank, G, meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, A.qcap, e0, gwork, prof, mold_g, false);
+                if (!ctl) worker_pass<NT, EPT, PASS_OLD, true, MX>(D, sh, R, tab, atom_s, dhs_ts, D.dhs, D.dhs_typed, rank, G, meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, A.qcap, e0, gwork, prof, mold_g);
                 __syncthreads();
                 reduce_pass(sh, red, xch, RV_F + 3 * na0, G, rank, xpar, cluster);
                 xpar ^= 1;
@@ -1463,8 +1646,8 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
 
         // ------------------------------------------------ the pass over the new positions
         if (!ctl) {
-            if constexpr (SPLIT) worker_pass<NT, EPT, PASS_NEW, true, MX>(D, sh, R, tab, atom_s, dhs_ts, D.dhs, D.dhs_typed, rank, G, meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, A.qcap, e0, gwork, prof, mold_g, false);
-            else worker_pass<NT, EPT, PASS_BOTH, false, MX>(D, sh, R, tab, atom_s, dhs_ts, D.dhs, D.dhs_typed, rank, G, meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, A.qcap, e0, gwork, prof, mold_g, false);
+            if constexpr (SPLIT) worker_pass<NT, EPT, PASS_NEW, true, MX>(D, sh, R, tab, atom_s, dhs_ts, D.dhs, D.dhs_typed, rank, G, meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, A.qcap, e0, gwork, prof, mold_g);
+            else worker_pass<NT, EPT, PASS_BOTH, false, MX>(D, sh, R, tab, atom_s, dhs_ts, D.dhs, D.dhs_typed, rank, G, meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, A.qcap, e0, gwork, prof, mold_g);
         } else if (speculate && it + 1 < n_moves) {
             // prepare the next move's candidates while the workers run: lanes 1-2 after the
             // acceptance draw, lane 2 with the molecule in flight at its proposed positions (used
@@ -1581,6 +1764,7 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
                 flags |= acc;
             }
             sh.accepted = 0;
+            sh.imoved = sh.icur;
             if (out) {
                 sh.abort = kAbortStream;  // the interrupted move restarts from its first draw (sh.cursor unchanged)
             } else {
@@ -1657,17 +1841,26 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
         YAMC_PH(PH_DECIDE);
         if (sh.abort) break;
         if (sh.accepted) {
-            // commit: rho += delta (MC.f90:1245), in registers or in memory by the entry's owner
+            // commit: rho += delta (MC.f90:1245), in registers or in memory by the entry's owner; the
+            // rows of LJ types that the molecule does not carry have no delta
+            const MolK<MX> mk(sh.cand[sh.imoved].slot, sh.cand[sh.imoved].na);
+            static_for<0, EPT>([&](auto kc) {
+                constexpr int k = decltype(kc)::value;
+                R.rho[k][0].x += R.dl[k][0].x; R.rho[k][0].y += R.dl[k][0].y;
 #pragma unroll
-            for (int k = 0; k < EPT; ++k)
-#pragma unroll
-                for (int t = 0; t <= NT; ++t) { R.rho[k][t].x += R.dl[k][t].x; R.rho[k][t].y += R.dl[k][t].y; }
+                for (int t = 1; t <= NT; ++t) {
+                    const Rt dx = pick<Rt>(mk.simple, R.dl[k][1].x, R.dl[k][t].x), dy = pick<Rt>(mk.simple, R.dl[k][1].y, R.dl[k][t].y);
+                    const bool hit = (mk.tmask >> (t - 1)) & 1;
+                    R.rho[k][t].x += hit ? (double)dx : 0.0; R.rho[k][t].y += hit ? (double)dy : 0.0;
+                }
+            });
             if constexpr (EPT <= 0) {
                 if (!ctl) {
                     const R2 *dl_g = scratch_buf<MX>(D.scratch, 1, 1 + NT, S);
                     for (int e = e0; e < S; e += gwork)
 #pragma unroll
                         for (int t = 0; t <= NT; ++t) {
+                            if (t > 0 && !((mk.tmask >> (t - 1)) & 1)) continue;
                             double2 r = D.rho[(size_t)t * S + e];
                             const double2 d = to_d2(dl_g[(size_t)t * S + e]);
                             r.x += d.x; r.y += d.y;
@@ -1684,7 +1877,13 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
         if constexpr (MX) {
             acc_since += sh.accepted;  // the same decisions in every CTA: every thread agrees
             if (refresh_every > 0 && acc_since >= refresh_every) {
-                refresh_in_chain<NT, EPT>(D, R, scr, scr_atoms, e0, gwork, G, rank, sh, red, xch, xpar, cluster);
+                refresh_in_chain<NT, EPT>(D, scr, scr_atoms, e0, gwork, G, rank, sh, red, xch, xpar, cluster);
+                static_for<0, EPT>([&](auto kc) {
+                    constexpr int k = decltype(kc)::value;
+#pragma unroll
+                    for (int t = 0; t <= NT; ++t)
+                        if (R.e[k] >= 0) R.rho[k][t] = D.rho[(size_t)t * S + R.e[k]];
+                });
                 xpar ^= 1;
                 acc_since = 0;
                 ++refreshes;

@@ -309,36 +309,45 @@ __host__ __device__ inline void entry_phase(const T2 *tx, const T2 *ty, const T2
 // ------------------------------------------------------------------ random stream
 // rand() of random.f90:65-93: successive REAL(4) random_number values, values
 // outside [1e-14, 1-1e-14] are drawn again.  The buffer holds the raw stream.
+// One stretch of the stream [wb, wb + wn) may be read from a copy (a window in shared memory on
+// the device) instead of the buffer.
 struct RngReader {
     const float *buf;  // holds stream positions [off, n)
     long long off;
     long long n;       // end of the stream available
     long long cur;     // next position to read
     int out;           // set once the stream ran out
-    // optional copies of stream windows [b0, b0+n0) and [b1, b1+n1) (shared memory on the device)
-    const float *w0 = nullptr;
-    long long b0 = 0;
-    int n0 = 0;
-    const float *w1 = nullptr;
-    long long b1 = 0;
-    int n1 = 0;
+    const float *w = nullptr;
+    long long wb = 0;
+    int wn = 0;
     __host__ __device__ inline float raw() {
         if (cur >= n) { out = 1; return 0.5f; }
         const long long i = cur++;
-        if (w0 && i >= b0 && i < b0 + n0) return w0[i - b0];
-        if (w1 && i >= b1 && i < b1 + n1) return w1[i - b1];
-        return buf[i - off];
+        const unsigned long long k = (unsigned long long)(i - wb);
+        return k < (unsigned long long)wn ? w[k] : buf[i - off];
     }
+    // (the limits 1e-14 and 1 - 1e-14 are FP64: a float is below the first exactly when it is below
+    // the first float that is not, and above the second exactly when it is 1 or more)
     __host__ __device__ inline double next() {
-        const double eps = 1e-14;
+        constexpr float lo = 1e-14f;
         float v = 0.0f;
-        while ((double)v < eps || (double)v > 1.0 - eps) {
+        while (((double)lo < 1e-14 ? v <= lo : v < lo) || v >= 1.0f) {
             v = raw();
             if (out) return 0.5;
         }
         return (double)v;
     }
 };
+
+// a load from a table that nothing writes while the kernel runs (through the read-only cache)
+template <class T>
+__host__ __device__ inline T ld_table(const T *p) {
+#ifdef __CUDA_ARCH__
+    return __ldg(p);
+#else
+    return *p;
+#endif
+}
 
 // BiasedRandom_choose (BiasedRandom.f90:81-109): first i with beg(i) < r < end(i),
 // else 1.  The intervals are contiguous (beg(i) = end(i-1)) and increasing when
@@ -353,9 +362,9 @@ __host__ __device__ inline int choose_molecule(double r, const double *beg, cons
     if (!(end[hi] > r)) return 1;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (end[mid] > r) hi = mid; else lo = mid + 1;
+        if (ld_table(end + mid) > r) hi = mid; else lo = mid + 1;
     }
-    return (r > beg[lo]) ? lo + 1 : 1;
+    return (r > ld_table(beg + lo)) ? lo + 1 : 1;
 }
 
 // Same answer with one round trip for flat weights: interval i holds (i, i+1)/M up to the
@@ -368,7 +377,7 @@ __host__ __device__ inline int choose_molecule_guess(double r, const double *beg
     if (g > M - 1) g = M - 1;
     if (g < 0) g = 0;
     for (int step = 0; step < 6; ++step) {
-        const double b = beg[g], e = end[g];
+        const double b = ld_table(beg + g), e = ld_table(end + g);
         if (r > b && r < e) return g + 1;
         if (r == b || r == e) return 1;
         if (r > e) { if (g == M - 1) return 1; ++g; }
@@ -580,7 +589,7 @@ __host__ __device__ inline void mcm_choose_rotation(MoveState &m, RngReader &rng
         if (rng.out) return;
         vmax = 0.0; m.qold = 1.0;
     }
-    m.ca = cos(angle); m.sa = sin(angle);
+    sincos(angle, &m.sa, &m.ca);
     m.ct = vz; m.st = sqrt(1.0 - m.ct * m.ct);
     m.cphi = 0.0; m.sphi = 0.0;
     if (m.st > 0.0) { m.cphi = vx / m.st; m.sphi = vy / m.st; }

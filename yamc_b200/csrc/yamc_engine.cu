@@ -658,11 +658,9 @@ __global__ void __launch_bounds__(kMoveThreads) k_move_pass(DevSys D, MoveIn in,
     const int s_lo = EVAL ? 0 : na, s_hi = EVAL ? na : 2 * na;
     R2 *tab = reinterpret_cast<R2 *>(move_smem);
     build_tables<MX>(tab, sl, s_lo, s_hi, KM, tid, kMoveThreads);
-    int tmask = 0;
-    for (int a = 0; a < na; ++a)
-        if (sl[a].type > 0) tmask |= 1 << (sl[a].type - 1);
+    const MolK<MX> mk(sl, na);
     __syncthreads();
-    const PhaseTabs<MX> pt{tab, KM, tmask};
+    const PhaseTabs<MX> pt{tab, KM};
     Acc<MX> acc;
     acc.zero();
     const int gt = blockIdx.x * kMoveThreads + tid, gs = gridDim.x * kMoveThreads;
@@ -687,7 +685,7 @@ __global__ void __launch_bounds__(kMoveThreads) k_move_pass(DevSys D, MoveIn in,
             rho[t] = D.rho[(size_t)t * S + e];
             mold[t] = EVAL ? mold_g[(size_t)t * S + e] : mk2(R(0), R(0));
         }
-        kspace_entry<NT, KIND, true, MX>(pt, sl, na, kv.x, kv.y, kv.z, beta, bl, rho, mold, dl, acc);
+        kspace_entry<NT, KIND, true, MX>(pt, mk, kv.x, kv.y, kv.z, beta, bl, rho, mold, dl, acc);
 #pragma unroll
         for (int t = 0; t <= NT; ++t) {
             if (EVAL) dl_g[(size_t)t * S + e] = dl[t];
@@ -809,7 +807,7 @@ int upload(T *d, const T *h, size_t n, cudaStream_t s) {
 size_t chain_smem_bytes(int G, int B, int kmax, int nt, int nown_max, int qcap) {
     const int KM = kmax + 1;
     const size_t nblk_max = (size_t)(nown_max + kBlk - 1) / kBlk;
-    size_t b = sizeof(double2) * 2 * kMaxA * 3 * KM;
+    size_t b = sizeof(double2) * kTabRow * 3 * KM;
     b += sizeof(float4) * 2 * nblk_max;
     b += (sizeof(double4) + sizeof(int2)) * (size_t)nown_max;
     b += sizeof(int) * (size_t)((qcap + 1) & ~1);
@@ -999,7 +997,7 @@ int launch_move_pass(yamc_ctx *c, MoveIn &in, bool eval) {
         if ((r = dalloc(&c->d_mpart, (size_t)c->mblocks * kNV)) || (r = dalloc(&c->d_mcount, 1))) return r;
         CUDA_TRY(cudaMemsetAsync(c->d_mcount, 0, sizeof(unsigned), c->stream));
     }
-    const size_t smem = sizeof(double2) * 2 * kMaxA * 3 * (size_t)(H.kmax + 1);
+    const size_t smem = sizeof(double2) * kTabRow * 3 * (size_t)(H.kmax + 1);
     const bool mx = is_mixed(c);
     switch (H.nt) {
         case 1: return mx ? launch_move_pass_t<1, true>(c, in, eval, smem) : launch_move_pass_t<1, false>(c, in, eval, smem);
