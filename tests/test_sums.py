@@ -1,0 +1,94 @@
+"""The whole-configuration sums over spatial tiles, at sizes around their edges (tiles of 32 atoms,
+cell grids of 1 to 8 per axis) and with molecules outside the unit box, where the reference's single
+conditional wrap and the nearest image differ: the tiles must hand over every pair that the wrap puts
+inside the cutoff.  Real space against a direct numpy sum of all pairs, 1e-11 of the sum of magnitudes
+(about 1e5 terms of FP64 rounding); forces against its gradient by the same formula; k space against
+the unshifted configuration (whole-box shifts change no phase beyond rounding, 1e-11).  RDF counts
+equal the oracle's."""
+import math
+
+import numpy as np
+import pytest
+
+import pyoracle
+from yamc_b200 import api, systems
+
+pytestmark = pytest.mark.gpu
+
+
+def _erfc(x):
+    x2, e2 = x * x, np.exp(-x * x)
+    t = 1.0 / (1.0 + 0.3275911 * x)
+    mid = t * (0.254829592 + t * (-0.284496736 + t * (1.421413741 + t * (-1.453152027 + t * 1.061405429)))) * e2
+    low = 1.0 - 2.0 / 1.7724538509055 * x * (1.0 - x2 * (1 / 3 - x2 * (0.1 - x2 * (1 / 42 - x2 / 216))))
+    far = (1.0 - 0.5 * (1.0 - 1.5 / x2) / x2) / (1.7724538509055 * x) * e2
+    return np.where(x < 0.455, low, np.where(x > 3.0, far, mid))
+
+
+def _real_space(inp, eng, x):
+    """(uu_ew, uu_lj6, uu_lj12) and the sums of their magnitudes, every pair once."""
+    p = eng.current_params()
+    mol = np.repeat(np.arange(inp.nmol), inp.last_atom - inp.first_atom + 1)
+    tot, mag = np.zeros(3), np.zeros(3)
+    for i in range(len(x) - 1):
+        d = x[i] - x[i + 1:]
+        d = np.where(d > 0.5, d - 1.0, d)
+        d = np.where(d < -0.5, d + 1.0, d)
+        r2 = (d * d).sum(1)
+        j = np.nonzero(r2 < p.rmax2)[0]
+        r2, k = r2[j], j + i + 1
+        r = np.sqrt(r2)
+        a = p.alpha * r
+        f = _erfc(a) - (mol[k] == mol[i])
+        ew = p.xclb * inp.charge[i] * inp.charge[k] * f / r
+        lj = (inp.sigma[i] > 1e-8) & (inp.sigma[k] > 1e-8)
+        s6 = np.where(lj, ((inp.sigma[i] + inp.sigma[k]) / 2) ** 6 / r2 ** 3, 0.0)
+        e4 = 4 * np.sqrt(inp.epsilon[i] * inp.epsilon[k]) * np.exp(-a * a)
+        a2 = a * a
+        c6 = 1 + a2 * (1 + a2 / 2)
+        c12 = c6 + a2 ** 3 * (1 + a2 * (1 + a2 / 5) / 4) / 6
+        for v, t in enumerate((ew, e4 * s6 * c6, e4 * s6 * s6 * c12)):
+            tot[v] += t.sum()
+            mag[v] += np.abs(t).sum()
+    return tot, mag
+
+
+@pytest.mark.parametrize("n_water,n_ion", [(10, 1), (11, 0), (85, 0), (171, 1), (700, 5)])
+def test_real_space_tiles_with_molecules_outside_the_box(tmp_path, n_water, n_ion):
+    box = ((n_water + 2 * n_ion) / 0.015) ** (1 / 3)
+    rc = min(9.0, 0.48 * box)
+    spec = systems.SystemSpec("odd", n_water, n_ion, n_ion, box, 3.2 / rc, rc, 5)
+    files = systems.write_system(spec, str(tmp_path), seed=n_water)
+    inp = api.load_inputs(files["parameters"], files["composition"], files["moltab"])
+    eng = api.Engine(inp)
+    base = eng.energies()
+    f0 = eng.forces()[0]
+    x = np.stack([inp.x, inp.y, inp.z], 1)
+    tot, mag = _real_space(inp, eng, x)
+    assert np.all(np.abs(base[3:6] - tot) <= 1e-11 * mag)
+    r = np.random.default_rng(3)
+    shift = r.integers(-1, 2, (inp.nmol, 3)) * (r.random((inp.nmol, 1)) < 0.3)
+    y = x + np.repeat(shift, inp.last_atom - inp.first_atom + 1, axis=0)
+    e = eng.set_positions(y[:, 0], y[:, 1], y[:, 2])
+    tot, mag = _real_space(inp, eng, y)
+    assert np.all(np.abs(e[3:6] - tot) <= 1e-11 * mag)
+    assert np.all(np.abs(e[6:8] - base[6:8]) <= 1e-11 * np.abs(base[6:8]).max())
+    eng.set_positions(*(np.ascontiguousarray(v) for v in x.T))
+    assert np.abs(eng.forces()[0] - f0).max() <= 1e-12 * np.abs(f0).max()
+
+
+@pytest.mark.parametrize("m", [1023, 1024, 1057, 2001])
+def test_rdf_tiles_count_as_all_pairs(m):
+    r = np.random.default_rng(m)
+    x, y, z = r.uniform(-0.5, 0.5, (3, m))
+    x[::7] += 1.0   # outside the unit box: counted by the single conditional wrap
+    z[::11] -= 1.0
+    mol_type = np.where(np.arange(m) % 5 == 0, 2, 1).astype(np.int32)
+    counts = np.array([(mol_type == 1).sum(), (mol_type == 2).sum()], dtype=np.int32)
+    o = pyoracle.RDF(mol_type, counts, dr=0.1, rmax=12.0)
+    o.add_frame(x, y, z, 31.0)
+    g = api.RDF(mol_type, counts, dr=0.1, rmax=12.0)
+    g.add_frame(x, y, z, 31.0)
+    _, _, c, n = g.result()
+    assert n == 1 and np.array_equal(c.ravel(), np.asarray(o.cnt4).ravel())
+    assert c.sum() > 0 and math.isfinite(c.sum())

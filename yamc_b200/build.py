@@ -22,7 +22,7 @@ UNITS = [("yamc_chain_inst.cu", f"yamc_chain_nt{n}.o", [f"-DYAMC_NT={n}"]) for n
     (src, src.rsplit(".", 1)[0] + ".o", []) for src in
     ("yamc_engine.cu", "yamc_static.cu", "yamc_peaks.cu", "yamc_host.cpp", "yamc_inputs.cpp")]
 SOURCES = sorted({u[0] for u in UNITS})
-HEADERS = ["yamc_chain.cuh", "yamc_device.cuh", "yamc_internal.h", os.path.join("..", "..", "include", "yamc.h")]
+HEADERS = ["yamc_chain.cuh", "yamc_device.cuh", "yamc_sums.cuh", "yamc_internal.h", os.path.join("..", "..", "include", "yamc.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -1,8 +1,8 @@
 // B200 engine for YAMC's per-trial-move energy evaluation (movemc, MC.f90:831-1322).
 //
 // Kernels (sm_100a):
-//   k_realspace_full  all-pairs real-space sum (EwaldSumRealSpace_calc, full)      -- init / full recompute
-//   k_rho_full        structure factors rho(k) of all atoms (RhoSquared_addAtoms)  -- init / full recompute
+//   k_real_energy     full real-space sum (EwaldSumRealSpace_calc, full)           -- init / full recompute
+//   k_rho_rows        structure factors rho(k) of all atoms (RhoSquared_addAtoms)  -- init / full recompute
 //   k_kspace_energy   k-space Coulomb + dispersion energy of rho(k)               -- init / full recompute
 //   k_chain<NT,EPT>   persistent Markov chain: one thread-block cluster per chain; every move runs
 //                     proposal -> fused real-space + k-space pass -> cluster reduction -> Metropolis
@@ -33,6 +33,7 @@
 #include "yamc_chain.cuh"
 #include "yamc_device.cuh"
 #include "yamc_internal.h"
+#include "yamc_sums.cuh"
 
 
 // an NVTX range around each public entry point (header-only NVTX 3: it costs nothing unless a
@@ -48,9 +49,6 @@ namespace yamc {
 // ------------------------------------------------------------------------------------------
 // full sums
 // ------------------------------------------------------------------------------------------
-constexpr int kFullTile = 256;
-constexpr int kFullParts = 8;  // ew, lj6, lj12, ew_intra, lj6_intra, lj12_intra, overlap, spare
-
 template <int BS>
 __device__ inline void block_sum(double *vals, int nv, double *sh) {
     // deterministic block reduction of nv values: warp xor tree, then warps in order
@@ -72,163 +70,32 @@ __device__ inline void block_sum(double *vals, int nv, double *sh) {
     __syncthreads();
 }
 
-// EwaldSumRealSpace_calc on the full sum (EwaldSumRealSpace.f90:233-500, j0 = i+1): the
-// energy totals of every pair once.  One block per pair of atom tiles (ti <= tj, the upper
-// triangle, listed in tpairs), so the grid grows as (N/256)^2/2 and fills the GPU even for a
-// few thousand atoms; the j tile sits in shared memory, each thread owns one atom i and runs
-// over it (j > i on the diagonal tile).  Intra-molecular pairs use -erf_Luc and count in the
-// intra totals too; LJ-LJ pairs of different molecules closer than their mean hard-core
-// diameter set the overlap flag.  One partial per block (part[blk*8 + v]), reduced in block
-// order by k_sum_parts.  (The reference's per-atom uu/F of the full sum are not needed: the
-// chain kernel evaluates the moved molecule's old energy directly.)
-__global__ void __launch_bounds__(kFullTile) k_realspace_full(DevSys D, const int2 *tpairs, double *part) {
-    __shared__ double4 tp[kFullTile];
-    __shared__ int2 tm[kFullTile];
-    __shared__ double td[kFullTile];
-    __shared__ double red[(kFullTile / 32 + 1) * kFullParts];
-    const int2 tt = tpairs[blockIdx.x];
-    const int i = tt.x * kFullTile + threadIdx.x, j0 = tt.y * kFullTile;
-    const bool valid = i < D.N;
-    double4 pi = make_double4(0, 0, 0, 0);
-    int2 mi = make_int2(-1, 0);
-    double di = 0;
-    if (valid) { pi = D.atom[i]; mi = D.meta[i]; di = D.dhs[i]; }
-    double acc[kFullParts] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const int nt = D.nt;
-    {
-        const int j = j0 + threadIdx.x;
-        if (j < D.N) { tp[threadIdx.x] = D.atom[j]; tm[threadIdx.x] = D.meta[j]; td[threadIdx.x] = D.dhs[j]; }
-    }
-    __syncthreads();
-    const int nj = min(kFullTile, D.N - j0);
-    if (valid) {
-        const int jstart = tt.x == tt.y ? threadIdx.x + 1 : 0;  // j > i
-        for (int jj = jstart; jj < nj; ++jj) {
-            const double4 pj = tp[jj];
-            const int2 mj = tm[jj];
-            const bool same = mi.x == mj.x;
-            const double dx = min_image(pi.x - pj.x), dy = min_image(pi.y - pj.y), dz = min_image(pi.z - pj.z);
-            const double r2 = dx * dx + dy * dy + dz * dz;
-            const bool lj = mi.y > 0 && mj.y > 0;
-            if (!same && lj) {
-                const double d12 = (di + td[jj]) / 2;
-                if (r2 < d12 * d12) acc[6] = 1.0;
-            }
-            if (r2 >= D.rmax2) continue;
-            const int off = lj ? (mi.y - 1) * nt + (mj.y - 1) : 0;
-            const PairTerm<double> t = pair_term<double, false>(r2, D.xclb * pi.w * pj.w, lj, lj ? D.lj_sig6[off] : 0.0,
-                                                                 lj ? D.lj_feps[off] : 0.0, D.alpha, D.taosp, same);
-            acc[0] += t.ew; acc[1] += t.lj6; acc[2] += t.lj12;
-            if (same) { acc[3] += t.ew; acc[4] += t.lj6; acc[5] += t.lj12; }
-        }
-    }
-    block_sum<kFullTile>(acc, kFullParts, red);
-    if (threadIdx.x < kFullParts) part[(size_t)blockIdx.x * kFullParts + threadIdx.x] = acc[threadIdx.x];
-}
-
-// part[b*nv + v] over b in [0, nb) -> out[v]: thread t adds blocks t, t+256, ... in order, then
-// a fixed tree over the threads (deterministic); value vmax is a flag, reduced by max
-constexpr int kSumThreads = 256;
+// part[v nb + b] over b in [0, nb) -> out[v]: 64 threads per value add blocks t, t + 64, ... in
+// order, then a fixed tree over them (deterministic); value vmax is a flag, reduced by max
+constexpr int kSumThreads = 1024;  // up to 16 values
 __global__ void __launch_bounds__(kSumThreads) k_sum_parts(const double *part, int nb, int nv, int vmax, double *out) {
-    __shared__ double sh[kSumThreads];
-    for (int v = 0; v < nv; ++v) {
-        double x = 0;
-        for (int b = threadIdx.x; b < nb; b += kSumThreads) {
-            const double y = part[(size_t)b * nv + v];
-            x = v == vmax ? fmax(x, y) : x + y;
-        }
-        sh[threadIdx.x] = x;
-        __syncthreads();
-        for (int w = kSumThreads / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) sh[threadIdx.x] = v == vmax ? fmax(sh[threadIdx.x], sh[threadIdx.x + w]) : sh[threadIdx.x] + sh[threadIdx.x + w];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[v] = sh[0];
-        __syncthreads();
-    }
-}
-
-// RhoSquared_addAtoms (RhoSquared.f90:188-243): for each signed entry the sum over atoms, in
-// atom order within a slice, of the charge-weighted phase (Coulomb) and of the unit phase per
-// LJ type, the LJ phase being the Coulomb one times 1/q like RhoSquared_addAtom
-// (RhoSquared.f90:173-176).  Grid: entry blocks x atom slices (blockIdx.y), so a few thousand
-// entries still fill the GPU; slice s writes its partial sums to
-// part[((1+t) * nslice + s) * S + e], and k_rho_reduce adds the slices in order.
-constexpr int kRhoBlock = 512;  // entries per block: the block's atom tables serve 512 entries
-constexpr int kRhoChunk = 32;
-
-template <int NT>
-__global__ void __launch_bounds__(kRhoBlock) k_rho_full(DevSys D, int slice_atoms, double2 *part) {
-    extern __shared__ double2 stab[];  // [kRhoChunk][3][kmax+1]
-    __shared__ double sq[kRhoChunk];
-    __shared__ int st[kRhoChunk];
-    const int KM = D.kmax + 1;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = e < D.S;
-    const int abeg = blockIdx.y * slice_atoms, aend = min(D.N, abeg + slice_atoms);
-    int4 kv = make_int4(0, 0, 0, 0);
-    if (valid) kv = D.kvec[e];
-    double cC = 0, sC = 0;
-    double cL[NT > 0 ? NT : 1], sL[NT > 0 ? NT : 1];
+    __shared__ double half[16];
+    const int v = threadIdx.x >> 6, t = threadIdx.x & 63, lane = threadIdx.x & 31;
+    const bool flag = v == vmax;
+    double x = 0;
+    if (v < nv) {
+        const double *p = part + (size_t)v * nb;
+        for (int b = t; b < nb; b += 64 * 8) {
+            double y[8];
 #pragma unroll
-    for (int t = 0; t < NT; ++t) { cL[t] = 0; sL[t] = 0; }
-    for (int a0 = abeg; a0 < aend; a0 += kRhoChunk) {
-        const int na = min(kRhoChunk, aend - a0);
-        for (int idx = threadIdx.x; idx < na * 3 * KM; idx += blockDim.x) {
-            const int a = idx / (3 * KM), r = idx % (3 * KM), d = r / KM, m = r % KM;
-            const double4 p = D.atom[a0 + a];
-            const double u = d == 0 ? p.x : (d == 1 ? p.y : p.z);
-            double s, c;
-            sincospi(2.0 * (double)m * u, &s, &c);
-            if (m == 0) { s = 0.0; c = 1.0; }
-            stab[(a * 3 + d) * KM + m] = make_double2(c, s);
-        }
-        if (threadIdx.x < na) { sq[threadIdx.x] = D.atom[a0 + threadIdx.x].w; st[threadIdx.x] = D.meta[a0 + threadIdx.x].y; }
-        __syncthreads();
-        if (valid) {
-            for (int a = 0; a < na; ++a) {
-                const double2 *T = stab + (size_t)a * 3 * KM;
-                const double q = sq[a];
-                const int t = st[a];
-                double c = 0, s = 0;
-                if (q != 0.0) {
-                    entry_phase<double, double2>(T, T + KM, T + 2 * KM, kv.x, kv.y, kv.z, q, c, s);
-                    cC = cC + c; sC = sC + s;
-                }
-                if (t > 0) {
-                    double cl, sl;
-                    if (q != 0.0) { const double iq = 1.0 / q; cl = c * iq; sl = s * iq; }
-                    else entry_phase<double, double2>(T, T + KM, T + 2 * KM, kv.x, kv.y, kv.z, 1.0, cl, sl);
+            for (int k = 0; k < 8; ++k) y[k] = b + 64 * k < nb ? p[b + 64 * k] : 0.0;
 #pragma unroll
-                    for (int tt = 0; tt < NT; ++tt) {  // selects, not an indexed store: the sums stay in registers
-                        const bool hit = tt == t - 1;
-                        cL[tt] = hit ? cL[tt] + cl : cL[tt];
-                        sL[tt] = hit ? sL[tt] + sl : sL[tt];
-                    }
-                }
-            }
+            for (int k = 0; k < 8; ++k) x = flag ? fmax(x, y[k]) : x + y[k];
         }
-        __syncthreads();
     }
-    if (valid) {
-        const size_t ns = gridDim.y, s0 = blockIdx.y;
-        part[s0 * D.S + e] = make_double2(cC, sC);
 #pragma unroll
-        for (int t = 0; t < NT; ++t) part[((1 + t) * ns + s0) * D.S + e] = make_double2(cL[t], sL[t]);
+    for (int o = 16; o > 0; o >>= 1) {
+        const double y = __shfl_xor_sync(0xffffffffu, x, o);
+        x = flag ? fmax(x, y) : x + y;
     }
-}
-
-// rho[(t)*S + e] = sum over slices s in order of part[(t*nslice + s)*S + e], t over 1+nt rows
-__global__ void k_rho_reduce(const double2 *part, int nslice, int S, int nrow, double2 *rho) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= nrow * S) return;
-    const int t = idx / S, e = idx % S;
-    double c = 0, s = 0;
-    for (int k = 0; k < nslice; ++k) {
-        const double2 v = part[((size_t)t * nslice + k) * S + e];
-        c = c + v.x; s = s + v.y;
-    }
-    rho[idx] = make_double2(c, s);
+    if (t == 32) half[v] = x;
+    __syncthreads();
+    if (t == 0 && v < nv) out[v] = flag ? fmax(x, half[v]) : x + half[v];
 }
 
 // EwaldSumKSpace_calc_coulomb_energy / _calc_LJ_energy (EwaldSumKSpace.f90:389-526) per entry,
@@ -255,155 +122,7 @@ __global__ void __launch_bounds__(256) k_kspace_energy(DevSys D, const double2 *
             }
     }
     block_sum<256>(acc, 2, red);
-    if (threadIdx.x < 2) part[blockIdx.x * 2 + threadIdx.x] = acc[threadIdx.x];
-}
-
-// ------------------------------------------------------------------------------------------
-// adjoint: forces = -dE/dr of the implemented total energy
-// ------------------------------------------------------------------------------------------
-// Real space: one thread per atom i over the j tiles of one slice (blockIdx.y; tiles in shared
-// memory, increasing j), every pair inside the cutoff, intra-molecular pairs with the -erf_Luc
-// energy; F_i += FR (r_i - r_j).  Slices let a few thousand atoms fill the GPU: slice s writes
-// its partial forces to pf[(c * nslice + s) * N + i] (c = x, y, z), k_forces_reduce adds them.
-__global__ void __launch_bounds__(kFullTile) k_forces_real(DevSys D, int slice_tiles, double *pf) {
-    __shared__ double4 tp[kFullTile];
-    __shared__ int2 tm[kFullTile];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < D.N;
-    double4 pi = make_double4(0, 0, 0, 0);
-    int2 mi = make_int2(-1, 0);
-    if (valid) { pi = D.atom[i]; mi = D.meta[i]; }
-    double gx = 0, gy = 0, gz = 0;
-    const int nt = D.nt;
-    const int jbeg = blockIdx.y * slice_tiles * kFullTile, jend = min(D.N, jbeg + slice_tiles * kFullTile);
-    for (int t0 = jbeg; t0 < jend; t0 += kFullTile) {
-        const int j = t0 + threadIdx.x;
-        if (j < jend) { tp[threadIdx.x] = D.atom[j]; tm[threadIdx.x] = D.meta[j]; }
-        __syncthreads();
-        const int nj = min(kFullTile, jend - t0);
-        if (valid) {
-            for (int jj = 0; jj < nj; ++jj) {
-                if (t0 + jj == i) continue;
-                const double4 pj = tp[jj];
-                const int2 mj = tm[jj];
-                const double dx = min_image(pi.x - pj.x), dy = min_image(pi.y - pj.y), dz = min_image(pi.z - pj.z);
-                const double r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 >= D.rmax2) continue;
-                const bool lj = mi.y > 0 && mj.y > 0;
-                const int off = lj ? (mi.y - 1) * nt + (mj.y - 1) : 0;
-                const double FR = pair_force_adjoint<double>(r2, D.xclb * pi.w * pj.w, lj, lj ? D.lj_sig6[off] : 0.0,
-                                                             lj ? D.lj_feps[off] : 0.0, D.alpha, mi.x == mj.x);
-                gx = gx + dx * FR; gy = gy + dy * FR; gz = gz + dz * FR;
-            }
-        }
-        __syncthreads();
-    }
-    if (valid) {
-        const size_t ns = gridDim.y, s0 = blockIdx.y, N = D.N;
-        pf[(0 * ns + s0) * N + i] = gx; pf[(1 * ns + s0) * N + i] = gy; pf[(2 * ns + s0) * N + i] = gz;
-    }
-}
-
-// f{x,y,z}[i] = sum over slices in order of pf[(c * nslice + s) * N + i]
-__global__ void k_forces_reduce(const double *pf, int nslice, int N, double *fx, double *fy, double *fz) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    double g[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        double x = 0;
-        for (int k = 0; k < nslice; ++k) x = x + pf[((size_t)c * nslice + k) * N + i];
-        g[c] = x;
-    }
-    fx[i] = g[0]; fy[i] = g[1]; fz[i] = g[2];
-}
-
-// k space (ForceKSpace_coulomb / _LJ, ForceKSpace.f90:59-302, over the signed entries): one
-// warp per kForceAPW atoms, the lanes over the entries, so each entry's k, rho and beta rows are
-// loaded once for kForceAPW atoms; sin/cos(k r) come from the atoms' per-axis tables,
-// recomputed here instead of stored per atom and k.  Adds to fx/fy/fz.
-constexpr int kForceWarps = 8;  // warps per block
-constexpr int kForceAPW = 4;    // atoms per warp
-
-template <int NT>
-__global__ void __launch_bounds__(32 * kForceWarps, 2) k_forces_kspace(DevSys D, double *fx, double *fy, double *fz) {
-    extern __shared__ double2 ftab[];  // [kForceWarps][kForceAPW][3][KM]
-    const int KM = D.kmax + 1;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i0 = (blockIdx.x * kForceWarps + w) * kForceAPW;
-    if (i0 >= D.N) return;
-    const int na = min(kForceAPW, D.N - i0);
-    double2 *T = ftab + (size_t)w * kForceAPW * 3 * KM;
-    double q[kForceAPW], iq[kForceAPW];
-    int ta[kForceAPW];
-#pragma unroll
-    for (int a = 0; a < kForceAPW; ++a) {
-        q[a] = 0; iq[a] = 0; ta[a] = 0;
-        if (a < na) {
-            const double4 p = D.atom[i0 + a];
-            q[a] = p.w; iq[a] = p.w != 0.0 ? 1.0 / p.w : 0.0; ta[a] = D.meta[i0 + a].y;
-        }
-    }
-    for (int idx = lane; idx < na * 3 * KM; idx += 32) {
-        const int a = idx / (3 * KM), r = idx % (3 * KM), d = r / KM, m = r % KM;
-        const double4 p = D.atom[i0 + a];
-        const double u = d == 0 ? p.x : (d == 1 ? p.y : p.z);
-        double sn, cs;
-        sincospi(2.0 * (double)m * u, &sn, &cs);
-        if (m == 0) { sn = 0.0; cs = 1.0; }
-        T[idx] = make_double2(cs, sn);
-    }
-    __syncwarp();
-    const int S = D.S;
-    double gx[kForceAPW], gy[kForceAPW], gz[kForceAPW];
-#pragma unroll
-    for (int a = 0; a < kForceAPW; ++a) { gx[a] = 0; gy[a] = 0; gz[a] = 0; }
-    for (int e = lane; e < S; e += 32) {
-        const int4 kv = D.kvec[e];
-        const double2 C = D.rho[e];
-        const double be = D.ebeta[e];
-        double2 Ct[NT > 0 ? NT : 1];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) Ct[t] = D.rho[(size_t)(1 + t) * S + e];
-        double bl[NT * (NT + 1) / 2 > 0 ? NT * (NT + 1) / 2 : 1];
-#pragma unroll
-        for (int pr = 0; pr < NT * (NT + 1) / 2; ++pr) bl[pr] = D.ebetalj[(size_t)pr * S + e];
-#pragma unroll
-        for (int a = 0; a < kForceAPW; ++a) {
-            if (a >= na) break;
-            const double2 *Ta = T + (size_t)a * 3 * KM;
-            double c = 0, sn = 0, wgt = 0;
-            if (q[a] != 0.0) {
-                entry_phase<double, double2>(Ta, Ta + KM, Ta + 2 * KM, kv.x, kv.y, kv.z, q[a], c, sn);
-                wgt = be * (C.x * sn - C.y * c);
-            }
-            if (ta[a] > 0) {
-                double cl, sl;
-                if (q[a] != 0.0) { cl = c * iq[a]; sl = sn * iq[a]; }
-                else entry_phase<double, double2>(Ta, Ta + KM, Ta + 2 * KM, kv.x, kv.y, kv.z, 1.0, cl, sl);
-#pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    const int row = pair_idx<NT>(ta[a] - 1, t);
-                    double b = bl[0];  // selects, not an indexed load: bl stays in registers
-#pragma unroll
-                    for (int pr = 1; pr < NT * (NT + 1) / 2; ++pr) b = row == pr ? bl[pr] : b;
-                    wgt += b * (Ct[t].x * sl - Ct[t].y * cl);
-                }
-            }
-            const double f = kFourPi * wgt;
-            gx[a] = gx[a] + f * kv.x; gy[a] = gy[a] + f * kv.y; gz[a] = gz[a] + f * kv.z;
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < kForceAPW; ++a) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            gx[a] += __shfl_xor_sync(0xffffffffu, gx[a], o);
-            gy[a] += __shfl_xor_sync(0xffffffffu, gy[a], o);
-            gz[a] += __shfl_xor_sync(0xffffffffu, gz[a], o);
-        }
-        if (lane == 0 && a < na) { fx[i0 + a] += gx[a]; fy[i0 + a] += gy[a]; fz[i0 + a] += gz[a]; }
-    }
+    if (threadIdx.x < 2) part[threadIdx.x * gridDim.x + blockIdx.x] = acc[threadIdx.x];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -457,7 +176,7 @@ __global__ void __launch_bounds__(256) k_xchg_real(DevSys D, XchgIn X, double *p
         }
     }
     block_sum<256>(acc, kXParts, red);
-    if (threadIdx.x < kXParts) part[(size_t)blockIdx.x * kXParts + threadIdx.x] = acc[threadIdx.x];
+    if (threadIdx.x < kXParts) part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = acc[threadIdx.x];
 }
 
 // k space: per signed entry the structure factors of both molecules at the new positions minus
@@ -533,7 +252,7 @@ __global__ void __launch_bounds__(256) k_xchg_kspace(DevSys D, XchgIn X, double2
         }
     }
     block_sum<256>(acc, 2, red);
-    if (threadIdx.x < 2) part[(size_t)blockIdx.x * 2 + threadIdx.x] = acc[threadIdx.x];
+    if (threadIdx.x < 2) part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = acc[threadIdx.x];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -798,6 +517,23 @@ int dalloc(T **p, size_t n) {
     return YAMC_OK;
 }
 
+// Device arrays allocated together: add() each array, then commit() makes one allocation and sets
+// the pointers (an allocation costs about 0.1 ms, whatever its size).
+struct DeviceArena {
+    std::vector<std::pair<void **, size_t>> want;  // pointer to set, offset
+    size_t bytes = 0;
+    template <class T>
+    void add(T **p, size_t n) {
+        want.push_back({(void **)p, bytes});
+        bytes += (sizeof(T) * std::max<size_t>(n, 1) + 255) / 256 * 256;
+    }
+    int commit(char **base) {
+        if (const int r = dalloc(base, bytes)) return r;
+        for (const auto &w : want) *w.first = *base + w.second;
+        return YAMC_OK;
+    }
+};
+
 template <class T>
 int upload(T *d, const T *h, size_t n, cudaStream_t s) {
     if (n) CUDA_TRY(cudaMemcpyAsync(d, h, n * sizeof(T), cudaMemcpyHostToDevice, s));
@@ -821,13 +557,22 @@ size_t chain_smem_bytes(int G, int B, int kmax, int nt, int nown_max, int qcap) 
 
 }  // namespace
 
+// Points in spatial tiles: position -> point, a bounding box per tile (k_sort_*, k_tile_boxes)
+struct SpatialOrder {
+    char *base = nullptr;  // its own allocation (null: the arrays belong to an arena)
+    int n = 0, nc = 1, chunk = 0, nblock = 0, ntile = 0;
+    int *order = nullptr, *hist = nullptr, *total = nullptr;
+    float4 *box = nullptr;
+};
+
 struct yamc_ctx {
     HostSystem H;
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_ms = 0.f;
-    // device state
+    // device state: the arrays of yamc_create in one allocation, others when first needed
+    char *arena = nullptr;
     double4 *atom = nullptr;
     int2 *meta = nullptr, *mol = nullptr;
     double *dhs = nullptr, *mass = nullptr, *ebeta = nullptr, *ebetalj = nullptr, *lj_sig6 = nullptr, *lj_feps = nullptr;
@@ -844,10 +589,13 @@ struct yamc_ctx {
     int4 *spec = nullptr;
     int *slot = nullptr, *atom_of = nullptr;  // the chain kernel's staging order (k_stage_order)
     double *part = nullptr, *sums = nullptr;  // block partials of the full sums, their totals
-    int2 *tpairs = nullptr;                    // atom-tile pairs of the real-space full sum
-    int ntpairs = 0;
+    SpatialOrder tiles;                        // the atoms in spatial tiles (full sums, adjoint)
+    // the k grid by rows (k_rho_rows, k_forces_rows): items, entry maps, atom lists and their slices
+    int4 *k_items = nullptr, *k_emap = nullptr, *k_slices = nullptr, *k_frows = nullptr, *k_fmap = nullptr;
+    int2 *k_place = nullptr;
+    int *k_alist = nullptr, *k_sbeg = nullptr;
+    int k_nitem = 0, k_threads = 0, k_nslice = 0, k_nfrow = 0, k_nf = 0, k_npos = 0, k_lbeg[kMaxLists + 1] = {};
     double2 *rho_part = nullptr;               // per-slice rho(k) sums of the full recompute
-    int rho_slices = 1, rho_slice_atoms = 0;
     int nsm = 148;                             // SMs of the device
     DevSys hsys{};
     DevSys *d_sys = nullptr;
@@ -881,8 +629,9 @@ struct yamc_ctx {
     double api_dmu[3] = {};
     long long *d_prof = nullptr;
     bool prof_on = false;
-    double *d_gx = nullptr, *d_gy = nullptr, *d_gz = nullptr;  // adjoint forces
-    double *d_fpart = nullptr;                                  // their per-slice real-space parts
+    double *d_f = nullptr;                                      // adjoint forces [3][N]
+    double *d_gf = nullptr, *d_kf = nullptr;                    // their real-space parts; k-space forces by list position
+    double4 *d_field = nullptr;                                 // the k-space fields they sum
     // NPT volume move: rho(k) as it was before the step, accepted volume steps
     double2 *rho_save = nullptr;
     double n_vol_accepted = 0;
@@ -1056,17 +805,165 @@ int launch_chain(yamc_ctx *c, const ChainArgs &args) {
                             args);
 }
 
-template <int NT>
-int launch_rho_full(yamc_ctx *c) {
-    const int KM = c->H.kmax + 1;
-    const size_t sm = sizeof(double2) * kRhoChunk * 3 * KM;
-    CUDA_TRY(cudaFuncSetAttribute(k_rho_full<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    const dim3 grid((c->H.S + kRhoBlock - 1) / kRhoBlock, c->rho_slices);
-    k_rho_full<NT><<<grid, kRhoBlock, sm, c->stream>>>(c->hsys, c->rho_slice_atoms, c->rho_part);
+// sizes and buffers of the spatial order of n points
+void spatial_plan(SpatialOrder &o, int n, DeviceArena &arena) {
+    o.n = n;
+    o.nc = sort_cells(n);
+    o.chunk = std::max(kSortChunk, (((n + kSortBlocks - 1) / kSortBlocks) + 31) / 32 * 32);
+    o.nblock = (n + o.chunk - 1) / o.chunk;
+    o.ntile = (n + kTile - 1) / kTile;
+    const size_t ncell = (size_t)o.nc * o.nc * o.nc;
+    arena.add(&o.order, n);
+    arena.add(&o.hist, o.nblock * ncell);
+    arena.add(&o.total, ncell);
+    arena.add(&o.box, (size_t)2 * 5 * o.ntile);
+}
+
+// (each sort leaves the totals at 0)
+int spatial_reset(const SpatialOrder &o, cudaStream_t stream) {
+    CUDA_TRY(cudaMemsetAsync(o.total, 0, sizeof(int) * o.nc * o.nc * o.nc, stream));
+    return YAMC_OK;
+}
+
+// the order and the boxes of the points as they stand
+int spatial_order(const SpatialOrder &o, const Points &P, cudaStream_t stream) {
+    const int ncell = o.nc * o.nc * o.nc;
+    const size_t smem = sizeof(int) * ((size_t)ncell + o.chunk);
+    if (smem > 48 * 1024)
+        CUDA_TRY(cudaFuncSetAttribute(k_sort_place, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_sort_count<<<o.nblock, kSortThreads, 0, stream>>>(P, o.nc, o.chunk, o.hist, o.total);
+    k_sort_scan<<<(ncell + 255) / 256, 256, 0, stream>>>(o.total, o.hist, o.nblock, ncell);
+    k_sort_place<<<o.nblock, kSortThreads, smem, stream>>>(P, o.nc, o.chunk, o.hist, o.total, o.order);
+    k_tile_boxes<<<(o.ntile + 7) / 8, 256, 0, stream>>>(P, o.order, o.ntile, o.box);
     CUDA_TRY(cudaGetLastError());
-    const int n = (1 + NT) * c->H.S;
-    k_rho_reduce<<<(n + 255) / 256, 256, 0, c->stream>>>(c->rho_part, c->rho_slices, c->H.S, 1 + NT, c->rho);
+    return YAMC_OK;
+}
+
+int order_atoms(yamc_ctx *c) {
+    const double *a = reinterpret_cast<const double *>(c->atom);
+    return spatial_order(c->tiles, Points{a, a + 1, a + 2, 4, c->H.N}, c->stream);
+}
+
+// squared reach of the tile pairs, box units: the pairs of two tiles farther apart (any periodic
+// image) are outside the cutoff (widened beyond the rounding of the distance)
+double tile_reach2(double reach) { return reach * reach * (1.0 + 1e-9); }
+
+// shares of a tile's near tiles (blockIdx.y): enough blocks of kRealWarps warps for about twelve per SM
+int tile_shares(int ntile, int nsm) { return std::max(1, std::min(16, (12 * nsm + ntile - 1) / ntile)); }
+
+AtomLists atom_lists(const yamc_ctx *c) {
+    AtomLists L;
+    L.alist = c->k_alist;
+    std::copy(c->k_lbeg, c->k_lbeg + kMaxLists + 1, L.lbeg);
+    return L;
+}
+
+int launch_rho(yamc_ctx *c) {
+    const HostSystem &H = c->H;
+    const size_t sm = sizeof(double2) * (3 * (H.kmax + 1) + kRowZ) * (kRhoChunk + 1);
+    CUDA_TRY(cudaFuncSetAttribute(k_rho_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    const dim3 grid((c->k_nitem + c->k_threads - 1) / c->k_threads, c->k_nslice);
+    k_rho_rows<<<grid, c->k_threads, sm, c->stream>>>(c->hsys, atom_lists(c), c->k_slices, c->k_items, c->k_emap, c->k_nitem,
+                                                      c->rho_part);
     CUDA_TRY(cudaGetLastError());
+    k_rho_reduce<<<dim3((H.S + 31) / 32, 1 + H.nt), 256, 0, c->stream>>>(c->rho_part, c->k_sbeg, H.S, c->rho);
+    CUDA_TRY(cudaGetLastError());
+    return YAMC_OK;
+}
+
+// the k grid by rows, the atom lists and the slices of the structure-factor sums (host side; their
+// sizes to the context and their arrays to the arena)
+struct RowTables {
+    std::vector<int4> items, emap, frows, fmap, slices;
+    std::vector<int2> place;
+    std::vector<int> alist, sbeg;
+};
+void plan_rows(yamc_ctx *c, RowTables &T, DeviceArena &arena) {
+    const HostSystem &H = c->H;
+    const int km = H.kmax, w = 2 * km + 1;
+    std::vector<int> at((size_t)(km + 1) * w * w, -1);  // entry of (kx, ky, kz)
+    auto entry = [&](int kx, int ky, int kz) -> int & { return at[((size_t)kx * w + ky + km) * w + kz + km]; };
+    for (int e = 0; e < H.S; ++e) entry(H.ekx[e], H.eky[e], H.ekz[e]) = e;
+    auto nz = [&](int kx, int ky) {  // kz = 0 .. nz - 1 of the row (kz = 0 is missing at kx = ky = 0)
+        int n = (kx == 0 && ky == 0) || entry(kx, ky, 0) >= 0 ? 1 : 0;
+        if (n) while (n <= km && entry(kx, ky, n) >= 0) ++n;
+        return n;
+    };
+    std::vector<int4> &items = T.items, &emap = T.emap, &frows = T.frows, &fmap = T.fmap, &slices = T.slices;
+    std::vector<int> &alist = T.alist, &sbeg = T.sbeg;
+    std::vector<int2> &place = T.place;
+    // the four signed entries of (kx, +-ky, +-kz), -1 where there is none
+    auto signs = [&](int kx, int ky, int kz) {
+        return make_int4(entry(kx, ky, kz), kz ? entry(kx, ky, -kz) : -1, ky ? entry(kx, -ky, kz) : -1,
+                         ky && kz ? entry(kx, -ky, -kz) : -1);
+    };
+    for (int z0 = 0; z0 <= km; z0 += kRowZ)  // items of one z0 together: a warp shares its kz factors
+        for (int kx = 0; kx <= km; ++kx)
+            for (int ky = 0; ky <= km; ++ky) {
+                const int n = std::min(nz(kx, ky) - z0, kRowZ);
+                if (n <= 0) continue;
+                items.push_back(make_int4(kx, ky, z0, n));
+                for (int j = 0; j < kRowZ; ++j) emap.push_back(j < n ? signs(kx, ky, z0 + j) : make_int4(-1, -1, -1, -1));
+            }
+    for (int kx = 0; kx <= km; ++kx)
+        for (int ky = 0; ky <= km; ++ky) {
+            const int n = nz(kx, ky);
+            if (n <= 0) continue;
+            frows.push_back(make_int4(kx, ky, (int)fmap.size(), n));
+            for (int kz = 0; kz < n; ++kz) fmap.push_back(signs(kx, ky, kz));
+        }
+    c->k_nitem = (int)items.size();
+    c->k_nfrow = (int)frows.size();
+    c->k_nf = (int)fmap.size();
+    // items per block: one block of up to kRhoMaxThreads, or as many even ones as that takes
+    const int nib = (c->k_nitem + kRhoMaxThreads - 1) / kRhoMaxThreads;
+    c->k_threads = ((c->k_nitem + nib - 1) / nib + 31) / 32 * 32;
+    // the atom lists: charged atoms, then the atoms of each LJ type
+    place.assign(H.N, make_int2(-1, -1));
+    int nl = 1 + H.nt;
+    for (int l = 0; l < nl; ++l) {
+        c->k_lbeg[l] = (int)alist.size();
+        for (int i = 0; i < H.N; ++i)
+            if (l == 0 ? H.q[i] != 0.0 : H.type_by_index[i] == l) {
+                (l == 0 ? place[i].x : place[i].y) = (int)alist.size();
+                alist.push_back(i);
+            }
+        while (alist.size() % 32) alist.push_back(-1);
+    }
+    for (int l = nl; l <= kMaxLists; ++l) c->k_lbeg[l] = (int)alist.size();
+    c->k_npos = (int)alist.size();
+    // slices of whole 32-atom chunks: as many as one wave of blocks holds (the SMs take
+    // kRhoMaxThreads threads each), or four waves when the item blocks alone pass one
+    const int slots = c->nsm * std::max(1, kRhoMaxThreads / c->k_threads), target = nib * nl > slots ? 4 * slots : slots;
+    for (int per = 1;; ++per) {  // chunks per slice
+        int n = 0;
+        for (int l = 0; l < nl; ++l) n += ((c->k_lbeg[l + 1] - c->k_lbeg[l]) / 32 + per - 1) / per;
+        if ((long long)n * nib > target && per < c->k_npos / 32) continue;
+        for (int l = 0; l < nl; ++l) {
+            sbeg.push_back((int)slices.size());
+            for (int p = c->k_lbeg[l]; p < c->k_lbeg[l + 1]; p += 32 * per)
+                slices.push_back(make_int4(l, p, std::min(p + 32 * per, c->k_lbeg[l + 1]), 0));
+        }
+        sbeg.push_back((int)slices.size());
+        break;
+    }
+    c->k_nslice = (int)slices.size();
+    arena.add(&c->k_items, items.size()); arena.add(&c->k_emap, emap.size()); arena.add(&c->k_frows, frows.size());
+    arena.add(&c->k_fmap, fmap.size()); arena.add(&c->k_slices, slices.size()); arena.add(&c->k_alist, alist.size());
+    arena.add(&c->k_place, place.size()); arena.add(&c->k_sbeg, sbeg.size());
+    arena.add(&c->rho_part, (size_t)c->k_nslice * H.S);
+}
+int upload_rows(yamc_ctx *c, const RowTables &T) {
+    int r;
+    if ((r = upload(c->k_items, T.items.data(), T.items.size(), c->stream)) ||
+        (r = upload(c->k_emap, T.emap.data(), T.emap.size(), c->stream)) ||
+        (r = upload(c->k_frows, T.frows.data(), T.frows.size(), c->stream)) ||
+        (r = upload(c->k_fmap, T.fmap.data(), T.fmap.size(), c->stream)) ||
+        (r = upload(c->k_slices, T.slices.data(), T.slices.size(), c->stream)) ||
+        (r = upload(c->k_alist, T.alist.data(), T.alist.size(), c->stream)) ||
+        (r = upload(c->k_place, T.place.data(), T.place.size(), c->stream)) ||
+        (r = upload(c->k_sbeg, T.sbeg.data(), T.sbeg.size(), c->stream)))
+        return r;
     return YAMC_OK;
 }
 
@@ -1107,9 +1004,12 @@ int full_sums(yamc_ctx *c, int *overlap = nullptr) {
     HostSystem &H = c->H;
     int r = sync_positions(c);
     if (r) return r;
-    k_realspace_full<<<c->ntpairs, kFullTile, 0, c->stream>>>(c->hsys, c->tpairs, c->part);
+    if ((r = order_atoms(c))) return r;
+    const int shares = tile_shares(c->tiles.ntile, c->nsm);
+    k_real_energy<<<dim3(c->tiles.ntile, shares), 32 * kRealWarps, 0, c->stream>>>(
+        c->hsys, c->tiles.order, c->tiles.box, c->tiles.ntile, tile_reach2(c->hsys.rpre), c->part);
     CUDA_TRY(cudaGetLastError());
-    k_sum_parts<<<1, kSumThreads, 0, c->stream>>>(c->part, c->ntpairs, kFullParts, 6, c->sums);
+    k_sum_parts<<<1, kSumThreads, 0, c->stream>>>(c->part, c->tiles.ntile * shares, kFullParts, 6, c->sums);
     CUDA_TRY(cudaGetLastError());
     double tot[kFullParts] = {};
     CUDA_TRY(cudaMemcpyAsync(tot, c->sums, sizeof(tot), cudaMemcpyDeviceToHost, c->stream));
@@ -1118,14 +1018,8 @@ int full_sums(yamc_ctx *c, int *overlap = nullptr) {
         if (!std::isfinite(tot[v])) { set_error("non-finite real-space sum"); return YAMC_ENAN; }
     if (overlap) *overlap = tot[6] > 0;
     else if (tot[6] > 0) { set_error("hard-core overlap in the configuration"); return YAMC_EOVERLAP_INIT; }
-    switch (H.nt) {
-        case 1: r = launch_rho_full<1>(c); break;
-        case 2: r = launch_rho_full<2>(c); break;
-        case 3: r = launch_rho_full<3>(c); break;
-        case 4: r = launch_rho_full<4>(c); break;
-        default: set_error("LJ type count outside 1..4"); return YAMC_ELIMITS;
-    }
-    if (r) return r;
+    if (H.nt < 1 || H.nt > 4) { set_error("LJ type count outside 1..4"); return YAMC_ELIMITS; }
+    if ((r = launch_rho(c))) return r;
     const int nbk = (H.S + 255) / 256;
     switch (H.nt) {
         case 1: r = launch_kspace_energy<1>(c, nbk); break;
@@ -1167,13 +1061,30 @@ int ensure_cfg(yamc_ctx *c) {
     return pick_launch(c, &c->cfg);
 }
 
+// the adjoint's device forces, real space and k space, into c->d_f
 template <int NT>
-int launch_forces_kspace(yamc_ctx *c) {
-    const size_t sm = sizeof(double2) * kForceWarps * kForceAPW * 3 * (c->H.kmax + 1);
-    const int per_block = kForceWarps * kForceAPW;
-    CUDA_TRY(cudaFuncSetAttribute(k_forces_kspace<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_forces_kspace<NT><<<(c->H.N + per_block - 1) / per_block, 32 * kForceWarps, sm, c->stream>>>(c->hsys, c->d_gx,
-                                                                                                      c->d_gy, c->d_gz);
+int launch_forces(yamc_ctx *c) {
+    const HostSystem &H = c->H;
+    const size_t sm = sizeof(double2) * 32 * 3 * (H.kmax + 1), smr = sizeof(double) * kRealWarps * 3 * kForceBatch;
+    const int nblk = c->k_npos / 32, shares = tile_shares(c->tiles.ntile, c->nsm);
+    // the row pairs split over blockIdx.y until the blocks fill the GPU about four times
+    const int nsplit = std::max(1, std::min((4 * c->nsm + nblk - 1) / nblk, (c->k_nfrow + kForceRowWarps - 1) / kForceRowWarps));
+    int r;
+    if (!c->d_f && ((r = dalloc(&c->d_gf, (size_t)3 * shares * H.N)) || (r = dalloc(&c->d_kf, (size_t)3 * nsplit * c->k_npos)) ||
+                    (r = dalloc(&c->d_field, (size_t)2 * (1 + NT) * c->k_nf)) || (r = dalloc(&c->d_f, (size_t)3 * H.N))))
+        return r;
+    CUDA_TRY(cudaFuncSetAttribute(k_real_forces, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smr));
+    k_real_forces<<<dim3(c->tiles.ntile, shares), 32 * kRealWarps, smr, c->stream>>>(
+        c->hsys, c->tiles.order, c->tiles.box, c->tiles.ntile, tile_reach2(std::sqrt(c->hsys.rmax2)), c->d_gf);
+    CUDA_TRY(cudaGetLastError());
+    k_row_fields<NT><<<dim3((c->k_nf + 255) / 256, 1 + NT), 256, 0, c->stream>>>(c->hsys, c->k_fmap, c->k_nf, c->d_field);
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaFuncSetAttribute(k_forces_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_forces_rows<<<dim3(nblk, nsplit), 32 * kForceRowWarps, sm, c->stream>>>(c->hsys, atom_lists(c), c->k_frows, c->k_nfrow,
+                                                                              c->d_field, c->k_nf, c->k_npos, c->d_kf);
+    CUDA_TRY(cudaGetLastError());
+    k_forces_add<<<(H.N + 255) / 256, 256, 0, c->stream>>>(c->hsys, c->k_place, c->d_gf, shares, c->d_kf, c->k_npos, nsplit,
+                                                           c->d_f);
     CUDA_TRY(cudaGetLastError());
     return YAMC_OK;
 }
@@ -1448,47 +1359,37 @@ static int create_impl(yamc_ctx *c, const yamc_system *sys, const yamc_params *p
     CUDA_TRY(cudaEventCreate(&c->ev0));
     CUDA_TRY(cudaEventCreate(&c->ev1));
     const int N = H.N, M = H.M, S = H.S, nt = H.nt;
-    if ((r = dalloc(&c->atom, N)) || (r = dalloc(&c->meta, N)) || (r = dalloc(&c->dhs, N)) || (r = dalloc(&c->mass, N)) ||
-        (r = dalloc(&c->mol, M)) || (r = dalloc(&c->kvec, S)) || (r = dalloc(&c->kpack, S)) ||
-        (r = dalloc(&c->rho_f, (size_t)(1 + nt) * S)) || (r = dalloc(&c->d_check, 1)) || (r = dalloc(&c->ebeta, S)) ||
-        (r = dalloc(&c->ebeta_f, S)) || (r = dalloc(&c->ebetalj_f, (size_t)H.npair * S)) ||
-        (r = dalloc(&c->ebetalj, (size_t)H.npair * S)) || (r = dalloc(&c->pair_index, nt * nt)) ||
-        (r = dalloc(&c->lj_sig6, nt * nt)) || (r = dalloc(&c->lj_feps, nt * nt)) || (r = dalloc(&c->rho, (size_t)(1 + nt) * S)) ||
-        (r = dalloc(&c->scratch, (size_t)2 * (1 + nt) * S)) || (r = dalloc(&c->freq_beg, M)) || (r = dalloc(&c->freq_end, M)) ||
-        (r = dalloc(&c->scal, SC_COUNT)) || (r = dalloc(&c->cnt, CN_COUNT)) ||
-        (r = dalloc(&c->d_sys, 1)) || (r = dalloc(&c->d_run, 1)) || (r = dalloc(&c->slot, N)) ||
-        (r = dalloc(&c->atom_of, (size_t)N + 16)) || (r = dalloc(&c->spec, H.spec.size() / 4)))
-        return r;
+    int nsm = 148;
+    CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+    c->nsm = nsm;
+    if (H.kmax > 127) { set_error("kmax above 127 (the packed k of the chain kernel holds 8 bits per component)"); return YAMC_ELIMITS; }
+    RowTables rows;
+    {
+        DeviceArena arena;
+        arena.add(&c->atom, N); arena.add(&c->meta, N); arena.add(&c->dhs, N); arena.add(&c->mass, N);
+        arena.add(&c->mol, M); arena.add(&c->kvec, S); arena.add(&c->kpack, S);
+        arena.add(&c->rho_f, (size_t)(1 + nt) * S); arena.add(&c->d_check, 1); arena.add(&c->ebeta, S);
+        arena.add(&c->ebeta_f, S); arena.add(&c->ebetalj_f, (size_t)H.npair * S);
+        arena.add(&c->ebetalj, (size_t)H.npair * S); arena.add(&c->pair_index, nt * nt);
+        arena.add(&c->lj_sig6, nt * nt); arena.add(&c->lj_feps, nt * nt); arena.add(&c->rho, (size_t)(1 + nt) * S);
+        arena.add(&c->scratch, (size_t)2 * (1 + nt) * S); arena.add(&c->freq_beg, M); arena.add(&c->freq_end, M);
+        arena.add(&c->scal, SC_COUNT); arena.add(&c->cnt, CN_COUNT);
+        arena.add(&c->d_sys, 1); arena.add(&c->d_run, 1); arena.add(&c->slot, N);
+        arena.add(&c->atom_of, (size_t)N + 16); arena.add(&c->spec, H.spec.size() / 4);
+        spatial_plan(c->tiles, N, arena);
+        plan_rows(c, rows, arena);
+        // block partials: the real-space sum's tiles, the k-space energy blocks and the exchange
+        // step's atom blocks (kXParts each); the totals of any of them
+        arena.add(&c->part, std::max({(size_t)c->tiles.ntile * tile_shares(c->tiles.ntile, nsm) * kFullParts,
+                                      (size_t)(S + 255) / 256 * 2, (size_t)(N + 255) / 256 * kXParts}));
+        arena.add(&c->sums, std::max(kFullParts + 2, kXParts));
+        if ((r = arena.commit(&c->arena))) return r;
+    }
     CUDA_TRY(cudaHostAlloc(&c->h_out, sizeof(double) * (kNV + SC_COUNT) + sizeof(long long) * (CN_COUNT + 1),
                            cudaHostAllocMapped));
     move_pass_done(c) = 0;
     CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&c->d_hout), c->h_out, 0));
-    // full-sum work split: atom-tile pairs of the real-space sum; atom slices of rho(k) so that
-    // entry blocks x slices cover the SMs about twice
-    int nsm = 148;
-    CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-    c->nsm = nsm;
-    {
-        const int T = (N + kFullTile - 1) / kFullTile;
-        std::vector<int2> tp;
-        tp.reserve((size_t)T * (T + 1) / 2);
-        for (int ti = 0; ti < T; ++ti)
-            for (int tj = ti; tj < T; ++tj) tp.push_back(make_int2(ti, tj));
-        c->ntpairs = (int)tp.size();
-        const int eb = (S + kRhoBlock - 1) / kRhoBlock;
-        const int chunks = (N + kRhoChunk - 1) / kRhoChunk;
-        const int want = std::max(1, std::min(chunks, (2 * nsm + eb - 1) / eb));
-        c->rho_slice_atoms = ((chunks + want - 1) / want) * kRhoChunk;
-        c->rho_slices = (N + c->rho_slice_atoms - 1) / c->rho_slice_atoms;
-        if ((r = dalloc(&c->tpairs, tp.size())) || (r = upload(c->tpairs, tp.data(), tp.size(), c->stream)) ||
-            // block partials: the full sums' tile pairs, the k-space energy blocks and the
-            // exchange step's atom blocks (kXParts each); the totals of any of them
-            (r = dalloc(&c->part, std::max({(size_t)c->ntpairs * kFullParts, (size_t)(S + 255) / 256 * 2,
-                                            (size_t)(N + 255) / 256 * kXParts}))) ||
-            (r = dalloc(&c->sums, std::max(kFullParts + 2, kXParts))) ||
-            (r = dalloc(&c->rho_part, (size_t)(1 + nt) * c->rho_slices * S)))
-            return r;
-    }
+    if ((r = spatial_reset(c->tiles, c->stream)) || (r = upload_rows(c, rows))) return r;
     std::vector<double4> a(N);
     std::vector<int2> m(N);
     for (int i = 0; i < N; ++i) { a[i] = make_double4(H.x[i], H.y[i], H.z[i], H.q[i]); m[i] = make_int2(H.molnum[i], H.type_by_index[i]); }
@@ -1496,7 +1397,6 @@ static int create_impl(yamc_ctx *c, const yamc_system *sys, const yamc_params *p
     for (int i = 0; i < M; ++i) mo[i] = make_int2(H.first[i], H.natoms[i]);
     std::vector<int4> kv(S);
     for (int e = 0; e < S; ++e) kv[e] = make_int4(H.ekx[e], H.eky[e], H.ekz[e], H.ekk[e]);
-    if (H.kmax > 127) { set_error("kmax above 127 (the packed k of the chain kernel holds 8 bits per component)"); return YAMC_ELIMITS; }
     std::vector<int> kp(S);
     for (int e = 0; e < S; ++e) kp[e] = H.ekx[e] | ((H.eky[e] + 128) << 8) | ((H.ekz[e] + 128) << 16);
     std::vector<int> pidx(nt * nt);
@@ -1554,12 +1454,8 @@ int yamc_destroy(yamc_ctx *c) {
     if (!c) return YAMC_OK;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    void *ptrs[] = {c->atom, c->meta, c->mol, c->dhs, c->mass, c->ebeta, c->ebetalj, c->ebeta_f, c->ebetalj_f,
-                    c->lj_sig6, c->lj_feps, c->kvec, c->kpack, c->rho_f, c->d_check,
-                    c->pair_index, c->rho, c->scratch, c->freq_beg, c->freq_end, c->scal, c->cnt, c->part, c->sums,
-                    c->tpairs, c->rho_part, c->d_sys, c->d_run, c->d_rng, c->d_log, c->d_rows,
-                    c->d_prof, c->spec, c->d_gx, c->d_gy, c->d_gz, c->d_fpart, c->rho_save, c->d_mpart,
-                    c->d_mcount, c->slot, c->atom_of};
+    void *ptrs[] = {c->arena, c->d_rng, c->d_log, c->d_rows, c->d_prof, c->d_f, c->d_gf, c->d_kf, c->d_field, c->rho_save,
+                    c->d_mpart, c->d_mcount};
     for (void *p : ptrs) if (p) cudaFree(p);
     if (c->h_out) cudaFreeHost(c->h_out);
     if (c->ev0) cudaEventDestroy(c->ev0);
@@ -2183,12 +2079,27 @@ struct yamc_rdf {
     int *type = nullptr;
     double *cx = nullptr, *cy = nullptr, *cz = nullptr;
     unsigned long long *hist = nullptr;  // [ntypes^2][nbin] counts, then [ntypes^2] pair totals
+    SpatialOrder tiles;                  // the centres in spatial tiles
+    bool tile_path = false;              // enough centres, and the histogram leaves room for the tiles
+    int tile_grid = 1, tile_split = 1;
 };
+
+// From this many centres a frame without periodic images goes over near tiles: the sort's four
+// launches and the tiles' tests cost about 15 us, which all M^2 pairs pass at about a thousand centres
+constexpr int kRdfTileMin = 1024;
+constexpr size_t kRdfTileStatic = 40 * 1024;  // k_rdf_tiles' own shared memory beside the histogram
 
 static int rdf_frame(yamc_rdf *h, double L) {
     const int nbox = h->rmax < L / 2 ? 0 : (int)((h->rmax - L / 2) / L) + 1;  // mcrdf2.f90:206-210
-    k_rdf_count<<<h->grid, 256, h->smem, h->stream>>>(h->cx, h->cy, h->cz, h->type, h->M, h->ntypes, h->nbin, L, h->dr,
-                                                      h->rmax * h->rmax, nbox, h->hist);
+    if (nbox == 0 && h->tile_path) {
+        if (const int r = spatial_order(h->tiles, Points{h->cx, h->cy, h->cz, 1, h->M}, h->stream)) return r;
+        k_rdf_tiles<<<dim3(h->tile_grid, h->tile_split), 256, h->smem, h->stream>>>(h->cx, h->cy, h->cz, h->type, h->tiles.order, h->tiles.box,
+                                                               h->tiles.ntile, tile_reach2(h->rmax / L), h->M, h->ntypes,
+                                                               h->nbin, L, h->dr, h->rmax * h->rmax, h->hist);
+    } else {
+        k_rdf_count<<<h->grid, 256, h->smem, h->stream>>>(h->cx, h->cy, h->cz, h->type, h->M, h->ntypes, h->nbin, L, h->dr,
+                                                          h->rmax * h->rmax, nbox, h->hist);
+    }
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     h->n_frame += 1;
@@ -2202,6 +2113,7 @@ int yamc_rdf_destroy(yamc_rdf *h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     void *ptrs[] = {h->type, h->cx, h->cy, h->cz, h->hist};
     for (void *p : ptrs) if (p) cudaFree(p);
+    if (h->tiles.base) cudaFree(h->tiles.base);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return YAMC_OK;
@@ -2222,9 +2134,20 @@ static int rdf_create_impl(yamc_rdf *h, int32_t nmol, const int32_t *mol_type, i
     CUDA_TRY(cudaGetDeviceProperties(&prop, device));
     if (h->smem > prop.sharedMemPerBlockOptin) { set_error("too many RDF bins x species pairs for one block's histogram"); return YAMC_ELIMITS; }
     CUDA_TRY(cudaFuncSetAttribute(k_rdf_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem));
+    h->tile_path = nmol >= kRdfTileMin && h->smem + kRdfTileStatic <= prop.sharedMemPerBlockOptin;
+    if (h->tile_path) {
+        CUDA_TRY(cudaFuncSetAttribute(k_rdf_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem));
+        DeviceArena arena;
+        spatial_plan(h->tiles, nmol, arena);
+        if (const int r = arena.commit(&h->tiles.base)) return r;
+        h->tile_grid = std::min(h->tiles.ntile, 4 * prop.multiProcessorCount);
+        h->tile_split = std::min(4, tile_shares(h->tiles.ntile, prop.multiProcessorCount));
+    }
     const long long pairs = (long long)nmol * nmol;
     h->grid = (int)std::max(1LL, std::min((pairs + 255) / 256, 4LL * prop.multiProcessorCount));
     CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
+    if (h->tile_path)
+        if (const int r = spatial_reset(h->tiles, h->stream)) return r;
     int r;
     if ((r = dalloc(&h->type, nmol)) || (r = dalloc(&h->cx, nmol)) || (r = dalloc(&h->cy, nmol)) || (r = dalloc(&h->cz, nmol)) ||
         (r = dalloc(&h->hist, nh)) || (r = upload(h->type, mol_type, nmol, h->stream)))
@@ -2965,30 +2888,18 @@ int yamc_forces(yamc_ctx *c, double *fx, double *fy, double *fz, double *mol_f, 
     HostSystem &H = c->H;
     const int N = H.N;
     int r;
-    // real space over atom tiles x j slices (about two blocks per SM), the slices added in order
-    const int T = (N + kFullTile - 1) / kFullTile;
-    const int want = std::max(1, std::min(T, (2 * c->nsm + T - 1) / T));
-    const int slice_tiles = (T + want - 1) / want, nslice = (T + slice_tiles - 1) / slice_tiles;
-    if (!c->d_gx && ((r = dalloc(&c->d_gx, N)) || (r = dalloc(&c->d_gy, N)) || (r = dalloc(&c->d_gz, N)) ||
-                     (r = dalloc(&c->d_fpart, (size_t)3 * nslice * N))))
-        return r;
-    if ((r = sync_positions(c)) || (r = pull_state(c))) return r;
-    k_forces_real<<<dim3(T, nslice), kFullTile, 0, c->stream>>>(c->hsys, slice_tiles, c->d_fpart);
-    CUDA_TRY(cudaGetLastError());
-    k_forces_reduce<<<(N + 255) / 256, 256, 0, c->stream>>>(c->d_fpart, nslice, N, c->d_gx, c->d_gy, c->d_gz);
-    CUDA_TRY(cudaGetLastError());
+    if ((r = sync_positions(c)) || (r = pull_state(c)) || (r = order_atoms(c))) return r;
     switch (H.nt) {
-        case 1: r = launch_forces_kspace<1>(c); break;
-        case 2: r = launch_forces_kspace<2>(c); break;
-        case 3: r = launch_forces_kspace<3>(c); break;
-        default: r = launch_forces_kspace<4>(c); break;
+        case 1: r = launch_forces<1>(c); break;
+        case 2: r = launch_forces<2>(c); break;
+        case 3: r = launch_forces<3>(c); break;
+        default: r = launch_forces<4>(c); break;
     }
     if (r) return r;
-    std::vector<double> gx(N), gy(N), gz(N);
-    CUDA_TRY(cudaMemcpyAsync(gx.data(), c->d_gx, sizeof(double) * N, cudaMemcpyDeviceToHost, c->stream));
-    CUDA_TRY(cudaMemcpyAsync(gy.data(), c->d_gy, sizeof(double) * N, cudaMemcpyDeviceToHost, c->stream));
-    CUDA_TRY(cudaMemcpyAsync(gz.data(), c->d_gz, sizeof(double) * N, cudaMemcpyDeviceToHost, c->stream));
+    std::vector<double> g((size_t)3 * N);
+    CUDA_TRY(cudaMemcpyAsync(g.data(), c->d_f, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
+    double *gx = g.data(), *gy = gx + N, *gz = gy + N;
     // external term: F = -2 kext q mu (EwaldSumExternal.f90:84-102)
     const double mx = c->sc[SC_MU_X], my = c->sc[SC_MU_Y], mz = c->sc[SC_MU_Z], m2k = H.p.minus_two_kext;
     bool finite = true;
