@@ -32,7 +32,7 @@ namespace cg = cooperative_groups;
 
 struct LaunchCfg {
     int G = 0, B = 0, EPT = 0;  // EPT: entries per worker in registers; 0 streamed; -1 streamed, wide CTAs
-    int nown_max = 0, qcap = 0;
+    int nown_max = 0;
     size_t smem = 0;
 };
 
@@ -68,7 +68,6 @@ struct ChainArgs {
     RunSlot *run;       // [R]
     int G;              // CTAs per chain (cluster size)
     int nown_max;       // atoms staged per CTA (interleaved ownership: atom j lives in CTA j % G, in slot D.slot[j])
-    int qcap;           // pair queue capacity per CTA
     double2 *scratch;      // [2][(1+nt) S]: molecule old sums, rho deltas (scratch_buf: FP32 pairs in the mixed form)
     long long *prof;       // optional per-phase cycle counters (PH_* layout), CTA 0
 };
@@ -87,10 +86,20 @@ enum PassKind { PASS_OLD = 0, PASS_NEW = 1, PASS_BOTH = 2 };
 
 struct Slot { double x, y, z, q, iq, dhs; int type, pad; };
 constexpr int kMaxSpecies = 8;
-constexpr int kCPT = 8;   // atoms each worker thread tests per filter round
-constexpr int kBlk = 32;  // atoms per bounding box of the pair filter (one warp's candidates per round and c)
-constexpr int kQueueMax = 2560;  // pair-queue chunk (items); a round's pairs are consumed in chunks
+constexpr int kBlk = 32;  // atoms per bounding box of the pair filter: one warp's lanes
+constexpr int kNear = 256;  // near atoms a warp gathers before it tests them against the molecule's slots
+constexpr int kPairs = 32 * 2 * kMaxA + 64;  // pairs a warp's queue holds: those of 32 atoms and a rest below 64
+constexpr int kBlkList = 96;  // near blocks of one warp: those of kMaxOwn atoms over three warps and more
+constexpr int kWarpBuf = (kNear + kPairs + kBlkList) / 2;  // a warp's buffers, ints
 constexpr int kWin = 256; // random-stream window held in shared memory
+constexpr int kMaxOwn = 8192;  // atoms staged per CTA: a pair names its atom in 13 bits
+
+// ints of the warps' near-atom and pair buffers of a B-thread CTA; at least room for the phase
+// tables of two atoms (the mixed form's refresh works in it)
+__host__ __device__ inline int wbuf_ints(int B, int kmax) {
+    const int warps = (B / 32) * kWarpBuf, tables = 4 + 2 * (3 * 4 * (kmax + 1) + 3);
+    return ((warps > tables ? warps : tables) + 1) & ~1;
+}
 constexpr int kCtl = 32;  // threads of the control warp
 constexpr int kChainMaxThreads = 256;  // one CTA per SM, up to 255 registers per thread
 constexpr int kChainMaxThreadsWide = YAMC_WIDE_THREADS;  // streamed k entries, more warps, fewer registers
@@ -239,25 +248,34 @@ struct Cand {
     MoveState mv;
 };
 
+// the CTA's staged atoms and buffers (shared memory), as the real-space part reads them
+struct StageView {
+    const double4 *atom;   // x, y, z, q by staging slot
+    const int2 *meta;      // molecule, LJ type
+    const float4 *box;     // bounding boxes of the blocks
+    const double *dhs_ts, *lj;  // hard cores by LJ type; LJ tables
+    double *red;           // [worker warp][kNV]
+    int *wbuf;             // the warps' near atoms and pairs
+    int nown, grank, gsize;
+};
+
 struct ChainShared {
+    StageView view;
     Cand cand[4];         // the move being evaluated (cand[icur]) and up to three prepared next moves
     int icur;             // buffer of the move being evaluated
-    int imoved;           // buffer of the move just decided (its commit)
     int spec[3];          // buffers of the candidates: after an overlap / after a draw / accepted same molecule
     int abort, accepted, overlap, last_mol, spec_ok;
     long long cursor;     // stream position after the last completed move
     long long icycle, mic;
-    double eold[3], fold[3 * kMaxA];
+    double eold[3];
     // the biased proposal on two warps: the rotation thread's result and stream positions
     MoveState mrot;
     long long disp_end, rot_start, rot_end;
     int disp_out, rot_out;
     double sc[SC_COUNT];
     double lx[kMaxA], ly[kMaxA], lz[kMaxA];  // last accepted move (staged copies may lag in other CTAs)
-    int qcount;
-    int wcount[64];       // per-warp pair counts and their exclusive prefix
-    int wmore[32];        // per worker warp: near blocks left after this filter round
-    int qmore;            // some worker warp has near blocks left
+    // the move just decided, for the workers' commit (its candidate buffer may be taken meanwhile)
+    int mv_first, mv_na, mv_tmask, mv_simple, mv_slot[kMaxA];
     double tot[kNV];
     double du[4];
     int flags;
@@ -825,242 +843,190 @@ __device__ __noinline__ void kspace_part_call(const DevSys &D, RegsOf<NT, EPT, M
     kspace_part<NT, EPT, KIND, FORCES, MX, SIMPLE>(D, R, pt, MolK<MX>(slots, na), e0, estep, mold_g, row);
 }
 
-// The workers' part of one pass over the molecule's slots: k-space over their entries, real
-// space over the CTA's atoms (pairs inside the cutoff laid out in the queue by a prefix sum
-// over threads -- a deterministic order -- then evaluated item i by worker i % nwork), and a
-// per-warp reduction into red[worker warp][value].  Worker-only barriers (bar 1).
-template <int NT, int EPT, int KIND, bool FORCES, bool MX>
-__device__ __forceinline__ void worker_pass_body(const DevSys &D, ChainShared &sh, RegsOf<NT, EPT, MX> &R, double2 *tab_raw,
-                                            const double4 *atom_s, const double *dhs_ts, const double *dhs_g,
-                                            int dhs_typed, int grank, int gsize, const int2 *meta_s, const float4 *box_s,
-                                            int *blist, int *queue,
-                                            int *nearbuf,
-                                            double *red, const double *lj_s, int nown, int qcap, int e0, int estep,
-                                            long long *prof, typename Prec<MX>::R2 *mold_buf) {
-    constexpr int NVMAX = FORCES ? kNVP : RV_F;
+// Real space of one pass, by the worker warps: the moving molecule's pairs with the CTA's staged atoms,
+// and the reduction into red[worker warp][value].  FORCES: the old positions (is_new false) or the new
+// ones with their forces; otherwise both positions at once, signed.
+#define YAMC_WPH(ph) do { if (pf) { const long long t_now = clock64(); prof[ph] += t_now - t_mark; t_mark = t_now; } } while (0)
+template <bool FORCES, bool MX>
+__device__ __forceinline__ void real_part(const DevSys &D, ChainShared &sh, bool is_new, long long *prof) {
     const Cand &m = sh.cand[sh.icur];
-    const int na = m.na;
-    const int KM = D.kmax + 1;
-    const int nt = D.nt;
-    const int imol0 = m.imol - 1;
-    const int nwork = blockDim.x - kCtl;
-    const int wtid = threadIdx.x - kCtl;
-    const int lane = threadIdx.x & 31;
-    const int wwarp = wtid >> 5, nww = nwork >> 5;
-    const int s_lo = (KIND == PASS_OLD) ? na : 0;  // active slots [s_lo, s_hi)
-    const int s_hi = (KIND == PASS_NEW) ? na : 2 * na;
-    using Rt = typename Prec<MX>::R;
-    using R2 = typename Prec<MX>::R2;
-    R2 *tab = reinterpret_cast<R2 *>(tab_raw);
+    const StageView &V = sh.view;
+    const double4 *atom_s = V.atom;
+    const int2 *meta_s = V.meta;
+    const float4 *box_s = V.box;
+    const double *lj_s = V.lj;
+    const int na = m.na, nt = D.nt, nown = V.nown, imol0 = m.imol - 1;
+    const int wtid = threadIdx.x - kCtl, lane = threadIdx.x & 31;
+    const int wwarp = wtid >> 5, nww = (blockDim.x - kCtl) >> 5;
+    const int s_lo = FORCES && !is_new ? na : 0, s_hi = FORCES && is_new ? na : 2 * na;  // active slots [s_lo, s_hi)
+    const bool hard = !FORCES || is_new;  // hard cores are tested at the new positions
+    const int nv = FORCES ? (RV_F + 3 * na) : RV_F;
+    double *red = V.red;
+    int *wbuf = V.wbuf;
     const bool pf = prof && wtid == 0;
     long long t_mark = pf ? clock64() : 0;
-#define YAMC_WPH(ph) do { if (pf) { const long long t_now = clock64(); prof[ph] += t_now - t_mark; t_mark = t_now; } } while (0)
-
-    build_tables<MX>(tab, m.slot, s_lo, s_hi, KM, wtid, nwork);
-    worker_sync(nwork);
-    YAMC_WPH(PH_TABLES);
-    const PhaseTabs<MX> pt{tab, KM};
-
-    // k space, out of line when the entries are streamed: each sweep then has the register budget to
-    // itself, and its sums are in the warp's row of red before the real-space part begins
-    const int nv = FORCES ? (RV_F + 3 * na) : RV_F;
-    {
-        const MolK<MX> mk(m.slot, na);
-        double *row = red + wwarp * kNV;
-        if constexpr (EPT > 0) {
-            if (mk.simple) kspace_part<NT, EPT, KIND, FORCES, MX, true>(D, R, pt, mk, e0, estep, mold_buf, row);
-            else kspace_part<NT, EPT, KIND, FORCES, MX, false>(D, R, pt, mk, e0, estep, mold_buf, row);
-        } else {
-            if (mk.simple) kspace_part_call<NT, EPT, KIND, FORCES, MX, true>(D, R, pt, m.slot, na, e0, estep, mold_buf, row);
-            else kspace_part_call<NT, EPT, KIND, FORCES, MX, false>(D, R, pt, m.slot, na, e0, estep, mold_buf, row);
-        }
-    }
     Acc<MX> acc;
     acc.zero();
-    YAMC_WPH(PH_KSPACE);
 
-    // bounding spheres of the molecule at its new (slot 0) and old (slot na) positions: an atom
-    // farther than rpre + radius from a centre is outside the cutoff and every hard core of all
-    // that position's slots (triangle inequality on the periodic box), so its slot tests are skipped
-    double rp2;
+    // Real space, warp by warp: the staged blocks are dealt to the warps in turn (neighbours in space
+    // go to different warps); a warp gathers the atoms of its near blocks inside the query sphere, four
+    // blocks at a time, tests them 32 at a time against the molecule's slots (cutoff, hard core), and
+    // evaluates the pairs that pass 64 at a time from its own queue: no barrier between the warps,
+    // full warps in every step, and in each step independent work (with two warps per scheduler it is
+    // latency that bounds it), in an order that the positions alone decide.
     {
-        double rad2 = 0.0;
-        for (int a = 1; a < na; ++a) {
-            const double dx = m.slot[a].x - m.slot[0].x, dy = m.slot[a].y - m.slot[0].y, dz = m.slot[a].z - m.slot[0].z;
-            rad2 = fmax(rad2, dx * dx + dy * dy + dz * dz);
-            const double ex = m.slot[na + a].x - m.slot[na].x, ey = m.slot[na + a].y - m.slot[na].y,
-                         ez = m.slot[na + a].z - m.slot[na].z;
-            rad2 = fmax(rad2, ex * ex + ey * ey + ez * ez);
-        }
-        const double rp = (D.rpre + sqrt(rad2)) * (1.0 + 1e-9);
-        rp2 = rp * rp;
-    }
-    const double cnx = m.slot[0].x, cny = m.slot[0].y, cnz = m.slot[0].z;
-    const double cox = m.slot[na].x, coy = m.slot[na].y, coz = m.slot[na].z;
-    // a pass over both positions tests one sphere around the midpoint of the two centres that
-    // holds both spheres (the centre may have been wrapped: the shift is taken by minimum image)
-    double cbx = cox, cby = coy, cbz = coz, rb2 = rp2;
-    if (KIND == PASS_BOTH) {
-        const double hx = 0.5 * min_image(cnx - cox), hy = 0.5 * min_image(cny - coy), hz = 0.5 * min_image(cnz - coz);
-        cbx = cox + hx; cby = coy + hy; cbz = coz + hz;
-        const double rb = (sqrt(rp2) + sqrt(hx * hx + hy * hy + hz * hz)) * (1.0 + 1e-9);
-        rb2 = rb * rb;
-    }
-
-    // this warp's near blocks: of the blocks wwarp + nww k (kBlk consecutive slots each; the
-    // staged atoms are in spatial order), those whose bounding box comes within the query sphere.
-    // A block outside it holds no atom that the per-atom test below keeps.
-    const int nblk = (nown + kBlk - 1) / kBlk;
-    const int wcap = (nblk + nww - 1) / nww;
-    int *wl = blist + wwarp * wcap;
-    int nnb = 0;
-    {
-        const double qx = KIND == PASS_BOTH ? cbx : (KIND == PASS_NEW ? cnx : cox);
-        const double qy = KIND == PASS_BOTH ? cby : (KIND == PASS_NEW ? cny : coy);
-        const double qz = KIND == PASS_BOTH ? cbz : (KIND == PASS_NEW ? cnz : coz);
-        const double qr2 = KIND == PASS_BOTH ? rb2 : rp2;
-        for (int k0 = 0; k0 < wcap; k0 += 32) {
-            const int k = k0 + lane, b = wwarp + nww * k;
-            const bool near = k < wcap && b < nblk && box_near(box_s, b, qx, qy, qz, qr2);
-            const unsigned bal = __ballot_sync(0xffffffffu, near);
-            if (near) wl[YAMC_IX(nnb + __popc(bal & ((1u << lane) - 1u)), wcap)] = b;
-            nnb += __popc(bal);
-        }
-        __syncwarp();
-    }
-    int *nb = nearbuf + wwarp * 32 * kCPT;  // this warp's near atoms of the round
-    for (int r0 = 0;; r0 += kCPT) {
-        // near atoms of the warp's next kCPT near blocks, compacted in (block, lane) order
-        int nnear = 0;
-#pragma unroll
-        for (int c = 0; c < kCPT; ++c) {
-            const int jl = r0 + c < nnb ? wl[YAMC_IX(r0 + c, wcap)] * kBlk + lane : nown;
-            bool near = false;
-            if (jl < nown && meta_s[YAMC_IX(jl, nown)].x != imol0) {
-                const double4 pj = atom_s[YAMC_IX(jl, nown)];
-                if (KIND == PASS_BOTH) {
-                    const double dx = min_image(cbx - pj.x), dy = min_image(cby - pj.y), dz = min_image(cbz - pj.z);
-                    near = dx * dx + dy * dy + dz * dz < rb2;
-                } else if (KIND == PASS_NEW) {
-                    const double dx = min_image(cnx - pj.x), dy = min_image(cny - pj.y), dz = min_image(cnz - pj.z);
-                    near = dx * dx + dy * dy + dz * dz < rp2;
-                } else {
-                    const double dx = min_image(cox - pj.x), dy = min_image(coy - pj.y), dz = min_image(coz - pj.z);
-                    near = dx * dx + dy * dy + dz * dz < rp2;
-                }
+        unsigned short *nb = reinterpret_cast<unsigned short *>(wbuf + wwarp * kWarpBuf);  // near atoms
+        unsigned short *queue = nb + kNear, *blocks = queue + kPairs;                      // pairs (slot << 13 | atom); near blocks
+        const unsigned lt = (1u << lane) - 1u;
+        // the query sphere: an atom farther than the pair filter's reach plus the molecule's radius from
+        // its centre (slot 0 new, slot na old) is outside the cutoff and every hard core of all slots
+        // (triangle inequality on the periodic box).  A pass over both positions takes one sphere
+        // around the midpoint of the two centres that holds both (the centre may have been wrapped: the
+        // shift is taken by minimum image).  Radii in FP32, rounded up.
+        double qx, qy, qz, qr2;
+        {
+            double rad2 = 0.0;
+            for (int a = 1; a < na; ++a) {
+                const double dx = m.slot[a].x - m.slot[0].x, dy = m.slot[a].y - m.slot[0].y, dz = m.slot[a].z - m.slot[0].z;
+                const double ex = m.slot[na + a].x - m.slot[na].x, ey = m.slot[na + a].y - m.slot[na].y,
+                             ez = m.slot[na + a].z - m.slot[na].z;
+                rad2 = fmax(rad2, fmax(dx * dx + dy * dy + dz * dz, ex * ex + ey * ey + ez * ez));
             }
+            double r = D.rpre + (double)__fsqrt_ru(__double2float_ru(rad2));
+            const Slot &c = m.slot[is_new ? 0 : na];
+            qx = c.x; qy = c.y; qz = c.z;
+            if constexpr (!FORCES) {
+                const double hx = 0.5 * min_image(m.slot[0].x - qx), hy = 0.5 * min_image(m.slot[0].y - qy),
+                             hz = 0.5 * min_image(m.slot[0].z - qz);
+                qx += hx; qy += hy; qz += hz;
+                r += (double)__fsqrt_ru(__double2float_ru(hx * hx + hy * hy + hz * hz));
+            }
+            r *= 1.0 + 1e-9;
+            qr2 = r * r;
+        }
+        // this warp's blocks whose bounding box comes within the query sphere.  A block outside it
+        // holds no atom that the per-atom test below keeps.
+        const int nblk = (nown + kBlk - 1) / kBlk;
+        int nnear = 0, npair = 0, nmine = 0;
+        bool ovl = false;
+        for (int b0 = wwarp; b0 < nblk; b0 += 32 * nww) {
+            const int b = b0 + nww * lane;
+            const bool near = b < nblk && box_near(box_s, b, qx, qy, qz, qr2);
             const unsigned bal = __ballot_sync(0xffffffffu, near);
-            if (near) nb[YAMC_IX(nnear + __popc(bal & ((1u << lane) - 1u)), 32 * kCPT)] = jl;
-            nnear += __popc(bal);
+            if (near) blocks[YAMC_IX(nmine + __popc(bal & lt), kBlkList)] = (unsigned short)b;
+            nmine += __popc(bal);
         }
         __syncwarp();
-        // slot tests of the near atoms, densely: lane takes entries lane, lane + 32, ...
-        unsigned long long masks = 0;  // kCPT slot masks of 8 bits
-        int count = 0;
+        // (one loop with one copy of each step: the code of a move runs once per move, so its size is
+        // instruction fetches, not only cache)
+        for (int i0 = 0;;) {
+            if (i0 < nmine) {
+                // near atoms of four blocks
+                int jl[4];
+                bool near[4];
 #pragma unroll
-        for (int c = 0; c < kCPT; ++c) {
-            const int k = c * 32 + lane;
-            if (k < nnear) {
-                const int jl = nb[YAMC_IX(k, 32 * kCPT)];
+                for (int u = 0; u < 4; ++u) {
+                    jl[u] = i0 + u < nmine ? blocks[i0 + u] * kBlk + lane : nown;
+                    const int j = jl[u] < nown ? jl[u] : 0;
+                    const double4 pj = atom_s[YAMC_IX(j, nown)];
+                    const double dx = min_image(qx - pj.x), dy = min_image(qy - pj.y), dz = min_image(qz - pj.z);
+                    near[u] = jl[u] < nown && meta_s[YAMC_IX(j, nown)].x != imol0 && dx * dx + dy * dy + dz * dz < qr2;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const unsigned bal = __ballot_sync(0xffffffffu, near[u]);
+                    if (near[u]) nb[YAMC_IX(nnear + __popc(bal & lt), kNear)] = (unsigned short)jl[u];
+                    nnear += __popc(bal);
+                }
+                i0 += 4;
+            }
+            const bool last = i0 >= nmine;
+            if (!last && nnear <= kNear - 4 * kBlk) continue;
+            __syncwarp();
+            if (last) YAMC_WPH(PH_FILTER);
+            int k0 = 0;
+            do {
+                // slot tests of 32 gathered atoms
+                const bool valid = k0 + lane < nnear;
+                const int jl = valid ? nb[k0 + lane] : 0;
                 const double4 pj = atom_s[YAMC_IX(jl, nown)];
                 const int tj = meta_s[YAMC_IX(jl, nown)].y;
-                // hard-core diameter: by LJ type when every atom of a type has the same one
-                // (a shared-memory table), else the atom's own (global memory, by the atom in slot jl)
-                const double dj = dhs_typed ? dhs_ts[tj] : dhs_g[D.atom_of[YAMC_IX(jl * gsize + grank, D.N + 16)]];
-                unsigned msk = 0;
+                // hard-core diameter: by LJ type when every atom of a type has the same one (a
+                // shared-memory table), else the atom's own (global memory, by the atom in slot jl)
+                const double dj = !hard        ? 0.0
+                                  : D.dhs_typed ? V.dhs_ts[tj]
+                                                : D.dhs[D.atom_of[YAMC_IX(jl * V.gsize + V.grank, D.N + 16)]];
+                unsigned in = 0;  // slots inside the cutoff
+#pragma unroll 3
                 for (int s = s_lo; s < s_hi; ++s) {
                     const Slot &sl = m.slot[s];
                     const double dx = min_image(sl.x - pj.x), dy = min_image(sl.y - pj.y), dz = min_image(sl.z - pj.z);
                     const double r2 = dx * dx + dy * dy + dz * dz;
-                    if (KIND != PASS_OLD && s < na && sl.type > 0 && tj > 0) {  // hard core (EwaldSumRealSpace.f90:409)
+                    if (hard && s < na && sl.type > 0 && tj > 0) {  // hard core (EwaldSumRealSpace.f90:409)
                         const double d12 = (sl.dhs + dj) / 2;
-                        if (r2 < d12 * d12) acc.flag(RV_OVL);
+                        if (valid && r2 < d12 * d12) ovl = true;
                     }
-                    if (r2 < D.rmax2) msk |= 1u << s;
+                    if (valid && r2 < D.rmax2) in |= 1u << s;
                 }
-                masks |= (unsigned long long)msk << (8 * c);
-                count += __popc(msk);
-            }
-        }
-        int incl = count;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) { sh.wcount[wwarp] = incl; sh.wmore[wwarp] = nnb > r0 + kCPT; }
-        worker_sync(nwork);
-        if (wwarp == 0) {
-            const int v = lane < nww ? sh.wcount[lane] : 0;
-            int x = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            if (lane < nww) sh.wcount[32 + lane] = x - v;
-            if (lane == 31) sh.qcount = x;
-            const bool more = __any_sync(0xffffffffu, lane < nww && sh.wmore[lane] != 0);
-            if (lane == 0) sh.qmore = more;
-        }
-        worker_sync(nwork);
-        // another round while some warp has near blocks left (read here: the next round's
-        // writes come after its first barrier)
-        const bool more_rounds = sh.qmore != 0;
-        // the round's pairs in queue order (thread order by the prefix sums), consumed in chunks of
-        // qcap: each thread writes its items that fall in the chunk, the workers evaluate them
-        const int base = sh.wcount[32 + wwarp] + incl - count;
-        const int nq = sh.qcount;
-        for (int q0 = 0; q0 < nq; q0 += qcap) {
-            if (base < q0 + qcap && base + count > q0) {
-                int pos = base;
-#pragma unroll
-                for (int c = 0; c < kCPT; ++c) {
-                    unsigned msk = (unsigned)(masks >> (8 * c)) & 0xffu;
-                    const int jl = msk ? nb[c * 32 + lane] : 0;
-                    while (msk) {
-                        const int s = __ffs(msk) - 1;
-                        msk &= msk - 1;
-                        if (pos >= q0 && pos < q0 + qcap) queue[YAMC_IX(pos - q0, qcap)] = (jl << 3) | s;
-                        ++pos;
-                    }
+                // the pairs slot by slot, an atom each lane
+                for (int s = s_lo; s < s_hi; ++s) {
+                    const unsigned bal = __ballot_sync(0xffffffffu, in >> s & 1);
+                    if (in >> s & 1) queue[YAMC_IX(npair + __popc(bal & lt), kPairs)] = (unsigned short)(s << 13 | jl);
+                    npair += __popc(bal);
                 }
-            }
-            worker_sync(nwork);
-            if (q0 == 0) YAMC_WPH(PH_FILTER);
-            const int nc = min(qcap, nq - q0);
-            for (int qi = wtid; qi < nc; qi += nwork) {
-                const int item = queue[YAMC_IX(qi, qcap)];
-                const int jl = item >> 3, s = item & 7;
-                const Slot &sl = m.slot[s];
-                const double4 pj = atom_s[YAMC_IX(jl, nown)];
-                const int tj = meta_s[YAMC_IX(jl, nown)].y;
-                const double dx = min_image(sl.x - pj.x), dy = min_image(sl.y - pj.y), dz = min_image(sl.z - pj.z);
-                const double r2 = dx * dx + dy * dy + dz * dz;
-                const bool lj = sl.type > 0 && tj > 0;
-                const int off = lj ? (sl.type - 1) * nt + (tj - 1) : 0;
-                const double qq = D.xclb * sl.q * pj.w;
-                const double s6 = lj ? lj_s[off] : 0.0, fe = lj ? lj_s[nt * nt + off] : 0.0;
-                const bool isnew = s < na;
-                const double sign = (KIND == PASS_BOTH && !isnew) ? -1.0 : 1.0;
-                const PairTerm<double> t = MX ? pair_term_mx<FORCES>(r2, qq, lj, s6, fe, D.alpha, D.taosp, false)
-                                              : pair_term<double, FORCES>(r2, qq, lj, s6, fe, D.alpha, D.taosp, false);
-                acc.add(RV_EW, sign * t.ew); acc.add(RV_LJ6, sign * t.lj6); acc.add(RV_LJ12, sign * t.lj12);
-                if constexpr (FORCES) {
-                    const int a = isnew ? s : s - na;
+                __syncwarp();
+                k0 += 32;
+                // whole groups of 64 pairs (at the end all) are evaluated, two per lane side by side; the
+                // rest moves to the queue's front
+                const int n = last && k0 >= nnear ? npair : npair & ~63;
+                for (int q0 = lane; q0 < n; q0 += 64) {
 #pragma unroll
-                    for (int aa = 0; aa < kMaxA; ++aa)
-                        if (aa == a) {
-                            acc.add(RV_F + 3 * aa, dx * t.FR);
-                            acc.add(RV_F + 3 * aa + 1, dy * t.FR);
-                            acc.add(RV_F + 3 * aa + 2, dz * t.FR);
+                    for (int u = 0; u < 2; ++u) {
+                        const int q = q0 + 32 * u;
+                        const int item = queue[q < n ? q : q0];
+                        const int ji = item & 8191, s = item >> 13;
+                        const Slot &sl = m.slot[s];
+                        const double4 pi = atom_s[YAMC_IX(ji, nown)];
+                        const int ti = meta_s[YAMC_IX(ji, nown)].y;
+                        const double dx = min_image(sl.x - pi.x), dy = min_image(sl.y - pi.y), dz = min_image(sl.z - pi.z);
+                        const double r2 = dx * dx + dy * dy + dz * dz;
+                        const bool lj = sl.type > 0 && ti > 0;
+                        const int off = lj ? (sl.type - 1) * nt + (ti - 1) : 0;
+                        const double qq = D.xclb * sl.q * pi.w;
+                        const double s6 = lj ? lj_s[off] : 0.0, fe = lj ? lj_s[nt * nt + off] : 0.0;
+                        const bool isnew = s < na;
+                        const double sign = (!FORCES && !isnew) ? -1.0 : 1.0;
+                        const PairTerm<double> t = MX ? pair_term_mx<FORCES>(r2, qq, lj, s6, fe, D.alpha, D.taosp, false)
+                                                      : pair_term<double, FORCES>(r2, qq, lj, s6, fe, D.alpha, D.taosp, false);
+                        if (q < n) {
+                            acc.add(RV_EW, sign * t.ew); acc.add(RV_LJ6, sign * t.lj6); acc.add(RV_LJ12, sign * t.lj12);
+                            if constexpr (FORCES) {
+                                const int a = isnew ? s : s - na;
+#pragma unroll
+                                for (int aa = 0; aa < kMaxA; ++aa)
+                                    if (aa == a) {
+                                        acc.add(RV_F + 3 * aa, dx * t.FR);
+                                        acc.add(RV_F + 3 * aa + 1, dy * t.FR);
+                                        acc.add(RV_F + 3 * aa + 2, dz * t.FR);
+                                    }
+                            }
                         }
+                    }
                 }
-            }
-            worker_sync(nwork);
+                if (n > 0) {
+                    __syncwarp();
+                    const unsigned short r0 = n + lane < npair ? queue[n + lane] : 0, r1 = n + 32 + lane < npair ? queue[n + 32 + lane] : 0;
+                    __syncwarp();
+                    queue[lane] = r0; queue[32 + lane] = r1;
+                    npair -= n;
+                    __syncwarp();
+                }
+            } while (k0 < nnear);
+            nnear = 0;
+            if (last) break;
         }
+        if (ovl) acc.flag(RV_OVL);
         YAMC_WPH(PH_PAIRS);
-        if (!more_rounds) break;
     }
 
     // the real-space sums over the warp, added to the k-space sums in the warp's row
@@ -1076,43 +1042,60 @@ __device__ __forceinline__ void worker_pass_body(const DevSys &D, ChainShared &s
         if (!(lane & 1) && i < NR && at < nv) row[at] = i < 3 ? x : row[at] + x;
         if (lane == 31) {
             row[RV_OVL] = ovl ? 1.0 : 0.0;
-            if (KIND == PASS_OLD) row[RV_DUC] = row[RV_DUL] = 0.0;
+            if (!hard) row[RV_DUC] = row[RV_DUL] = 0.0;
         }
     }
-#undef YAMC_WPH
 }
 
-// The passes are called, not inlined, when the k entries are streamed (EPT <= 0): each pass then
-// gets the kernel's whole register budget for its own loops instead of sharing it with the
-// control code and the other passes (fewer spills); with entries in registers (EPT > 0) they
-// are inlined, since the entry registers R must stay registers across the passes.
-template <int NT, int EPT, int KIND, bool FORCES, bool MX>
-__device__ __noinline__ void worker_pass_call(const DevSys &D, ChainShared &sh, RegsOf<NT, EPT, MX> &R, double2 *tab_raw,
-                                              const double4 *atom_s, const double *dhs_ts, const double *dhs_g,
-                                              int dhs_typed, int grank, int gsize, const int2 *meta_s, const float4 *box_s,
-                                            int *blist, int *queue,
-                                              int *nearbuf, double *red, const double *lj_s, int nown, int qcap, int e0,
-                                              int estep, long long *prof, typename Prec<MX>::R2 *mold_buf) {
-    worker_pass_body<NT, EPT, KIND, FORCES, MX>(D, sh, R, tab_raw, atom_s, dhs_ts, dhs_g, dhs_typed, grank, gsize, meta_s,
-                                                box_s, blist, queue, nearbuf, red, lj_s, nown, qcap, e0, estep, prof, mold_buf);
+// One copy for the two passes of a biased move, out of line: the second finds its instructions where
+// the first fetched them.  (WIDE: the copy of the wide CTAs, which have fewer registers a thread.)
+template <bool MX, bool WIDE>
+__device__ __noinline__ void real_part_forces(const DevSys &D, ChainShared &sh, bool is_new, long long *prof) {
+    real_part<true, MX>(D, sh, is_new, prof);
 }
 
-template <int NT, int EPT, int KIND, bool FORCES, bool MX>
-__device__ __forceinline__ void worker_pass(const DevSys &D, ChainShared &sh, RegsOf<NT, EPT, MX> &R, double2 *tab_raw,
-                                            const double4 *atom_s, const double *dhs_ts, const double *dhs_g,
-                                            int dhs_typed, int grank, int gsize, const int2 *meta_s, const float4 *box_s,
-                                            int *blist, int *queue,
-                                            int *nearbuf, double *red, const double *lj_s, int nown, int qcap, int e0,
+// The workers' part of one pass over the molecule's slots: the phase tables, k space over the worker's
+// entries, real space over the CTA's atoms (PASS_OLD and PASS_NEW with forces, PASS_BOTH without).
+// One worker barrier (bar 1), after the tables.
+template <int NT, int EPT, int KIND, bool MX>
+__device__ __forceinline__ void worker_pass(const DevSys &D, ChainShared &sh, RegsOf<NT, EPT, MX> &R, double2 *tab_raw, int e0,
                                             int estep, long long *prof, typename Prec<MX>::R2 *mold_buf) {
-    if constexpr (EPT > 0)
-        worker_pass_body<NT, EPT, KIND, FORCES, MX>(D, sh, R, tab_raw, atom_s, dhs_ts, dhs_g, dhs_typed, grank, gsize,
-                                                    meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, qcap, e0, estep, prof,
-                                                    mold_buf);
-    else
-        worker_pass_call<NT, EPT, KIND, FORCES, MX>(D, sh, R, tab_raw, atom_s, dhs_ts, dhs_g, dhs_typed, grank, gsize,
-                                                    meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, qcap, e0, estep, prof,
-                                                    mold_buf);
+    constexpr bool FORCES = KIND != PASS_BOTH;
+    const Cand &m = sh.cand[sh.icur];
+    const int na = m.na;
+    const int KM = D.kmax + 1;
+    const int nwork = blockDim.x - kCtl;
+    const int wtid = threadIdx.x - kCtl;
+    const int s_lo = (KIND == PASS_OLD) ? na : 0;  // active slots [s_lo, s_hi)
+    const int s_hi = (KIND == PASS_NEW) ? na : 2 * na;
+    using R2 = typename Prec<MX>::R2;
+    R2 *tab = reinterpret_cast<R2 *>(tab_raw);
+    const bool pf = prof && wtid == 0;
+    long long t_mark = pf ? clock64() : 0;
+
+    build_tables<MX>(tab, m.slot, s_lo, s_hi, KM, wtid, nwork);
+    worker_sync(nwork);
+    YAMC_WPH(PH_TABLES);
+    const PhaseTabs<MX> pt{tab, KM};
+
+    // k space, out of line when the entries are streamed: each sweep then has the register budget to
+    // itself (entries in registers must stay there across the passes)
+    {
+        const MolK<MX> mk(m.slot, na);
+        double *row = sh.view.red + (wtid >> 5) * kNV;
+        if constexpr (EPT > 0) {
+            if (mk.simple) kspace_part<NT, EPT, KIND, FORCES, MX, true>(D, R, pt, mk, e0, estep, mold_buf, row);
+            else kspace_part<NT, EPT, KIND, FORCES, MX, false>(D, R, pt, mk, e0, estep, mold_buf, row);
+        } else {
+            if (mk.simple) kspace_part_call<NT, EPT, KIND, FORCES, MX, true>(D, R, pt, m.slot, na, e0, estep, mold_buf, row);
+            else kspace_part_call<NT, EPT, KIND, FORCES, MX, false>(D, R, pt, m.slot, na, e0, estep, mold_buf, row);
+        }
+    }
+    YAMC_WPH(PH_KSPACE);
+    if constexpr (FORCES) real_part_forces<MX, (EPT < 0)>(D, sh, KIND == PASS_NEW, prof);
+    else real_part<false, MX>(D, sh, false, prof);
 }
+#undef YAMC_WPH
 
 // Control warp, after the workers' per-warp partials: trees over the worker warps, then over the
 // cluster's CTAs in a fixed order, so every CTA holds bit-identical totals in sh.tot.  Called by
@@ -1186,9 +1169,13 @@ __device__ inline RngReader make_reader(const ChooseCtx &X, const ChainShared &s
     // the window that holds cur (the newer one where both do): the draws of a move fit in it, and
     // one that passes its end reads the stream itself
     const int b = sh.wnext ^ 1;
-    const unsigned long long k = (unsigned long long)(cur - sh.wbase[b]);
-    const int s = sh.wbase[b] >= 0 && k < (unsigned long long)sh.wn[b] ? b : b ^ 1;
-    return RngReader{X.run->rng, X.run->rng_off, X.run->n_rng, cur, 0, s ? X.w1 : X.w0, sh.wbase[s], sh.wn[s]};
+    const unsigned long long k = (unsigned long long)(cur - sh.wbase[b]), k2 = (unsigned long long)(cur - sh.wbase[b ^ 1]);
+    const bool in = sh.wbase[b] >= 0 && k < (unsigned long long)sh.wn[b];
+    const bool in2 = !in && sh.wbase[b ^ 1] >= 0 && k2 < (unsigned long long)sh.wn[b ^ 1];
+    const int s = in ? b : b ^ 1;
+    const bool any = in || in2;
+    return RngReader{X.run->rng, X.run->rng_off, X.run->n_rng, s ? X.w1 : X.w0, any ? sh.wbase[s] : cur, any ? sh.wn[s] : 0,
+                     any ? (int)(in ? k : k2) : 0, 0};
 }
 
 __device__ inline void stage_molecule(const ChooseCtx &X, ChainShared &sh, Cand &C, int imol, int moving,
@@ -1250,14 +1237,12 @@ __device__ inline int draw_molecule(const DevSys &D, RngReader &rng, bool cycle_
     return choose_molecule_guess(r, D.freq_beg, D.freq_end, D.M, D.freq_monotone);
 }
 
-// movemc Step 5 (MC.f90:1031-1067) for a staged molecule; F/T are the old molecular force and
-// torque (zero for unbiased moves)
-__device__ inline void propose(const DevSys &D, Cand &C, RngReader &rng, const double F[3], const double T[3]) {
+// movemc Step 5 (MC.f90:1031-1067) of an unbiased move for a staged molecule
+__device__ inline void propose(const DevSys &D, Cand &C, RngReader &rng) {
     const int na = C.na;
     MoveState &m = C.mv;
-    mcm_init_old(m, F, T);
-    mcm_choose_displacement(m, rng, D.xlf, D.dr);
-    if (!rng.out) mcm_choose_rotation(m, rng, D.xlc, D.d_angle);
+    mcm_choose_unbiased(m, rng, D.dr, D.d_angle);
+    if (rng.out) return;
     // old positions from slots [na, 2 na), new ones into [0, na): no overlap
     const Slot *os = C.slot + na;
     Slot *ns = C.slot;
@@ -1421,17 +1406,15 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
     float4 *box_s = reinterpret_cast<float4 *>(tab + kTabRow * 3 * KM);       // [nblk_max][2]
     double4 *atom_s = reinterpret_cast<double4 *>(box_s + 2 * nblk_max);      // [nown_max]
     int2 *meta_s = reinterpret_cast<int2 *>(atom_s + A.nown_max);             // [nown_max]
-    int *queue = reinterpret_cast<int *>(meta_s + A.nown_max);                // [qcap]
-    int *nearbuf = queue + ((A.qcap + 1) & ~1);                               // [B/32][32 kCPT]
-    double *red = reinterpret_cast<double *>(nearbuf + B * kCPT);             // [B/32][kNV]
-    // the mixed form's rho refresh reuses the pair queue and near buffer as atom phase tables
-    double2 *scr = reinterpret_cast<double2 *>((reinterpret_cast<uintptr_t>(queue) + 15) & ~uintptr_t(15));
+    int *wbuf = reinterpret_cast<int *>(meta_s + A.nown_max);                 // [wbuf_ints]: the warps' near atoms and pairs
+    double *red = reinterpret_cast<double *>(wbuf + wbuf_ints(B, D.kmax));    // [B/32][kNV]
+    // the mixed form's rho refresh reuses the warps' buffers as atom phase tables
+    double2 *scr = reinterpret_cast<double2 *>((reinterpret_cast<uintptr_t>(wbuf) + 15) & ~uintptr_t(15));
     const int scr_atoms = (int)(((reinterpret_cast<char *>(red) - reinterpret_cast<char *>(scr))) /
                                 (long)(sizeof(double2) * 3 * KM + sizeof(double) + sizeof(int)));
     double *xch = red + (B / 32) * kNV;                                       // [2][G][kNV]
     double *lj_s = xch + 2 * G * kNV;                                         // [2][nt*nt]
     double *dhs_ts = lj_s + 2 * nt * nt;                                      // [nt+1] hard core by LJ type
-    int *blist = reinterpret_cast<int *>(dhs_ts + nt + 1);                    // [nblk_max + 32] near blocks
 
     // atoms of this CTA: j = rank + G * i (interleaved, so every CTA holds a spatial mix), in
     // the spatial order of k_stage_order (slot D.slot[j]), with the bounding box of every kBlk slots
@@ -1478,8 +1461,8 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
         sh.mic = D.cnt[CN_MOVE_IN_CYCLE];
         sh.cursor = run->cursor;
         sh.last_mol = -1;
+        sh.view = StageView{atom_s, meta_s, box_s, dhs_ts, lj_s, red, wbuf, nown, rank, G};
         sh.abort = 0;
-        sh.qcount = 0;
         sh.wnext = 0;
         sh.icur = 0;
         sh.spec_ok = 0;
@@ -1508,11 +1491,10 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
         if (lane == 0) { sh.wbase[0] = base; sh.wn[0] = nw; sh.wbase[1] = -1; sh.wn[1] = 0; sh.wnext = 1; }
     }
     __syncthreads();
-    const bool biased = SPLIT && (D.xlf > 0.0 || D.xlc > 0.0);
+    constexpr bool biased = SPLIT;  // (the SPLIT variant runs exactly the systems with a force bias)
     // the next move is prepared while the workers run the current pass: chosen and proposed for
     // unbiased moves, only chosen for force-biased ones (their proposal needs the old forces)
-    const bool choose_only = biased;
-    const bool speculate = !SPLIT || choose_only;
+    constexpr bool choose_only = biased;
     const ChooseCtx X{&D, run, rwin[0], rwin[1], atom_s, G};
 
     long long moves_done = 0;
@@ -1533,6 +1515,7 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
         if (pc) t_mark = clock64();
         R2 *mold_g = scratch_buf<MX>(D.scratch, 0, 1 + NT, S);  // the moved molecule's old phase sums
         if (!have_next) {
+            __syncthreads();  // every thread has read what the last decision left in sh
             // choose the molecule and stage its atoms (no move in flight)
             if (tid == 0) {
                 Cand &C = sh.cand[sh.icur];
@@ -1540,7 +1523,7 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
                 RngReader rng = make_reader(X, sh, sh.cursor);
                 int imol = draw_molecule(D, rng, sh.mic == 0);
                 C.valid = imol > 0;
-                C.cur_prop = rng.cur;
+                C.cur_prop = rng.cur();
                 if (!imol) imol = 1;
                 stage_molecule(X, sh, C, imol, -1, nullptr, cluster);
                 sh.abort = C.valid ? 0 : kAbortStream;
@@ -1552,89 +1535,94 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
         if (!have_next || choose_only) {
             const int na0 = sh.cand[sh.icur].na;
             // old forces for force-biased moves (movemc Steps 3-4)
-            if constexpr (SPLIT) if (biased) {
-                if (!ctl) worker_pass<NT, EPT, PASS_OLD, true, MX>(D, sh, R, tab, atom_s, dhs_ts, D.dhs, D.dhs_typed, rank, G, meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, A.qcap, e0, gwork, prof, mold_g);
+            if constexpr (biased) {
+                if (!ctl) worker_pass<NT, EPT, PASS_OLD, MX>(D, sh, R, tab, e0, gwork, prof, mold_g);
                 __syncthreads();
                 reduce_pass(sh, red, xch, RV_F + 3 * na0, G, rank, xpar, cluster);
                 xpar ^= 1;
                 __syncthreads();
                 YAMC_PH(PH_OLD_PASS);  // the force-biased old pass and its reduction (the control warp's view)
-                if (tid == 0) {
-                    sh.eold[0] = sh.tot[RV_EW]; sh.eold[1] = sh.tot[RV_LJ6]; sh.eold[2] = sh.tot[RV_LJ12];
-                    for (int a = 0; a < na0; ++a) {  // external-field force -2 kext q mu (MC.f90:988-997)
-                        const double q = sh.cand[sh.icur].slot[na0 + a].q;
-                        sh.fold[3 * a] = sh.tot[RV_F + 3 * a] + D.m2k * q * sh.sc[SC_MU_X];
-                        sh.fold[3 * a + 1] = sh.tot[RV_F + 3 * a + 1] + D.m2k * q * sh.sc[SC_MU_Y];
-                        sh.fold[3 * a + 2] = sh.tot[RV_F + 3 * a + 2] + D.m2k * q * sh.sc[SC_MU_Z];
-                    }
-                }
             }
             // the proposal (movemc Step 5)
-            if (biased) {
-                // on two warps: thread 0 draws the displacement (its Newton iteration is the long
-                // serial part) while thread 32 skips the displacement's draws and draws the rotation;
-                // both read the old forces thread 0 has just written
-                __syncthreads();
-                if (tid == 0 || tid == 32) {
+            if constexpr (biased) {
+                // on two warps: warp 0 draws the displacement (its Newton iteration is the long serial
+                // part) while warp 1 skips the displacement's draws and draws the rotation; all lanes of
+                // a warp run the same code on the same data, which lets them share the sum of the
+                // rotation's bias term (shi_sans_exp_warp)
+                if (tid < 64) {
                     const Cand &C = sh.cand[sh.icur];
                     double F[3], T[3];
-                    // (old positions and forces read where they are, in shared memory)
                     const Slot *os = C.slot + na0;
+                    // the old forces with the external field -2 kext q mu (MC.f90:988-997)
                     mol_force_torque_f(na0, [&](int i, int d) { return d == 0 ? os[i].x : (d == 1 ? os[i].y : os[i].z); },
-                                       C.mass, [&](int i, int d) { return sh.fold[3 * i + d]; }, F, T);
+                                       C.mass, [&](int i, int d) { return sh.tot[RV_F + 3 * i + d] + D.m2k * os[i].q * sh.sc[SC_MU_X + d]; },
+                                       F, T);
                     RngReader rng = make_reader(X, sh, C.cur_prop);
-                    if (tid == 0) {
-                        MoveState &m = sh.cand[sh.icur].mv;
-                        mcm_init_old(m, F, T);
+                    MoveState m;
+                    mcm_init_old(m, F, T);
+                    if (tid < 32) {
                         mcm_choose_displacement(m, rng, D.xlf, D.dr);
-                        sh.disp_end = rng.cur;
-                        sh.disp_out = rng.out;
+                        if (lane == 0) {
+                            sh.eold[0] = sh.tot[RV_EW]; sh.eold[1] = sh.tot[RV_LJ6]; sh.eold[2] = sh.tot[RV_LJ12];
+                            MoveState &d = sh.cand[sh.icur].mv;
+                            d.fxo = m.fxo; d.fyo = m.fyo; d.fzo = m.fzo; d.cxo = m.cxo; d.cyo = m.cyo; d.czo = m.czo; d.co = m.co;
+                            d.umaxold = m.umaxold; d.cold = m.cold; d.deltx = m.deltx; d.delty = m.delty; d.deltz = m.deltz;
+                            sh.disp_end = rng.cur();
+                            sh.disp_out = rng.out;
+                        }
                     } else {
-                        MoveState &mr = sh.mrot;
-                        mcm_init_old(mr, F, T);
-                        mcm_skip_displacement(mr, rng, D.xlf, D.dr);
-                        sh.rot_start = rng.cur;
-                        if (!rng.out) mcm_choose_rotation(mr, rng, D.xlc, D.d_angle);
-                        sh.rot_end = rng.cur;
-                        sh.rot_out = rng.out;
+                        mcm_skip_displacement(m, rng, D.xlf, D.dr);
+                        const long long start = rng.cur();
+                        if (!rng.out) mcm_choose_rotation(m, rng, D.xlc, D.d_angle, shi_sans_exp_warp, PickWarp());
+                        if (lane == 0) {
+                            copy_rotation(sh.mrot, m);
+                            sh.rot_start = start;
+                            sh.rot_end = rng.cur();
+                            sh.rot_out = rng.out;
+                        }
                     }
                 }
                 __syncthreads();
-                if (tid == 0) {
+                if (ctl) {
                     Cand &C = sh.cand[sh.icur];
                     MoveState &m = C.mv;
                     bool out = sh.disp_out != 0;
                     long long cur = sh.disp_end;
                     if (!out) {
                         if (sh.rot_start == sh.disp_end) {
-                            copy_rotation(m, sh.mrot);
+                            if (lane == 0) copy_rotation(m, sh.mrot);
                             cur = sh.rot_end;
                             out = sh.rot_out != 0;
                         } else {  // (the skip always draws what the displacement draws; kept as a guard)
                             RngReader rng = make_reader(X, sh, sh.disp_end);
-                            mcm_choose_rotation(m, rng, D.xlc, D.d_angle);
-                            cur = rng.cur;
+                            MoveState r;
+                            r.cxo = m.cxo; r.cyo = m.cyo; r.czo = m.czo; r.co = m.co;
+                            mcm_choose_rotation(r, rng, D.xlc, D.d_angle, shi_sans_exp_warp, PickWarp());
+                            if (lane == 0) copy_rotation(m, r);
+                            cur = rng.cur();
                             out = rng.out != 0;
                         }
+                        __syncwarp();
                     }
-                    if (out) {
-                        C.valid = 0;
-                        sh.abort = kAbortStream;
-                    } else {
-                        // old positions from slots [na0, 2 na0), new ones into [0, na0): no overlap
-                        const Slot *os = C.slot + na0;
-                        Slot *ns = C.slot;
-                        place_molecule_f(m, na0, [&](int i, int d) { return d == 0 ? os[i].x : (d == 1 ? os[i].y : os[i].z); },
-                                         C.mass, [&](int i, double x, double y, double z) { ns[i].x = x; ns[i].y = y; ns[i].z = z; });
-                        C.cur_prop = cur;
+                    if (lane == 0) {
+                        if (out) {
+                            C.valid = 0;
+                            sh.abort = kAbortStream;
+                        } else {
+                            // old positions from slots [na0, 2 na0), new ones into [0, na0): no overlap
+                            const Slot *os = C.slot + na0;
+                            Slot *ns = C.slot;
+                            place_molecule_f(m, na0, [&](int i, int d) { return d == 0 ? os[i].x : (d == 1 ? os[i].y : os[i].z); },
+                                             C.mass, [&](int i, double x, double y, double z) { ns[i].x = x; ns[i].y = y; ns[i].z = z; });
+                            C.cur_prop = cur;
+                        }
                     }
                 }
             } else if (tid == 0) {
                 Cand &C = sh.cand[sh.icur];
                 RngReader rng = make_reader(X, sh, C.cur_prop);
-                const double Z[3] = {0, 0, 0};
-                propose(D, C, rng, Z, Z);
-                C.cur_prop = rng.cur;
+                propose(D, C, rng);
+                C.cur_prop = rng.cur();
                 if (rng.out) { C.valid = 0; sh.abort = kAbortStream; }
             }
             __syncthreads();
@@ -1646,9 +1634,9 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
 
         // ------------------------------------------------ the pass over the new positions
         if (!ctl) {
-            if constexpr (SPLIT) worker_pass<NT, EPT, PASS_NEW, true, MX>(D, sh, R, tab, atom_s, dhs_ts, D.dhs, D.dhs_typed, rank, G, meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, A.qcap, e0, gwork, prof, mold_g);
-            else worker_pass<NT, EPT, PASS_BOTH, false, MX>(D, sh, R, tab, atom_s, dhs_ts, D.dhs, D.dhs_typed, rank, G, meta_s, box_s, blist, queue, nearbuf, red, lj_s, nown, A.qcap, e0, gwork, prof, mold_g);
-        } else if (speculate && it + 1 < n_moves) {
+            if constexpr (SPLIT) worker_pass<NT, EPT, PASS_NEW, MX>(D, sh, R, tab, e0, gwork, prof, mold_g);
+            else worker_pass<NT, EPT, PASS_BOTH, MX>(D, sh, R, tab, e0, gwork, prof, mold_g);
+        } else if (it + 1 < n_moves) {
             // prepare the next move's candidates while the workers run: lanes 1-2 after the
             // acceptance draw, lane 2 with the molecule in flight at its proposed positions (used
             // only if it is chosen again and accepted)
@@ -1681,14 +1669,13 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
                 Cand &C = sh.cand[buf];
                 RngReader rng = make_reader(X, sh, c1);
                 (void)rng.next();  // the acceptance draw (MonteCarloMove.f90:553)
-                C.cur_start = rng.cur;
+                C.cur_start = rng.cur();
                 const int imol = rng.out ? 0 : draw_molecule(D, rng, next_cycle);
                 C.valid = imol > 0;
                 const Slot *moving = (lane == 2) ? &M.slot[0] : &M.slot[M.na];
                 stage_molecule(X, sh, C, imol > 0 ? imol : 1, M.imol - 1, moving, cluster);
-                const double Z[3] = {0, 0, 0};
-                if (C.valid && !choose_only) propose(D, C, rng, Z, Z);
-                C.cur_prop = rng.cur;
+                if constexpr (!SPLIT) if (C.valid) propose(D, C, rng);
+                C.cur_prop = rng.cur();
                 if (rng.out) C.valid = 0;
             }
             if (pc) { const long long t_now = clock64(); prof[PH_SPECULATE] += t_now - t_mark; t_mark = t_now; }
@@ -1699,18 +1686,24 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
         YAMC_PH(PH_REDUCE);
 
         // ------------------------------------------------ Metropolis (Steps 7-13) and commit (Step 14)
-        if (tid == 0) {
+        // The control warp decides (all lanes on the same data); what the next move waits for is written
+        // before the barrier, the books are kept after it, beside the workers' commit and next pass.
+        bool overlap = false;
+        int flags = 0, acc = 0;
+        double du_real = 0, du_kc = 0, du_kl = 0, du_ext = 0, dmx = 0, dmy = 0, dmz = 0, dew = 0, dlj6 = 0, dlj12 = 0;
+        long long cur_after = 0;
+        int imol_moved = 0;
+        if (ctl) {
+            __syncwarp();  // (the lanes have written sh.tot)
             const Cand &M = sh.cand[sh.icur];
-            const bool overlap = sh.tot[RV_OVL] > 0.0;
-            int flags = overlap ? 2 : 0;
-            double du_real = 0, du_kc = 0, du_kl = 0, du_ext = 0, dmx = 0, dmy = 0, dmz = 0;
-            double dew = 0, dlj6 = 0, dlj12 = 0;
-            int acc = 0;
-            long long cur_after = M.cur_prop;
-            bool out = false;
+            overlap = sh.tot[RV_OVL] > 0.0;
+            flags = overlap ? 2 : 0;
+            cur_after = M.cur_prop;
+            imol_moved = M.imol;
+            bool out = false, finite = true;
             if (!overlap) {
                 RngReader rng = make_reader(X, sh, M.cur_prop);
-                if (biased) {
+                if constexpr (biased) {
                     dew = sh.tot[RV_EW] - sh.eold[0]; dlj6 = sh.tot[RV_LJ6] - sh.eold[1]; dlj12 = sh.tot[RV_LJ12] - sh.eold[2];
                     du_real = (sh.tot[RV_EW] + sh.tot[RV_LJ12] - sh.tot[RV_LJ6]) - (sh.eold[0] + sh.eold[2] - sh.eold[1]);
                 } else {
@@ -1725,87 +1718,92 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
                 const double mux = sh.sc[SC_MU_X], muy = sh.sc[SC_MU_Y], muz = sh.sc[SC_MU_Z];
                 // EwaldSumExternal_calc_dU (EwaldSumExternal.f90:68-82)
                 du_ext = D.kext * ((2 * mux + dmx) * dmx + (2 * muy + dmy) * dmy + (2 * muz + dmz) * dmz);
-                double F[3] = {0, 0, 0}, T[3] = {0, 0, 0};
-                if (biased) {
-                    // (loops over kMaxA with constant indices: the arrays stay in registers)
-                    double fx[kMaxA], fy[kMaxA], fz[kMaxA], x[kMaxA], y[kMaxA], z[kMaxA];
-#pragma unroll
-                    for (int a = 0; a < kMaxA; ++a) {
-                        const int b = a < na ? a : 0;
-                        const double q = M.slot[b].q;
-                        fx[a] = sh.tot[RV_F + 3 * b] + D.m2k * q * (mux + dmx);
-                        fy[a] = sh.tot[RV_F + 3 * b + 1] + D.m2k * q * (muy + dmy);
-                        fz[a] = sh.tot[RV_F + 3 * b + 2] + D.m2k * q * (muz + dmz);
-                        x[a] = M.slot[b].x; y[a] = M.slot[b].y; z[a] = M.slot[b].z;
-                    }
-                    mol_force_torque(na, x, y, z, M.mass, fx, fy, fz, F, T);
-                }
                 const double du_total = du_real + (du_kc + du_kl) + du_ext;
                 // a non-finite energy change or bias force (an input the arithmetic cannot take:
                 // NaN positions or random numbers, coincident charges) stops the chain before
                 // the move is decided, with the state as it was after the last completed move
-                bool finite = isfinite(du_total);
-                if (biased)
+                finite = isfinite(du_total);
+                if constexpr (biased) {
+                    double F[3], T[3];
+                    const double mu[3] = {mux + dmx, muy + dmy, muz + dmz};
+                    const Slot *ns = M.slot;
+                    mol_force_torque_f(na, [&](int i, int d) { return d == 0 ? ns[i].x : (d == 1 ? ns[i].y : ns[i].z); }, M.mass,
+                                       [&](int i, int d) { return sh.tot[RV_F + 3 * i + d] + D.m2k * ns[i].q * (d == 0 ? mu[0] : (d == 1 ? mu[1] : mu[2])); },
+                                       F, T);
                     for (int c = 0; c < 3; ++c) finite = finite && isfinite(F[c]) && isfinite(T[c]);
-                if (!finite) { sh.abort = kAbortNonFinite; sh.accepted = 0; goto decided; }
-                if (biased || SPLIT) {
-                    // (the bias state in shared memory, where the proposal left it: no copy to spill)
-                    MoveState &mv = sh.cand[sh.icur].mv;
-                    mcm_init_new(mv, F, T, D.xlf, D.xlc, D.dr, D.d_angle);
-                    acc = mcm_accept(mv, du_total, D.xlf, D.xlc, rng);
-                } else {
+                    if (finite) {
+                        const BiasNew b = mcm_init_new(F, T, D.xlf, D.xlc, D.dr, D.d_angle, shi_sans_exp_warp);
+                        acc = mcm_accept(M.mv, F, T, b, du_total, D.xlf, D.xlc, rng);
+                    }
+                } else if (finite) {
                     // MonteCarloMove_accept_or_decline without bias: every bias term is an exact 0
                     // or 1 (cold = qold = cnew = qnew = 1), so the factor is exp(-dU) bit for bit
-                    const double factor = exp(-du_total);
+                    const double factor = c_exp(-du_total);
                     acc = rng.next() > factor ? 0 : 1;
                 }
                 out = rng.out != 0;
-                cur_after = rng.cur;
+                cur_after = rng.cur();
                 flags |= acc;
             }
-            sh.accepted = 0;
-            sh.imoved = sh.icur;
-            if (out) {
-                sh.abort = kAbortStream;  // the interrupted move restarts from its first draw (sh.cursor unchanged)
-            } else {
+            if (out) acc = 0;
+            __syncwarp();
+            if (lane == 0) {
                 sh.accepted = acc;
+                if (!finite) sh.abort = kAbortNonFinite;
+                else if (out) sh.abort = kAbortStream;  // the interrupted move restarts from its first draw (sh.cursor unchanged)
+                else {
+                    if (acc) {
+                        sh.last_mol = M.imol - 1;
+                        for (int a = 0; a < na; ++a) {
+                            sh.lx[a] = M.slot[a].x; sh.ly[a] = M.slot[a].y; sh.lz[a] = M.slot[a].z;
+                            sh.mv_slot[a] = M.slot[a].pad;
+                        }
+                        const MolK<MX> mk(M.slot, na);
+                        sh.mv_first = M.first; sh.mv_na = na; sh.mv_tmask = mk.tmask; sh.mv_simple = mk.simple;
+                    }
+                    sh.cursor = cur_after;
+                    // the next move: the prepared candidate that matches what happened
+                    sh.spec_ok = 0;
+                    if (it + 1 < n_moves) {
+                        const int sel = overlap ? 0 : ((acc && sh.cand[sh.spec[2]].imol == M.imol) ? 2 : 1);
+                        const int buf = sh.spec[sel];
+                        const Cand &C = sh.cand[buf];
+                        if (C.valid && C.cur_start == cur_after) {
+                            sh.icur = buf;
+                            sh.spec_ok = 1;
+                        }
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        YAMC_PH(PH_DECIDE);
+        if (sh.abort) break;
+        const bool accepted = sh.accepted != 0;
+        if (ctl) {
+            // the totals, the log, the cycle counters and energy.dat rows (runmc.f90:230-279)
+            if (lane == 0) {
                 if (acc) {
                     sh.sc[SC_UU_EW] += dew; sh.sc[SC_UU_LJ6] += dlj6; sh.sc[SC_UU_LJ12] += dlj12;
                     sh.sc[SC_EK_C] += du_kc; sh.sc[SC_EK_LJ] += du_kl;
                     sh.sc[SC_MU_X] += dmx; sh.sc[SC_MU_Y] += dmy; sh.sc[SC_MU_Z] += dmz;
                     sh.sc[SC_N_MV_ACC] += 1.0;
-                    sh.last_mol = M.imol - 1;
-                    for (int a = 0; a < na; ++a) { sh.lx[a] = M.slot[a].x; sh.ly[a] = M.slot[a].y; sh.lz[a] = M.slot[a].z; }
-                    // this CTA's staged copy of the moved atoms; every reader of the old copy (this
-                    // move's pass, the candidates prepared during it, in any CTA) has passed the barriers
-                    for (int a = 0; a < na; ++a) {
-                        const int j = M.first + a;
-                        if (j % G == rank) {
-                            const int sl = (int)YAMC_IX(M.slot[a].pad, nown);  // the atom's staging slot
-                            double4 p = atom_s[sl];
-                            p.x = M.slot[a].x; p.y = M.slot[a].y; p.z = M.slot[a].z;
-                            atom_s[sl] = p;
-                            box_expand(box_s, sl / kBlk, p.x, p.y, p.z);
-                        }
-                    }
                     ++n_acc;
                 }
                 sh.sc[SC_N_MV_STEPS] += 1.0;
-                sh.cursor = cur_after;
                 if (rank == 0) {
                     if (acc)
                         for (int a = 0; a < na; ++a) {  // x, y, z of the double4 (q unchanged): no read
-                            double *pa = reinterpret_cast<double *>(D.atom + M.first + a);
-                            pa[0] = M.slot[a].x; pa[1] = M.slot[a].y; pa[2] = M.slot[a].z;
+                            double *pa = reinterpret_cast<double *>(D.atom + sh.mv_first + a);
+                            pa[0] = sh.lx[a]; pa[1] = sh.ly[a]; pa[2] = sh.lz[a];
                         }
                     if (run->log) {
                         yamc_move_record rec;
-                        rec.imol = M.imol; rec.flags = flags; rec.cursor = cur_after;
+                        rec.imol = imol_moved; rec.flags = flags; rec.cursor = cur_after;
                         rec.du_real = du_real; rec.du_k_coul = du_kc; rec.du_k_lj = du_kl; rec.du_ext = du_ext;
                         run->log[it] = rec;
                     }
                 }
-                // cycle bookkeeping and energy.dat rows (runmc.f90:230-279)
                 sh.mic += 1;
                 if (sh.mic == D.M) {
                     sh.mic = 0;
@@ -1823,59 +1821,54 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
                     }
                     sh.icycle += 1;
                 }
-                // the next move: the prepared candidate that matches what happened
-                sh.spec_ok = 0;
-                if (speculate && it + 1 < n_moves) {
-                    const int sel = overlap ? 0 : ((acc && sh.cand[sh.spec[2]].imol == M.imol) ? 2 : 1);
-                    const int buf = sh.spec[sel];
-                    const Cand &C = sh.cand[buf];
-                    if (C.valid && C.cur_start == sh.cursor) {
-                        sh.icur = buf;
-                        sh.spec_ok = 1;
-                    }
-                }
             }
-        decided:;
-        }
-        __syncthreads();
-        YAMC_PH(PH_DECIDE);
-        if (sh.abort) break;
-        if (sh.accepted) {
+            __syncwarp();
+        } else if (accepted) {
+            // this CTA's staged copy of the moved atoms, by one thread of the last warp (two atoms may
+            // share a block's box); the workers read it after the phase tables' barrier, and another CTA
+            // that stages the molecule meanwhile takes its positions from sh.lx (last_mol)
+            if (wtid == nwork - 1)
+                for (int a = 0; a < sh.mv_na; ++a) {
+                    if ((sh.mv_first + a) % G != rank) continue;
+                    const int sl = (int)YAMC_IX(sh.mv_slot[a], nown);  // the atom's staging slot
+                    double4 p = atom_s[sl];
+                    p.x = sh.lx[a]; p.y = sh.ly[a]; p.z = sh.lz[a];
+                    atom_s[sl] = p;
+                    box_expand(box_s, sl / kBlk, p.x, p.y, p.z);
+                }
             // commit: rho += delta (MC.f90:1245), in registers or in memory by the entry's owner; the
             // rows of LJ types that the molecule does not carry have no delta
-            const MolK<MX> mk(sh.cand[sh.imoved].slot, sh.cand[sh.imoved].na);
+            const int tmask = sh.mv_tmask;
+            const bool simple = sh.mv_simple != 0;
             static_for<0, EPT>([&](auto kc) {
                 constexpr int k = decltype(kc)::value;
                 R.rho[k][0].x += R.dl[k][0].x; R.rho[k][0].y += R.dl[k][0].y;
 #pragma unroll
                 for (int t = 1; t <= NT; ++t) {
-                    const Rt dx = pick<Rt>(mk.simple, R.dl[k][1].x, R.dl[k][t].x), dy = pick<Rt>(mk.simple, R.dl[k][1].y, R.dl[k][t].y);
-                    const bool hit = (mk.tmask >> (t - 1)) & 1;
+                    const Rt dx = pick<Rt>(simple, R.dl[k][1].x, R.dl[k][t].x), dy = pick<Rt>(simple, R.dl[k][1].y, R.dl[k][t].y);
+                    const bool hit = (tmask >> (t - 1)) & 1;
                     R.rho[k][t].x += hit ? (double)dx : 0.0; R.rho[k][t].y += hit ? (double)dy : 0.0;
                 }
             });
             if constexpr (EPT <= 0) {
-                if (!ctl) {
-                    const R2 *dl_g = scratch_buf<MX>(D.scratch, 1, 1 + NT, S);
-                    for (int e = e0; e < S; e += gwork)
+                const R2 *dl_g = scratch_buf<MX>(D.scratch, 1, 1 + NT, S);
+                for (int e = e0; e < S; e += gwork)
 #pragma unroll
-                        for (int t = 0; t <= NT; ++t) {
-                            if (t > 0 && !((mk.tmask >> (t - 1)) & 1)) continue;
-                            double2 r = D.rho[(size_t)t * S + e];
-                            const double2 d = to_d2(dl_g[(size_t)t * S + e]);
-                            r.x += d.x; r.y += d.y;
-                            D.rho[(size_t)t * S + e] = r;
-                            if constexpr (MX) D.rho_f[(size_t)t * S + e] = make_float2((float)r.x, (float)r.y);
-                        }
-                }
+                    for (int t = 0; t <= NT; ++t) {
+                        if (t > 0 && !((tmask >> (t - 1)) & 1)) continue;
+                        double2 r = D.rho[(size_t)t * S + e];
+                        const double2 d = to_d2(dl_g[(size_t)t * S + e]);
+                        r.x += d.x; r.y += d.y;
+                        D.rho[(size_t)t * S + e] = r;
+                        if constexpr (MX) D.rho_f[(size_t)t * S + e] = make_float2((float)r.x, (float)r.y);
+                    }
             }
         }
         ++moves_done;
         have_next = sh.spec_ok != 0;
-        __syncthreads();
         YAMC_PH(PH_COMMIT);
         if constexpr (MX) {
-            acc_since += sh.accepted;  // the same decisions in every CTA: every thread agrees
+            acc_since += accepted;  // the same decisions in every CTA: every thread agrees
             if (refresh_every > 0 && acc_since >= refresh_every) {
                 refresh_in_chain<NT, EPT>(D, scr, scr_atoms, e0, gwork, G, rank, sh, red, xch, xpar, cluster);
                 static_for<0, EPT>([&](auto kc) {

@@ -99,33 +99,48 @@ __host__ __device__ inline R rsq(R y) {
 #endif
 }
 
+// The long functions of the control code (proposal, acceptance), one copy each: the control warp runs
+// through its code once per move, so what it costs is largely the instructions it fetches, and an
+// inlined exp, log or FP64 division is 20 to 100 of them.
+static __host__ __device__ __noinline__ double c_exp(double x) { return exp(x); }
+static __host__ __device__ __noinline__ double c_log(double x) { return log(x); }
+static __host__ __device__ __noinline__ double c_sqrt(double x) { return sqrt(x); }
+static __host__ __device__ __noinline__ double c_div(double a, double b) { return a / b; }
+static __host__ __device__ __noinline__ double2 c_sincos(double x) { double2 r; sincos(x, &r.x, &r.y); return r; }  // (sin, cos)
+
 // ------------------------------------------------------------------ Functions.f90
 // erfc_Luc / erf_Luc (Functions.f90:116-171): Taylor series below 0.455,
 // Abramowitz & Stegun 7.1.26 up to 3, asymptotic series above (divisions by
 // multiplications with reciprocals, see rcp above).
+// The two outer pieces share one reciprocal without a branch (the lanes of a warp are on both sides
+// of 3 wherever the cutoff is): t = 1 / (1 + P x), or 1 / (sqrt(pi) x^3), which gives both
+// reciprocals of the asymptotic piece.
 template <class R>
-__host__ __device__ inline R d_erfc_luc(R x, R x2, R ee2) {
+__host__ __device__ inline R d_erfc_luc_outer(R x, R x2, R ee2) {
     const R P = R(0.3275911), A1 = R(0.254829592), A2 = R(-0.284496736), A3 = R(1.421413741),
             A4 = R(-1.453152027), A5 = R(1.061405429), pi05 = R(1.7724538509055);
-    if (x < R(0.455)) return R(1) - R(2) / pi05 * x * (R(1) - x2 * (R(1) / R(3) - x2 * (R(0.1) - x2 * (R(1) / R(42) - x2 * (R(1) / R(216))))));
-    if (x > R(3)) {
-        const R i2 = rcp(x2);
-        return (R(1) - R(0.5) * (R(1) - R(1.5) * i2) * i2) * rcp(pi05 * x) * ee2;
-    }
-    const R t = rcp(R(1) + P * x);
-    return t * (A1 + t * (A2 + t * (A3 + t * (A4 + t * A5)))) * ee2;
+    const bool far = x > R(3);
+    const R px = pi05 * x;
+    const R t = rcp(far ? px * x2 : R(1) + P * x);
+    const R i2 = t * px;
+    const R mid = A1 + t * (A2 + t * (A3 + t * (A4 + t * A5)));
+    const R asy = x2 * (R(1) - R(0.5) * (R(1) - R(1.5) * i2) * i2);
+    return t * (far ? asy : mid) * ee2;
+}
+template <class R>
+__host__ __device__ inline R d_erf_luc_series(R x, R x2) {
+    const R pi05 = R(1.7724538509055);
+    return R(2) / pi05 * x * (R(1) - x2 * (R(1) / R(3) - x2 * (R(0.1) - x2 * (R(1) / R(42) - x2 * (R(1) / R(216))))));
+}
+template <class R>
+__host__ __device__ inline R d_erfc_luc(R x, R x2, R ee2) {
+    if (x < R(0.455)) return R(1) - d_erf_luc_series(x, x2);
+    return d_erfc_luc_outer(x, x2, ee2);
 }
 template <class R>
 __host__ __device__ inline R d_erf_luc(R x, R x2, R ee2) {
-    const R P = R(0.3275911), A1 = R(0.254829592), A2 = R(-0.284496736), A3 = R(1.421413741),
-            A4 = R(-1.453152027), A5 = R(1.061405429), pi05 = R(1.7724538509055);
-    if (x < R(0.455)) return R(2) / pi05 * x * (R(1) - x2 * (R(1) / R(3) - x2 * (R(0.1) - x2 * (R(1) / R(42) - x2 * (R(1) / R(216))))));
-    if (x > R(3)) {
-        const R i2 = rcp(x2);
-        return R(1) - (R(1) - R(0.5) * (R(1) - R(1.5) * i2) * i2) * rcp(pi05 * x) * ee2;
-    }
-    const R t = rcp(R(1) + P * x);
-    return R(1) - t * (A1 + t * (A2 + t * (A3 + t * (A4 + t * A5)))) * ee2;
+    if (x < R(0.455)) return d_erf_luc_series(x, x2);
+    return R(1) - d_erfc_luc_outer(x, x2, ee2);
 }
 
 // d erfc_Luc(x) / dx of the piecewise function above, piece by piece: the adjoint of the
@@ -175,7 +190,7 @@ __host__ __device__ inline R pair_force_adjoint(R r2, R qq_xclb, bool lj, R sigm
 }
 
 // shi_sans_exp_f (Functions.f90:225-289): Shi(x) exp(-x), force-bias acceptance
-__host__ __device__ inline double d_shi_sans_exp(double x) {
+static __host__ __device__ __noinline__ double d_shi_sans_exp(double x) {
     const double dx0 = 0.2;
     double shi_f, x1;
     if (x <= 1.0) {
@@ -211,6 +226,34 @@ __host__ __device__ inline double d_shi_sans_exp(double x) {
     shi_f = shi_f - dx * s / t / 2.0 - dx * dx / 12.0 * (cosh(t) / t - s / (t * t));
     return exp(-x) * shi_f;
 }
+
+#ifdef __CUDACC__
+// The same function by a whole warp (the same x in every lane, the same value back): a lane takes one
+// term of the trapezoid sum, up to 26 of them with a sinh and a division each, which one thread adds
+// in 5 k cycles and more.  sinh and cosh from one exponential (all arguments are 1 or more).
+__device__ inline double shi_sans_exp_warp(double x) {
+    if (!(x > 1.0) || x > 20.0) return d_shi_sans_exp(x);
+    const double dx0 = 0.2;
+    double shi_f, x1;
+    if (x < 5.0) { x1 = 1.0; shi_f = 1.057250875; }
+    else if (x < 10.0) { x1 = 5.0; shi_f = 20.093211826; }
+    else if (x < 15.0) { x1 = 10.0; shi_f = 1246.11449; }
+    else { x1 = 15.0; shi_f = 117477.926; }
+    const int n = (int)((x - x1) / dx0 + 2);  // 2..27: lane l holds t_(l + 2), lane 31 x1
+    const double dx = c_div(x - x1, (double)(n - 1));
+    const int lane = threadIdx.x & 31;
+    const double t = lane == 31 ? x1 : x1 + (double)(lane + 1) * dx;
+    const double e = c_exp(t), r = c_div(1.0, e), sh = 0.5 * (e - r), ch = 0.5 * (e + r);
+    const double it = c_div(1.0, t), a = sh * it, b = (ch - a) * it;  // sinh / t, (cosh t - sinh) / t^2
+    double sum = lane < n - 1 ? dx * a : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const double a1 = __shfl_sync(0xffffffffu, a, 31), b1 = __shfl_sync(0xffffffffu, b, 31);
+    const double an = __shfl_sync(0xffffffffu, a, n - 2), bn = __shfl_sync(0xffffffffu, b, n - 2);
+    shi_f = shi_f + dx * a1 / 2.0 + dx * dx / 12.0 * b1 + sum - dx * an / 2.0 - dx * dx / 12.0 * bn;
+    return c_exp(-x) * shi_f;
+}
+#endif
 
 // ------------------------------------------------------------------ pair term
 // RealSumLocal (RealSumLocal.f90:63-168): one pair of the real-space sum.
@@ -309,32 +352,35 @@ __host__ __device__ inline void entry_phase(const T2 *tx, const T2 *ty, const T2
 // ------------------------------------------------------------------ random stream
 // rand() of random.f90:65-93: successive REAL(4) random_number values, values
 // outside [1e-14, 1-1e-14] are drawn again.  The buffer holds the raw stream.
-// One stretch of the stream [wb, wb + wn) may be read from a copy (a window in shared memory on
-// the device) instead of the buffer.
+// The reader stands at position wb + k; [wb, wb + wn) may be read from a copy (a window in shared
+// memory on the device), the rest from the buffer.
 struct RngReader {
     const float *buf;  // holds stream positions [off, n)
     long long off;
     long long n;       // end of the stream available
-    long long cur;     // next position to read
+    const float *w;    // the window
+    long long wb;
+    int wn;
+    int k;
     int out;           // set once the stream ran out
-    const float *w = nullptr;
-    long long wb = 0;
-    int wn = 0;
+    __host__ __device__ inline long long cur() const { return wb + k; }
     __host__ __device__ inline float raw() {
-        if (cur >= n) { out = 1; return 0.5f; }
-        const long long i = cur++;
-        const unsigned long long k = (unsigned long long)(i - wb);
-        return k < (unsigned long long)wn ? w[k] : buf[i - off];
+        float v = 0.5f;
+        if (k < wn) v = w[k];
+        else if (wb + k < n) v = buf[wb + k - off];
+        else { out = 1; return v; }
+        ++k;
+        return v;
     }
     // (the limits 1e-14 and 1 - 1e-14 are FP64: a float is below the first exactly when it is below
     // the first float that is not, and above the second exactly when it is 1 or more)
     __host__ __device__ inline double next() {
         constexpr float lo = 1e-14f;
-        float v = 0.0f;
-        while (((double)lo < 1e-14 ? v <= lo : v < lo) || v >= 1.0f) {
+        float v;
+        do {
             v = raw();
             if (out) return 0.5;
-        }
+        } while (((double)lo < 1e-14 ? v <= lo : v < lo) || v >= 1.0f);
         return (double)v;
     }
 };
@@ -390,7 +436,6 @@ __host__ __device__ inline int choose_molecule_guess(double r, const double *beg
 struct MoveState {
     double fxo, fyo, fzo, fo, cxo, cyo, czo, co, umaxold, vmaxold, cold, qold;
     double vx, vy, vz, deltx, delty, deltz, angle;
-    double fxn, fyn, fzn, fn, cxn, cyn, czn, cn, umaxnew, vmaxnew, cnew, qnew;
     double cphi, sphi, ct, st, ca, sa;  // rotation (TRotation)
 };
 
@@ -403,68 +448,72 @@ __host__ __device__ inline void cross(double x1, double y1, double z1, double x2
 
 // MonteCarloMove_init_old (MonteCarloMove.f90:34-54)
 __host__ __device__ inline void mcm_init_old(MoveState &m, const double f[3], const double t[3]) {
-    m.fxo = f[0]; m.fyo = f[1]; m.fzo = f[2]; m.fo = sqrt(f[0] * f[0] + f[1] * f[1] + f[2] * f[2]);
-    m.cxo = t[0]; m.cyo = t[1]; m.czo = t[2]; m.co = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
+    m.fxo = f[0]; m.fyo = f[1]; m.fzo = f[2]; m.fo = c_sqrt(f[0] * f[0] + f[1] * f[1] + f[2] * f[2]);
+    m.cxo = t[0]; m.cyo = t[1]; m.czo = t[2]; m.co = c_sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
 }
 
-// MonteCarloMove_init_new (MonteCarloMove.f90:56-106)
-__host__ __device__ inline void mcm_init_new(MoveState &m, const double f[3], const double t[3], double xlf, double xlc,
-                                             double dr, double d_angle) {
-    m.fxn = f[0]; m.fyn = f[1]; m.fzn = f[2]; m.fn = sqrt(f[0] * f[0] + f[1] * f[1] + f[2] * f[2]);
-    m.cxn = t[0]; m.cyn = t[1]; m.czn = t[2]; m.cn = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
-    double umax = xlf * m.fn * dr;
+// MonteCarloMove_init_new (MonteCarloMove.f90:56-106): the bias terms of the new positions.  shi(x) is
+// Shi(x) c_exp(-x).
+struct BiasNew { double umax, vmax, c, q; };
+template <class Shi>
+__host__ __device__ inline BiasNew mcm_init_new(const double f[3], const double t[3], double xlf, double xlc,
+                                                double dr, double d_angle, Shi shi) {
+    BiasNew b;
+    const double fn = c_sqrt(f[0] * f[0] + f[1] * f[1] + f[2] * f[2]);
+    const double cn = c_sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
+    double umax = xlf * fn * dr;
     if (umax > 1e-2) {
-        const double e = exp(-2.0 * umax);
+        const double e = c_exp(-2.0 * umax);
         const double t2 = (umax * (1.0 + e) - (1.0 - e)) / 2.0;
-        m.cnew = 3.0 * t2 / (umax * umax * umax);
-    } else { umax = 0.0; m.cnew = 1.0; }
-    m.umaxnew = umax;
-    double vmax = xlc * m.cn * d_angle;
-    if (vmax > 1e-2) m.qnew = d_shi_sans_exp(vmax) / vmax;
-    else { vmax = 0.0; m.qnew = 1.0; }
-    m.vmaxnew = vmax;
+        b.c = c_div(3.0 * t2, umax * umax * umax);
+    } else { umax = 0.0; b.c = 1.0; }
+    b.umax = umax;
+    double vmax = xlc * cn * d_angle;
+    if (vmax > 1e-2) b.q = c_div(shi(vmax), vmax);
+    else { vmax = 0.0; b.q = 1.0; }
+    b.vmax = vmax;
+    return b;
 }
 
 // MonteCarloMove_chooseDisplacement (MonteCarloMove.f90:109-266): a ball of
-// radius dr, or the force-biased distribution exp(lambda F.dr) when biased.
+// radius dr, or the force-biased distribution c_exp(lambda F.dr) when biased.
 __host__ __device__ inline void mcm_choose_displacement(MoveState &m, RngReader &rng, double xlf, double dr) {
     double umax = xlf * m.fo * dr;
     if (umax > 1e-2) {
-        double e = exp(-2.0 * umax);
+        double e = c_exp(-2.0 * umax);
         const double t = (umax * (1.0 + e) - (1.0 - e)) / 2.0;
-        m.cold = 3.0 * t / (umax * umax * umax);
+        m.cold = c_div(3.0 * t, umax * umax * umax);
         double xksi = 0.0;
         while (xksi < 1e-10) { xksi = rng.next(); if (rng.out) return; }
-        const double z = umax + log(xksi * t);
+        const double z = umax + c_log(xksi * t);
         double u;
-        if (z <= log(4.0)) { const double s = exp(z); u = pow(3.0 * s, 1.0 / 3.0) - s / 10.0; }
-        else u = z - log(z / 2.0);
-        // Newton on h(u) = u + ln(u ch u - sh u) = z, 10 iterations, the last one only for e at the
-        // final u.  Once an update leaves u unchanged every later iteration repeats the same
-        // arithmetic on the same u, so the loop stops there with the same u and e bit for bit.
-        for (int k = 1; k <= 10; ++k) {
-            e = exp(-2.0 * u);
+        if (z <= c_log(4.0)) { const double s = c_exp(z); u = cbrt(3.0 * s) - s / 10.0; }
+        else u = z - c_log(z / 2.0);
+        // Newton on h(u) = u + ln(u ch u - sh u) = z, at most 9 updates, then e at the final u.  The
+        // updates square the relative error, so one below 1e-8 leaves u at its last bit and the loop
+        // stops (4 updates where the 9 would only repeat the last bits; an update takes an exp, a log
+        // and two divisions, 0.8 k cycles).
+        for (int k = 1; k <= 9; ++k) {
+            e = c_exp(-2.0 * u);
             const double ch = (1.0 + e) / 2.0;
             double sh = (1.0 - e) / 2.0;
             if (u < 1e-5) sh = u - u * u;
             double g = u * ch - sh;
             if (u < 1e-3) g = u * u * u / 3.0;
-            const double h = u + log(g);
-            const double h1 = u * sh / g;
-            if (k < 10) {
-                const double un = u + (z - h) / h1;
-                if (un == u) break;
-                u = un;
-            }
+            const double h = u + c_log(g);
+            const double d = c_div((z - h) * g, u * sh);
+            u = u + d;
+            if (fabs(d) <= 1e-8 * u) break;
         }
-        const double deltar = u / (xlf * m.fo);
+        e = c_exp(-2.0 * u);
+        const double deltar = c_div(u, xlf * m.fo);
         xksi = 1.0;
         while (xksi > (1.0 - 1e-10) || xksi < 1e-10) { xksi = rng.next(); if (rng.out) return; }
-        double xc = 1.0 + log(xksi + (1.0 - xksi) * e) / u;
+        double xc = 1.0 + c_div(c_log(xksi + (1.0 - xksi) * e), u);
         if (u < 1e-7) xc = 1.0 - 2.0 * (1.0 - xksi);
         if (xc > 1.0 - 1e-14) xc = 1.0 - 1e-14;
         if (xc < -1.0 + 1e-14) xc = -1.0 + 1e-14;
-        const double xs = sqrt(1.0 - xc * xc);
+        const double xs = c_sqrt(1.0 - xc * xc);
         double w = -1.0, wx = 0, wy = 0, wz = 0;
         while (w <= 1e-10) {
             double v2 = 2.0, vx = 0, vy = 0, vz = 0;
@@ -474,11 +523,12 @@ __host__ __device__ inline void mcm_choose_displacement(MoveState &m, RngReader 
                 v2 = vx * vx + vy * vy + vz * vz;
             }
             cross(vx, vy, vz, m.fxo, m.fyo, m.fzo, wx, wy, wz);
-            w = sqrt(wx * wx + wy * wy + wz * wz);
+            w = c_sqrt(wx * wx + wy * wy + wz * wz);
         }
-        m.deltx = deltar * (xc * m.fxo / m.fo + xs * wx / w);
-        m.delty = deltar * (xc * m.fyo / m.fo + xs * wy / w);
-        m.deltz = deltar * (xc * m.fzo / m.fo + xs * wz / w);
+        const double cf = c_div(xc, m.fo), cw = c_div(xs, w);
+        m.deltx = deltar * (cf * m.fxo + cw * wx);
+        m.delty = deltar * (cf * m.fyo + cw * wy);
+        m.deltz = deltar * (cf * m.fzo + cw * wz);
     } else {
         double v2 = 2.0, vx = 0, vy = 0, vz = 0;
         while (v2 > 1.0) {
@@ -490,6 +540,34 @@ __host__ __device__ inline void mcm_choose_displacement(MoveState &m, RngReader 
         umax = 0.0; m.cold = 1.0;
     }
     m.umaxold = umax;
+}
+
+// MonteCarloMove_chooseDisplacement and _chooseRotation of an unbiased move (zero force and torque):
+// the ball and the uniform rotation alone, so the unbiased chain carries none of the biased code
+// (its moves run their control code once per move: what it does not hold it does not fetch)
+__host__ __device__ inline void mcm_uniform_axis(MoveState &m, double vx, double vy, double vz, double v2, double angle) {
+    const double v = c_sqrt(v2);
+    vx = c_div(vx, v); vy = c_div(vy, v); vz = c_div(vz, v);
+    const double2 r = c_sincos(angle);
+    m.sa = r.x; m.ca = r.y;
+    m.ct = vz; m.st = c_sqrt(1.0 - m.ct * m.ct);
+    m.cphi = 0.0; m.sphi = 0.0;
+    if (m.st > 0.0) { m.cphi = c_div(vx, m.st); m.sphi = c_div(vy, m.st); }
+}
+__host__ __device__ inline void mcm_choose_unbiased(MoveState &m, RngReader &rng, double dr, double d_angle) {
+    double v[2][3], v2[2];
+    for (int k = 0; k < 2; ++k) {  // the displacement in the ball, then the axis (not too short)
+        v2[k] = 2.0;
+        while (v2[k] > 1.0 || (k == 1 && v2[k] < 1e-10)) {
+            v[k][0] = 2.0 * rng.next() - 1.0; v[k][1] = 2.0 * rng.next() - 1.0; v[k][2] = 2.0 * rng.next() - 1.0;
+            if (rng.out) return;
+            v2[k] = v[k][0] * v[k][0] + v[k][1] * v[k][1] + v[k][2] * v[k][2];
+        }
+    }
+    const double angle = d_angle * (2.0 * rng.next() - 1.0);
+    if (rng.out) return;
+    m.deltx = dr * v[0][0]; m.delty = dr * v[0][1]; m.deltz = dr * v[0][2];
+    mcm_uniform_axis(m, v[1][0], v[1][1], v[1][2], v2[1], angle);
 }
 
 // The random numbers MonteCarloMove_chooseDisplacement draws, without its arithmetic: its
@@ -513,7 +591,7 @@ __host__ __device__ inline void mcm_skip_displacement(const MoveState &m, RngRea
                 v2 = vx * vx + vy * vy + vz * vz;
             }
             cross(vx, vy, vz, m.fxo, m.fyo, m.fzo, wx, wy, wz);
-            w = sqrt(wx * wx + wy * wy + wz * wz);
+            w = c_sqrt(wx * wx + wy * wy + wz * wz);
         }
     } else {
         v2 = 2.0;
@@ -532,32 +610,76 @@ __host__ __device__ inline void copy_rotation(MoveState &d, const MoveState &s) 
 }
 
 // MonteCarloMove_chooseRotation (MonteCarloMove.f90:269-444)
-__host__ __device__ inline void mcm_choose_rotation(MoveState &m, RngReader &rng, double xlc, double d_angle) {
+// One candidate of the biased rotation's rejection loop from its two random numbers: the value v, e =
+// c_exp(-2 v), and whether it is taken (v below 1e-10 draws its first number again)
+struct BiasedAngle { double v, e; bool again, taken; };
+__host__ __device__ inline BiasedAngle mcm_biased_angle(double x1, double x2, double vmax, double shmax, double emax) {
+    BiasedAngle b;
+    const double xs = x1 * shmax;
+    b.v = vmax + c_log(xs + c_sqrt(xs * xs + emax));
+    if (xs * xs < 1e-14 * emax) b.v = c_div(xs, c_sqrt(emax));
+    b.again = fabs(b.v) < 1e-10;
+    b.e = c_exp(-2.0 * b.v);
+    double proba = c_div(1.0 - b.e, b.v * (1.0 + b.e));
+    if (b.v < 1e-5) proba = c_div(2.0 * b.v - 2.0 * b.v * b.v, b.v * (1.0 + b.e));
+    b.taken = !(x2 >= proba);
+    return b;
+}
+// the loop itself: false when the stream ran out
+struct PickSerial {
+    __host__ __device__ bool operator()(RngReader &rng, double vmax, double shmax, double emax, double &v, double &e) const {
+        for (;;) {
+            const double x1 = rng.next();
+            if (rng.out) return false;
+            if (mcm_biased_angle(x1, 0.0, vmax, shmax, emax).again) continue;
+            const double x2 = rng.next();
+            if (rng.out) return false;
+            const BiasedAngle b = mcm_biased_angle(x1, x2, vmax, shmax, emax);
+            if (b.taken) { v = b.v; e = b.e; return true; }
+        }
+    }
+};
+#ifdef __CUDACC__
+// The same by a whole warp (all lanes on the same reader): a candidate is taken about once in vmax
+// tries, each a log, an exp and two divisions, so the lanes try the next 32 pairs of numbers together
+// and the first that is taken wins.  Where the pairs up to it hold a number that would be drawn again,
+// the serial loop goes on from where the stream stands.
+struct PickWarp {
+    __device__ bool operator()(RngReader &rng, double vmax, double shmax, double emax, double &v, double &e) const {
+        const int lane = threadIdx.x & 31;
+        for (;;) {
+            RngReader mine = rng;
+            mine.k = rng.k + 2 * lane;
+            const float r1 = mine.raw(), r2 = mine.raw();
+            constexpr float lo = 1e-14f;
+            const bool odd = mine.out || !(r1 > lo && r1 < 1.0f && r2 > lo && r2 < 1.0f);
+            const BiasedAngle b = mcm_biased_angle(odd ? 0.5 : (double)r1, odd ? 0.5 : (double)r2, vmax, shmax, emax);
+            const unsigned taken = __ballot_sync(0xffffffffu, !odd && b.taken), stop = __ballot_sync(0xffffffffu, odd || b.again);
+            const int first = taken ? __ffs(taken) - 1 : 32;
+            if (stop & (first < 31 ? (2u << first) - 1u : 0xffffffffu)) return PickSerial()(rng, vmax, shmax, emax, v, e);
+            rng.k += 2 * (first < 32 ? first + 1 : 32);
+            if (first == 32) continue;
+            v = __shfl_sync(0xffffffffu, b.v, first);
+            e = __shfl_sync(0xffffffffu, b.e, first);
+            return true;
+        }
+    }
+};
+#endif
+
+template <class Shi, class Pick>
+__host__ __device__ inline void mcm_choose_rotation(MoveState &m, RngReader &rng, double xlc, double d_angle, Shi shi, Pick pick) {
     double vmax = xlc * m.co * d_angle, vx, vy, vz, angle;
     if (vmax > 1e-2) {
-        const double emax = exp(-2.0 * vmax);
+        const double emax = c_exp(-2.0 * vmax);
         const double shmax = (1.0 - emax) / 2.0;
-        double xksi = 1.0, proba = 0.0, v = 0.0, e = 0.0;
-        while (xksi >= proba) {
-            v = 0.0;
-            while (fabs(v) < 1e-10) {
-                xksi = rng.next();
-                if (rng.out) return;
-                const double xs = xksi * shmax;
-                v = vmax + log(xs + sqrt(xs * xs + emax));
-                if (xs * xs < 1e-14 * emax) v = xs / sqrt(emax);
-            }
-            e = exp(-2.0 * v);
-            proba = (1.0 - e) / v / (1.0 + e);
-            if (v < 1e-5) proba = (2.0 * v - 2.0 * v * v) / v / (1.0 + e);
-            xksi = rng.next();
-            if (rng.out) return;
-        }
-        const double cosx = v / vmax;
-        m.qold = d_shi_sans_exp(vmax) / vmax;
+        double xksi, v = 0.0, e = 0.0;
+        if (!pick(rng, vmax, shmax, emax, v, e)) return;
+        const double cosx = c_div(v, vmax);
+        m.qold = c_div(shi(vmax), vmax);
         xksi = 1.0;
         while (xksi > (1.0 - 1e-10)) { xksi = rng.next(); if (rng.out) return; }
-        angle = d_angle * (1.0 + log(xksi + (1.0 - xksi) * e) / v);
+        angle = d_angle * (1.0 + c_div(c_log(xksi + (1.0 - xksi) * e), v));
         if (v < 1e-7) angle = d_angle * (1.0 - 2.0 * (1.0 - xksi));
         double w = -1.0, wx = 0, wy = 0, wz = 0;
         vx = vy = vz = 0;
@@ -569,12 +691,13 @@ __host__ __device__ inline void mcm_choose_rotation(MoveState &m, RngReader &rng
                 v2 = vx * vx + vy * vy + vz * vz;
             }
             cross(vx, vy, vz, m.cxo, m.cyo, m.czo, wx, wy, wz);
-            w = sqrt(wx * wx + wy * wy + wz * wz);
+            w = c_sqrt(wx * wx + wy * wy + wz * wz);
         }
-        const double sinx = sqrt(1.0 - cosx * cosx);
-        vx = m.cxo / m.co * cosx + wx / w * sinx;
-        vy = m.cyo / m.co * cosx + wy / w * sinx;
-        vz = m.czo / m.co * cosx + wz / w * sinx;
+        const double sinx = c_sqrt(1.0 - cosx * cosx);
+        const double cc = c_div(cosx, m.co), cw = c_div(sinx, w);
+        vx = cc * m.cxo + cw * wx;
+        vy = cc * m.cyo + cw * wy;
+        vz = cc * m.czo + cw * wz;
     } else {
         double v2 = 2.0;
         vx = vy = vz = 0;
@@ -583,27 +706,30 @@ __host__ __device__ inline void mcm_choose_rotation(MoveState &m, RngReader &rng
             if (rng.out) return;
             v2 = vx * vx + vy * vy + vz * vz;
         }
-        const double v = sqrt(v2);
-        vx = vx / v; vy = vy / v; vz = vz / v;
+        const double v = c_sqrt(v2);
+        vx = c_div(vx, v); vy = c_div(vy, v); vz = c_div(vz, v);
         angle = d_angle * (2.0 * rng.next() - 1.0);
         if (rng.out) return;
         vmax = 0.0; m.qold = 1.0;
     }
-    sincos(angle, &m.sa, &m.ca);
-    m.ct = vz; m.st = sqrt(1.0 - m.ct * m.ct);
+    const double2 r = c_sincos(angle);
+    m.sa = r.x; m.ca = r.y;
+    m.ct = vz; m.st = c_sqrt(1.0 - m.ct * m.ct);
     m.cphi = 0.0; m.sphi = 0.0;
-    if (m.st > 0.0) { m.cphi = vx / m.st; m.sphi = vy / m.st; }
+    if (m.st > 0.0) { m.cphi = c_div(vx, m.st); m.sphi = c_div(vy, m.st); }
     m.vx = vx; m.vy = vy; m.vz = vz; m.vmaxold = vmax; m.angle = angle;
 }
 
-// MonteCarloMove_accept_or_decline (MonteCarloMove.f90:447-570); one draw
-__host__ __device__ inline int mcm_accept(const MoveState &m, double dutot, double xlf, double xlc, RngReader &rng) {
+// MonteCarloMove_accept_or_decline (MonteCarloMove.f90:447-570); one draw.  f, t: the molecular force
+// and torque at the new positions, b their bias terms
+__host__ __device__ inline int mcm_accept(const MoveState &m, const double f[3], const double t[3], const BiasNew &b, double dutot,
+                                          double xlf, double xlc, RngReader &rng) {
     const double exposu = -dutot;
-    const double exposf = -xlf * ((m.fxo + m.fxn) * m.deltx + (m.fyo + m.fyn) * m.delty + (m.fzo + m.fzn) * m.deltz);
-    const double exposfcorr = m.umaxold - m.umaxnew;
-    const double exposc = -xlc * m.angle * ((m.cxo + m.cxn) * m.vx + (m.cyo + m.cyn) * m.vy + (m.czo + m.czn) * m.vz);
-    const double exposccorr = m.vmaxold - m.vmaxnew;
-    const double factor = m.cold * m.qold / (m.cnew * m.qnew) * exp(exposu + exposf + exposfcorr + exposc + exposccorr);
+    const double exposf = -xlf * ((m.fxo + f[0]) * m.deltx + (m.fyo + f[1]) * m.delty + (m.fzo + f[2]) * m.deltz);
+    const double exposfcorr = m.umaxold - b.umax;
+    const double exposc = -xlc * m.angle * ((m.cxo + t[0]) * m.vx + (m.cyo + t[1]) * m.vy + (m.czo + t[2]) * m.vz);
+    const double exposccorr = m.vmaxold - b.vmax;
+    const double factor = c_div(m.cold * m.qold, b.c * b.q) * c_exp(exposu + exposf + exposfcorr + exposc + exposccorr);
     const double xksi = rng.next();
     return xksi > factor ? 0 : 1;
 }
@@ -616,10 +742,11 @@ __host__ __device__ inline int mcm_accept(const MoveState &m, double dutot, doub
 template <class Pos, class Put>
 __host__ __device__ inline void place_molecule_f(const MoveState &m, int na, Pos pos, const double *mass, Put put) {
     double sx = 0, sy = 0, sz = 0, tm = 0;
-#pragma unroll
-    for (int i = 0; i < kMaxA; ++i)
-        if (i < na) { sx = sx + mass[i] * pos(i, 0); sy = sy + mass[i] * pos(i, 1); sz = sz + mass[i] * pos(i, 2); tm = tm + mass[i]; }
-    const double xc = sx / tm, yc = sy / tm, zc = sz / tm;
+#pragma unroll 1
+    for (int i = 0; i < na; ++i) {
+        sx = sx + mass[i] * pos(i, 0); sy = sy + mass[i] * pos(i, 1); sz = sz + mass[i] * pos(i, 2); tm = tm + mass[i];
+    }
+    const double xc = c_div(sx, tm), yc = c_div(sy, tm), zc = c_div(sz, tm);
     const double xcn = xc + m.deltx - round(xc + m.deltx);
     const double ycn = yc + m.delty - round(yc + m.delty);
     const double zcn = zc + m.deltz - round(zc + m.deltz);
@@ -634,13 +761,12 @@ __host__ __device__ inline void place_molecule_f(const MoveState &m, int na, Pos
         const double rzx = st * (ct * ca1 * cphi - sa * sphi);
         const double rzy = st * (ct * ca1 * sphi + sa * cphi);
         const double rzz = (st * st * ca + ct * ct);
-#pragma unroll
-        for (int i = 0; i < kMaxA; ++i)
-            if (i < na) {
-                const double xr = pos(i, 0) - xc, yr = pos(i, 1) - yc, zr = pos(i, 2) - zc;
-                put(i, (rxx * xr + rxy * yr + rxz * zr) + xcn, (ryx * xr + ryy * yr + ryz * zr) + ycn,
-                    (rzx * xr + rzy * yr + rzz * zr) + zcn);
-            }
+#pragma unroll 1
+        for (int i = 0; i < na; ++i) {
+            const double xr = pos(i, 0) - xc, yr = pos(i, 1) - yc, zr = pos(i, 2) - zc;
+            put(i, (rxx * xr + rxy * yr + rxz * zr) + xcn, (ryx * xr + ryy * yr + ryz * zr) + ycn,
+                (rzx * xr + rzy * yr + rzz * zr) + zcn);
+        }
     } else {
         put(0, xcn, ycn, zcn);
     }
@@ -657,21 +783,22 @@ __host__ __device__ inline void place_molecule(const MoveState &m, int na, const
 template <class Pos, class Frc>
 __host__ __device__ inline void mol_force_torque_f(int na, Pos pos, const double *mass, Frc frc, double F[3], double T[3]) {
     double sx = 0, sy = 0, sz = 0, tm = 0;
-#pragma unroll
-    for (int i = 0; i < kMaxA; ++i)
-        if (i < na) { sx = sx + mass[i] * pos(i, 0); sy = sy + mass[i] * pos(i, 1); sz = sz + mass[i] * pos(i, 2); tm = tm + mass[i]; }
-    const double xc = sx / tm, yc = sy / tm, zc = sz / tm;
-    F[0] = F[1] = F[2] = 0; T[0] = T[1] = T[2] = 0;
-#pragma unroll
-    for (int i = 0; i < kMaxA; ++i)
-        if (i < na) { F[0] = F[0] + frc(i, 0); F[1] = F[1] + frc(i, 1); F[2] = F[2] + frc(i, 2); }
-#pragma unroll
-    for (int i = 0; i < kMaxA; ++i)
-        if (i < na) {
-            double tx, ty, tz;
-            cross(pos(i, 0) - xc, pos(i, 1) - yc, pos(i, 2) - zc, frc(i, 0), frc(i, 1), frc(i, 2), tx, ty, tz);
-            T[0] = T[0] + tx; T[1] = T[1] + ty; T[2] = T[2] + tz;
-        }
+#pragma unroll 1
+    for (int i = 0; i < na; ++i) {
+        sx = sx + mass[i] * pos(i, 0); sy = sy + mass[i] * pos(i, 1); sz = sz + mass[i] * pos(i, 2); tm = tm + mass[i];
+    }
+    const double xc = c_div(sx, tm), yc = c_div(sy, tm), zc = c_div(sz, tm);
+    double fx = 0, fy = 0, fz = 0, tx = 0, ty = 0, tz = 0;
+#pragma unroll 1
+    for (int i = 0; i < na; ++i) {
+        const double gx = frc(i, 0), gy = frc(i, 1), gz = frc(i, 2);
+        fx = fx + gx; fy = fy + gy; fz = fz + gz;
+        double ax, ay, az;
+        cross(pos(i, 0) - xc, pos(i, 1) - yc, pos(i, 2) - zc, gx, gy, gz, ax, ay, az);
+        tx = tx + ax; ty = ty + ay; tz = tz + az;
+    }
+    F[0] = fx; F[1] = fy; F[2] = fz;
+    T[0] = tx; T[1] = ty; T[2] = tz;
 }
 __host__ __device__ inline void mol_force_torque(int na, const double *x, const double *y, const double *z,
                                                  const double *mass, const double *fx, const double *fy,

@@ -540,18 +540,16 @@ int upload(T *d, const T *h, size_t n, cudaStream_t s) {
     return YAMC_OK;
 }
 
-size_t chain_smem_bytes(int G, int B, int kmax, int nt, int nown_max, int qcap) {
+size_t chain_smem_bytes(int G, int B, int kmax, int nt, int nown_max) {
     const int KM = kmax + 1;
     const size_t nblk_max = (size_t)(nown_max + kBlk - 1) / kBlk;
     size_t b = sizeof(double2) * kTabRow * 3 * KM;
     b += sizeof(float4) * 2 * nblk_max;
     b += (sizeof(double4) + sizeof(int2)) * (size_t)nown_max;
-    b += sizeof(int) * (size_t)((qcap + 1) & ~1);
-    b += sizeof(int) * (size_t)B * kCPT;
+    b += sizeof(int) * (size_t)wbuf_ints(B, kmax);
     b += sizeof(double) * (size_t)(B / 32) * kNV;
     b += sizeof(double) * (size_t)2 * G * kNV;
     b += sizeof(double) * ((size_t)2 * nt * nt + nt + 1);
-    b += sizeof(int) * (nblk_max + 32);
     return b;
 }
 
@@ -691,10 +689,9 @@ int pick_launch_for(const std::vector<const HostSystem *> &hosts, int device, in
             }
             if (EPT > 2) continue;
             const int nown_max = (Nmax + G - 1) / G;
-            const int qcap = std::min(kQueueMax, std::min(nown_max, nwork * kCPT) * 2 * kMaxA);  // pair-queue chunk
-            const size_t sm = chain_smem_bytes(G, B, kmax, nt, nown_max, qcap);
-            if (sm > smem_max) continue;
-            out->G = G; out->B = B; out->EPT = EPT; out->nown_max = nown_max; out->qcap = qcap; out->smem = sm;
+            const size_t sm = chain_smem_bytes(G, B, kmax, nt, nown_max);
+            if (sm > smem_max || nown_max > kMaxOwn) continue;
+            out->G = G; out->B = B; out->EPT = EPT; out->nown_max = nown_max; out->smem = sm;
             return YAMC_OK;
         }
     }
@@ -1108,7 +1105,7 @@ void fill_dhs_types(const HostSystem &H, DevSys &D) {
 ChainArgs base_args(yamc_ctx *c) {
     ChainArgs a{};
     a.sys = c->d_sys; a.run = c->d_run; a.G = c->cfg.G;
-    a.nown_max = c->cfg.nown_max; a.qcap = c->cfg.qcap;
+    a.nown_max = c->cfg.nown_max;
     a.scratch = c->scratch;
     a.prof = c->prof_on ? c->d_prof : nullptr;
     return a;
@@ -1193,7 +1190,7 @@ int batch_build_graph(yamc_batch *b) {
         if (cudaStreamWaitEvent(g.stream, b->fork, 0) != cudaSuccess) { r = YAMC_ECUDA; break; }
         ChainArgs a{};
         a.sys = g.d_sys; a.run = g.d_run; a.G = g.cfg.G;
-        a.nown_max = g.cfg.nown_max; a.qcap = g.cfg.qcap;
+        a.nown_max = g.cfg.nown_max;
         if ((r = launch_chain_cfg(g.cfg, g.nt, g.split, g.mx, g.stream, (int)g.idx.size(), a))) break;
         if (cudaEventRecord(g.done, g.stream) != cudaSuccess || cudaStreamWaitEvent(b->stream, g.done, 0) != cudaSuccess)
             r = YAMC_ECUDA;
