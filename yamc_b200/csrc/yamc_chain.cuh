@@ -61,6 +61,8 @@ struct RunSlot {
     double *rows;           // optional energy rows (9 doubles)
     int max_rows, n_rows;
     int status, accepted;
+    double sc[SC_COUNT];    // out: the engine scalars and counters, so the host has them with the slot
+    long long cnt[CN_COUNT];
 };
 
 struct ChainArgs {
@@ -1893,11 +1895,12 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
                 for (int t = 0; t <= NT; ++t) D.rho[(size_t)t * S + R.e[k]] = R.rho[k][t];
             }
         if (tid == 0 && rank == 0) {
-            for (int c = 0; c < SC_COUNT; ++c) D.scal[c] = sh.sc[c];
-            D.cnt[CN_ICYCLE] = sh.icycle;
-            D.cnt[CN_ACC_SINCE_REFRESH] = acc_since;
-            D.cnt[CN_REFRESHES] += refreshes;
-            D.cnt[CN_MOVE_IN_CYCLE] = sh.mic;
+            for (int c = 0; c < SC_COUNT; ++c) D.scal[c] = run->sc[c] = sh.sc[c];
+            run->cnt[CN_ICYCLE] = sh.icycle;
+            run->cnt[CN_ACC_SINCE_REFRESH] = acc_since;
+            run->cnt[CN_REFRESHES] = D.cnt[CN_REFRESHES] + refreshes;
+            run->cnt[CN_MOVE_IN_CYCLE] = sh.mic;
+            for (int c = 0; c < CN_COUNT; ++c) D.cnt[c] = run->cnt[c];
             run->cursor = sh.cursor;
             run->moves_done = moves_done;
             run->n_rows = rows;

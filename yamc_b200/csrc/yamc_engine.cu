@@ -316,6 +316,22 @@ __global__ void __launch_bounds__(256) k_rdf_count(const double *cx, const doubl
         if (hs[k]) atomicAdd(&hist[k], (unsigned long long)hs[k]);
 }
 
+// the coordinates of the atoms, axis by axis
+__global__ void k_split_positions(const double4 *atom, int N, double *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    const double4 p = atom[i];
+    out[i] = p.x; out[(size_t)N + i] = p.y; out[2 * (size_t)N + i] = p.z;
+}
+
+// the other way: x, y, z of every atom (their charges stay)
+__global__ void k_join_positions(const double *in, int N, double4 *atom) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    double *a = reinterpret_cast<double *>(atom + i);
+    a[0] = in[i]; a[1] = in[(size_t)N + i]; a[2] = in[2 * (size_t)N + i];
+}
+
 // the exchange step's commit: rho += delta (MC.f90:1245 for the two molecules)
 __global__ void k_commit_rho(double2 *rho, const double2 *delta, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -602,6 +618,7 @@ struct yamc_ctx {
     // mapped pinned host memory the kernel writes directly (h_out on the host, d_hout on the device):
     // kNV pass values, SC_COUNT scalars, CN_COUNT counters, then the per-move passes' completion word
     double *h_out = nullptr, *d_hout = nullptr;
+    double *h_pos = nullptr, *d_hpos = nullptr;  // the same memory further on: x, y, z of every atom (sync_positions)
     long long move_seq = 0;  // sequence number of the last per-move pass
     // the per-move pass (k_move_pass): block partials and the finished-block counter
     double *d_mpart = nullptr;
@@ -617,6 +634,7 @@ struct yamc_ctx {
     double sc[SC_COUNT] = {};
     long long cnt_h[CN_COUNT] = {};
     bool pos_valid = true;  // H.x/y/z mirror the device positions
+    bool sc_valid = true;   // sc and cnt_h mirror the device scalars and counters (every run brings them back)
     LaunchCfg cfg;
     int force_G = 0, force_B = 0, force_layout = YAMC_KSPACE_AUTO;
     // per-move API state
@@ -627,8 +645,7 @@ struct yamc_ctx {
     double api_dmu[3] = {};
     long long *d_prof = nullptr;
     bool prof_on = false;
-    double *d_f = nullptr;                                      // adjoint forces [3][N]
-    double *d_gf = nullptr, *d_kf = nullptr;                    // their real-space parts; k-space forces by list position
+    double *d_gf = nullptr, *d_kf = nullptr;                    // adjoint forces: real-space parts, k-space by list position
     double4 *d_field = nullptr;                                 // the k-space fields they sum
     // NPT volume move: rho(k) as it was before the step, accepted volume steps
     double2 *rho_save = nullptr;
@@ -971,21 +988,38 @@ int launch_kspace_energy(yamc_ctx *c, int nb) {
     return YAMC_OK;
 }
 
+// x, y, z of every atom from the device into H: a kernel writes them to mapped pinned memory (a copy of
+// 12,440 atoms to pageable memory took 0.15 ms, this takes 0.03)
 int sync_positions(yamc_ctx *c) {
     if (c->pos_valid) return YAMC_OK;
-    std::vector<double4> a(c->H.N);
-    CUDA_TRY(cudaMemcpyAsync(a.data(), c->atom, sizeof(double4) * c->H.N, cudaMemcpyDeviceToHost, c->stream));
+    HostSystem &H = c->H;
+    const int N = H.N;
+    k_split_positions<<<(N + 255) / 256, 256, 0, c->stream>>>(c->atom, N, c->d_hpos);
+    CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(c->stream));
-    for (int i = 0; i < c->H.N; ++i) { c->H.x[i] = a[i].x; c->H.y[i] = a[i].y; c->H.z[i] = a[i].z; }
+    std::copy(c->h_pos, c->h_pos + N, H.x.begin());
+    std::copy(c->h_pos + N, c->h_pos + 2 * (size_t)N, H.y.begin());
+    std::copy(c->h_pos + 2 * (size_t)N, c->h_pos + 3 * (size_t)N, H.z.begin());
     c->pos_valid = true;
     return YAMC_OK;
 }
 
+// the engine scalars and counters into c->sc and c->cnt_h (there already unless a run failed)
 int pull_state(yamc_ctx *c) {
+    if (c->sc_valid) return YAMC_OK;
     CUDA_TRY(cudaMemcpyAsync(c->sc, c->scal, sizeof(double) * SC_COUNT, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(cudaMemcpyAsync(c->cnt_h, c->cnt, sizeof(long long) * CN_COUNT, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
+    c->sc_valid = true;
     return YAMC_OK;
+}
+
+// what a chain's run slot brings back
+void take_state(yamc_ctx *c, const RunSlot &rs) {
+    std::copy(rs.sc, rs.sc + SC_COUNT, c->sc);
+    std::copy(rs.cnt, rs.cnt + CN_COUNT, c->cnt_h);
+    c->sc_valid = true;
+    c->pos_valid = false;
 }
 
 int push_state(yamc_ctx *c) {
@@ -1058,7 +1092,7 @@ int ensure_cfg(yamc_ctx *c) {
     return pick_launch(c, &c->cfg);
 }
 
-// the adjoint's device forces, real space and k space, into c->d_f
+// the adjoint's forces, real space and k space, into the mapped pinned memory
 template <int NT>
 int launch_forces(yamc_ctx *c) {
     const HostSystem &H = c->H;
@@ -1067,8 +1101,8 @@ int launch_forces(yamc_ctx *c) {
     // the row pairs split over blockIdx.y until the blocks fill the GPU about four times
     const int nsplit = std::max(1, std::min((4 * c->nsm + nblk - 1) / nblk, (c->k_nfrow + kForceRowWarps - 1) / kForceRowWarps));
     int r;
-    if (!c->d_f && ((r = dalloc(&c->d_gf, (size_t)3 * shares * H.N)) || (r = dalloc(&c->d_kf, (size_t)3 * nsplit * c->k_npos)) ||
-                    (r = dalloc(&c->d_field, (size_t)2 * (1 + NT) * c->k_nf)) || (r = dalloc(&c->d_f, (size_t)3 * H.N))))
+    if (!c->d_field && ((r = dalloc(&c->d_gf, (size_t)3 * shares * H.N)) || (r = dalloc(&c->d_kf, (size_t)3 * nsplit * c->k_npos)) ||
+                        (r = dalloc(&c->d_field, (size_t)2 * (1 + NT) * c->k_nf))))
         return r;
     CUDA_TRY(cudaFuncSetAttribute(k_real_forces, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smr));
     k_real_forces<<<dim3(c->tiles.ntile, shares), 32 * kRealWarps, smr, c->stream>>>(
@@ -1081,7 +1115,7 @@ int launch_forces(yamc_ctx *c) {
                                                                               c->d_field, c->k_nf, c->k_npos, c->d_kf);
     CUDA_TRY(cudaGetLastError());
     k_forces_add<<<(H.N + 255) / 256, 256, 0, c->stream>>>(c->hsys, c->k_place, c->d_gf, shares, c->d_kf, c->k_npos, nsplit,
-                                                           c->d_f);
+                                                           c->d_hpos);
     CUDA_TRY(cudaGetLastError());
     return YAMC_OK;
 }
@@ -1254,6 +1288,7 @@ int batch_step(yamc_batch *b, const float *const *rng, const int64_t *rng_off, c
             rs.log = d_log ? d_log + (size_t)i * n_moves : nullptr;
         }
     }
+    for (yamc_ctx *c : b->reps) c->sc_valid = c->pos_valid = false;
     CUDA_TRY(cudaEventRecord(b->ev0, b->stream));
     CUDA_TRY(cudaGraphLaunch(b->graph, b->stream));
     CUDA_TRY(cudaEventRecord(b->ev1, b->stream));
@@ -1268,7 +1303,7 @@ int batch_step(yamc_batch *b, const float *const *rng, const int64_t *rng_off, c
             cursors[i] = rs.cursor;
             if (moves_done) moves_done[i] = rs.moves_done;
             if (status) status[i] = rs.status;
-            b->reps[i]->pos_valid = false;
+            take_state(b->reps[i], rs);
             if (rs.status != YAMC_OK && (worst == YAMC_OK || worst == YAMC_ERNG_EXHAUSTED)) worst = rs.status;
         }
     for (yamc_ctx *c : b->reps) {
@@ -1316,6 +1351,7 @@ int batch_copy_state(yamc_batch *b, BatchBackup &k, bool save) {
         }
     }
     CUDA_TRY(cudaStreamSynchronize(b->stream));
+    if (!save) for (yamc_ctx *c : b->reps) c->sc_valid = c->pos_valid = false;
     return YAMC_OK;
 }
 
@@ -1382,10 +1418,12 @@ static int create_impl(yamc_ctx *c, const yamc_system *sys, const yamc_params *p
         arena.add(&c->sums, std::max(kFullParts + 2, kXParts));
         if ((r = arena.commit(&c->arena))) return r;
     }
-    CUDA_TRY(cudaHostAlloc(&c->h_out, sizeof(double) * (kNV + SC_COUNT) + sizeof(long long) * (CN_COUNT + 1),
-                           cudaHostAllocMapped));
+    const size_t out_words = ((size_t)kNV + SC_COUNT + CN_COUNT + 1 + 31) / 32 * 32;
+    CUDA_TRY(cudaHostAlloc(&c->h_out, sizeof(double) * (out_words + 3 * (size_t)N), cudaHostAllocMapped));
     move_pass_done(c) = 0;
     CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&c->d_hout), c->h_out, 0));
+    c->h_pos = c->h_out + out_words;
+    c->d_hpos = c->d_hout + out_words;
     if ((r = spatial_reset(c->tiles, c->stream)) || (r = upload_rows(c, rows))) return r;
     std::vector<double4> a(N);
     std::vector<int2> m(N);
@@ -1451,7 +1489,7 @@ int yamc_destroy(yamc_ctx *c) {
     if (!c) return YAMC_OK;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    void *ptrs[] = {c->arena, c->d_rng, c->d_log, c->d_rows, c->d_prof, c->d_f, c->d_gf, c->d_kf, c->d_field, c->rho_save,
+    void *ptrs[] = {c->arena, c->d_rng, c->d_log, c->d_rows, c->d_prof, c->d_gf, c->d_kf, c->d_field, c->rho_save,
                     c->d_mpart, c->d_mcount};
     for (void *p : ptrs) if (p) cudaFree(p);
     if (c->h_out) cudaFreeHost(c->h_out);
@@ -1552,6 +1590,7 @@ static int run_chain_impl(yamc_ctx *c, const float *d_rng, long long rng_off, lo
     rs.log = d_log; rs.rows = d_rows; rs.max_rows = max_rows;
     if ((r = upload(c->d_run, &rs, 1, c->stream))) return r;
     ChainArgs a = base_args(c);
+    c->sc_valid = c->pos_valid = false;
     CUDA_TRY(cudaEventRecord(c->ev0, c->stream));
     if ((r = launch_chain(c, a))) return r;
     CUDA_TRY(cudaEventRecord(c->ev1, c->stream));
@@ -1559,7 +1598,7 @@ static int run_chain_impl(yamc_ctx *c, const float *d_rng, long long rng_off, lo
     CUDA_TRY(cudaMemcpyAsync(&back, c->d_run, sizeof(RunSlot), cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1);
-    c->pos_valid = false;
+    take_state(c, back);
     *cursor = back.cursor;
     if (moves_done) *moves_done = back.moves_done;
     if (n_rows) *n_rows = back.n_rows;
@@ -2893,10 +2932,8 @@ int yamc_forces(yamc_ctx *c, double *fx, double *fy, double *fz, double *mol_f, 
         default: r = launch_forces<4>(c); break;
     }
     if (r) return r;
-    std::vector<double> g((size_t)3 * N);
-    CUDA_TRY(cudaMemcpyAsync(g.data(), c->d_f, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
-    double *gx = g.data(), *gy = gx + N, *gz = gy + N;
+    double *gx = c->h_pos, *gy = gx + N, *gz = gy + N;  // (k_forces_add writes to the mapped pinned memory)
     // external term: F = -2 kext q mu (EwaldSumExternal.f90:84-102)
     const double mx = c->sc[SC_MU_X], my = c->sc[SC_MU_Y], mz = c->sc[SC_MU_Z], m2k = H.p.minus_two_kext;
     bool finite = true;
@@ -3071,14 +3108,16 @@ int yamc_set_positions(yamc_ctx *c, const double *x, const double *y, const doub
             set_error("non-finite coordinate of atom " + std::to_string(i + 1) + " (the configuration is unchanged)");
             return YAMC_ENAN;
         }
-    std::vector<double4> a(H.N);
-    for (int i = 0; i < H.N; ++i) {
-        H.x[i] = x[i]; H.y[i] = y[i]; H.z[i] = z[i];
-        a[i] = make_double4(x[i], y[i], z[i], H.q[i]);
-    }
-    int r = upload(c->atom, a.data(), H.N, c->stream);
-    if (r) return r;
+    // to the device through the mapped pinned memory (the stream is idle between calls, so nothing still
+    // reads it; the full sums below wait for the kernel)
+    const size_t N = H.N;
+    CUDA_TRY(cudaStreamSynchronize(c->stream));
+    std::copy(x, x + N, H.x.begin()); std::copy(y, y + N, H.y.begin()); std::copy(z, z + N, H.z.begin());
+    std::copy(x, x + N, c->h_pos); std::copy(y, y + N, c->h_pos + N); std::copy(z, z + N, c->h_pos + 2 * N);
+    k_join_positions<<<(int)((N + 255) / 256), 256, 0, c->stream>>>(c->d_hpos, H.N, c->atom);
+    CUDA_TRY(cudaGetLastError());
     c->pos_valid = true;
+    int r;
     if ((r = pull_state(c)) || (r = full_sums(c))) return r;
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     if (e) energies_from(c->sc, H.p.kext, e);

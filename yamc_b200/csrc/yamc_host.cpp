@@ -440,15 +440,25 @@ int prepare_host_system(const yamc_system *sys, const yamc_params *pin, HostSyst
     H.beta.resize(H.nk); H.beta6.resize(H.nk); H.beta12.resize(H.nk);
     const double alpha = p.alpha;
     const double poa = kPi / alpha, poa2 = poa * poa;
+    // (the tables depend on k^2 alone, an integer up to kmax^2: each value is computed once -- the
+    // quadrature of B6 and B12 is most of the set-up's time -- and taken by every k of that length)
+    struct Row { double e, B6, B12; };
+    std::vector<Row> rows((size_t)p.kmax * p.kmax + 1);
+    std::vector<char> have(rows.size(), 0);
     for (int k = 0; k < H.nk; ++k) {
-        const double xk2 = (double)(H.kx[k] * H.kx[k]) + (double)(H.ky[k] * H.ky[k]) + (double)(H.kz[k] * H.kz[k]);
-        const double b2 = poa2 * xk2;
-        const double e = std::exp(-b2);
-        H.beta[k] = p.xclb * e / xk2 / kTwoPi;
-        double erfcb, B6, B12;
-        erfc_luc_bet6_bet12(poa * std::sqrt(xk2), b2, e, &erfcb, &B6, &B12);
-        H.beta6[k] = powi(alpha, 3) * B6;
-        H.beta12[k] = powi(alpha, 9) * B12;
+        const int ik2 = H.kx[k] * H.kx[k] + H.ky[k] * H.ky[k] + H.kz[k] * H.kz[k];
+        const double xk2 = (double)ik2;
+        Row &row = rows[ik2];
+        if (!have[ik2]) {
+            const double b2 = poa2 * xk2;
+            row.e = std::exp(-b2);
+            double erfcb;
+            erfc_luc_bet6_bet12(poa * std::sqrt(xk2), b2, row.e, &erfcb, &row.B6, &row.B12);
+            have[ik2] = 1;
+        }
+        H.beta[k] = p.xclb * row.e / xk2 / kTwoPi;
+        H.beta6[k] = powi(alpha, 3) * row.B6;
+        H.beta12[k] = powi(alpha, 9) * row.B12;
         if (H.kx[k] > 0) { H.beta[k] *= 2.0; H.beta6[k] *= 2.0; H.beta12[k] *= 2.0; }
     }
     // signed list: (+,+,+) always, (+,-,+) if ky>0, (+,+,-) if kz>0, (+,-,-) if both
