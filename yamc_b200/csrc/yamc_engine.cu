@@ -358,9 +358,12 @@ constexpr int kMoveThreads = 256;
 // pass's arithmetic: the old phase sums to scratch buffer 0 (OLD), or the deltas against them to
 // buffer 1, dU_k and the k-space forces (EVAL)) and one slice of the atoms (the molecule's pairs
 // inside the cutoff with their forces; EVAL: the hard-core overlap test).  Block sums in a fixed
-// tree; the last block to finish adds the blocks in block order and writes the reduction vector
-// (RV_* layout; OLD: the old energies and forces with the external field -2 kext q mu added, as
-// the chain's old pass hands them on).  Deterministic run to run.
+// tree; the last block to finish adds the blocks, its eight warps every eighth block each and their
+// sums in order, and writes the reduction vector (RV_* layout; OLD: the old energies and forces with
+// the external field -2 kext q mu added, as the chain's old pass hands them on).  Deterministic run
+// to run.  Latency bound: what it waits for are round trips to L2, so the atoms' data come by one
+// thread each and the blocks' partials in independent loads (one thread per value reading block after
+// block took 25 round trips of nacl1m's 25 blocks).
 template <int NT, bool MX, bool EVAL>
 __global__ void __launch_bounds__(kMoveThreads) k_move_pass(DevSys D, MoveIn in, double *part, unsigned *counter,
                                                             double *out) {
@@ -369,27 +372,24 @@ __global__ void __launch_bounds__(kMoveThreads) k_move_pass(DevSys D, MoveIn in,
     constexpr int KIND = EVAL ? PASS_NEW : PASS_OLD;
     extern __shared__ __align__(16) unsigned char move_smem[];
     __shared__ Slot sl[2 * kMaxA];
-    __shared__ double red[(kMoveThreads / 32 + 1) * kNV];
-    __shared__ int na_s, last;
+    __shared__ double red[kMoveThreads / 32][kNV];
+    __shared__ int last;
     const int tid = threadIdx.x;
     const int KM = D.kmax + 1, S = D.S, nt = D.nt;
     const int imol0 = in.imol - 1;
-    if (tid == 0) {
-        const int2 mr = D.mol[imol0];
-        na_s = mr.y;
-        for (int a = 0; a < mr.y; ++a) {
-            const int j = mr.x + a;
-            const double4 p = D.atom[j];
-            Slot o;
-            o.x = p.x; o.y = p.y; o.z = p.z; o.q = p.w; o.iq = p.w != 0.0 ? 1.0 / p.w : 0.0;
-            o.dhs = D.dhs[j]; o.type = D.meta[j].y; o.pad = 0;
-            sl[mr.y + a] = o;
-            if (EVAL) { o.x = in.x[a]; o.y = in.y[a]; o.z = in.z[a]; }
-            sl[a] = o;
-        }
+    const int2 mr = D.mol[imol0];
+    const int na = mr.y;
+    if (tid < na) {
+        const int j = mr.x + tid;
+        const double4 p = D.atom[j];
+        Slot o;
+        o.x = p.x; o.y = p.y; o.z = p.z; o.q = p.w; o.iq = p.w != 0.0 ? 1.0 / p.w : 0.0;
+        o.dhs = D.dhs[j]; o.type = D.meta[j].y; o.pad = 0;
+        sl[na + tid] = o;
+        if (EVAL) { o.x = in.x[tid]; o.y = in.y[tid]; o.z = in.z[tid]; }
+        sl[tid] = o;
     }
     __syncthreads();
-    const int na = na_s;
     const int s_lo = EVAL ? 0 : na, s_hi = EVAL ? na : 2 * na;
     R2 *tab = reinterpret_cast<R2 *>(move_smem);
     build_tables<MX>(tab, sl, s_lo, s_hi, KM, tid, kMoveThreads);
@@ -455,20 +455,46 @@ __global__ void __launch_bounds__(kMoveThreads) k_move_pass(DevSys D, MoveIn in,
             acc.add(RV_F + 3 * a, dx * t.FR); acc.add(RV_F + 3 * a + 1, dy * t.FR); acc.add(RV_F + 3 * a + 2, dz * t.FR);
         }
     }
-    double v[kNV];
+    {
+        const int lane = tid & 31, warp = tid >> 5;
+        double v[16];  // the values but the overlap flag and the last force component
 #pragma unroll
-    for (int i = 0; i < kNV; ++i) v[i] = acc.get(i);
-    block_sum<kMoveThreads>(v, kNV, red);  // (the overlap flags add up: a positive total is an overlap)
-    if (tid < kNV) part[(size_t)blockIdx.x * kNV + tid] = v[tid];
+        for (int i = 0; i < 16; ++i) v[i] = acc.get(i < RV_OVL ? i : i + 1);
+        const double x = warp_sums(v);
+        const int i = lane >> 1;
+        if (!(lane & 1)) red[warp][i < RV_OVL ? i : i + 1] = x;
+        double y = acc.get(kNV - 1);
+        if (na == kMaxA)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+        const bool ovl = __any_sync(0xffffffffu, acc.get(RV_OVL) > 0.0);
+        if (lane == 0) { red[warp][kNV - 1] = y; red[warp][RV_OVL] = ovl ? 1.0 : 0.0; }
+    }
+    __syncthreads();
+    if (tid < kNV) {
+        double x = 0.0;
+#pragma unroll
+        for (int w = 0; w < kMoveThreads / 32; ++w) x += red[w][tid];
+        part[(size_t)blockIdx.x * kNV + tid] = x;
+    }
     __threadfence();
     __syncthreads();
     if (tid == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
-    if (tid < kNV) {
-        const volatile double *pv = part;
+    {
+        const int lane = tid & 31, warp = tid >> 5;
         double x = 0.0;
-        for (int b = 0; b < (int)gridDim.x; ++b) x += pv[(size_t)b * kNV + tid];
+        if (lane < kNV)
+#pragma unroll 8
+            for (int b = warp; b < (int)gridDim.x; b += kMoveThreads / 32) x += __ldcg(part + (size_t)b * kNV + lane);
+        if (lane < kNV) red[warp][lane] = x;
+    }
+    __syncthreads();
+    if (tid < kNV) {
+        double x = 0.0;
+#pragma unroll
+        for (int w = 0; w < kMoveThreads / 32; ++w) x += red[w][tid];
         if (tid == RV_OVL) x = x > 0.0 ? 1.0 : 0.0;
         if (!EVAL && tid >= RV_F && tid < RV_F + 3 * na) {  // the external field at the old dipole (MC.f90:988-997)
             const int a = (tid - RV_F) / 3, c = (tid - RV_F) % 3;
