@@ -1101,57 +1101,41 @@ __device__ __forceinline__ void worker_pass(const DevSys &D, ChainShared &sh, Re
 
 // Control warp, after the workers' per-warp partials: trees over the worker warps, then over the
 // cluster's CTAs in a fixed order, so every CTA holds bit-identical totals in sh.tot.  Called by
-// all threads (the cluster barrier needs everyone).  Lane l of the control warp owns values l and
-// l + 32 (nv <= 64).
+// all threads (the cluster barrier needs everyone).  Lane v of the control warp owns value v (a lane
+// writes its value to every CTA's exchange row, so there is no index arithmetic per value and CTA).
+static_assert(kNV <= 32, "a lane per value");
 __device__ __forceinline__ void reduce_pass(ChainShared &sh, const double *red, double *xch, int nv, int G, int rank,
                                             int xpar, cg::cluster_group &cluster) {
     // the worker warps' partials in warp order, then (cluster) every CTA's sum in rank order --
     // the same order in every CTA
-    const int lane = threadIdx.x & 31;
+    const int v = threadIdx.x;
     const int nww = (blockDim.x - kCtl) >> 5;
-    if (threadIdx.x < kCtl) {
-        double x[2] = {0.0, 0.0};
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int v = lane + 32 * h;
-            if (v < nv)
-                for (int w = 0; w < nww; ++w) {
-                    const double y = red[w * kNV + v];
-                    x[h] = (v == RV_OVL) ? fmax(x[h], y) : x[h] + y;
-                }
+    const bool own = v < nv, flag = v == RV_OVL;
+    if (own) {
+        double x = 0.0;
+#pragma unroll 4
+        for (int w = 0; w < nww; ++w) {
+            const double y = red[w * kNV + v];
+            x = flag ? fmax(x, y) : x + y;
         }
         if (G > 1) {
-            // value v of this CTA to every rank's exchange row; lanes cover (v, r) pairs
-            for (int idx = 0; idx < nv * G; idx += 32) {
-                const int my = idx + lane;
-                const int v = my % nv, r = my / nv;
-                const double x0 = __shfl_sync(0xffffffffu, x[0], v & 31);
-                const double x1 = __shfl_sync(0xffffffffu, x[1], v & 31);
-                if (my < nv * G) {
-                    double *dst = cluster.map_shared_rank(xch, r);
-                    dst[(xpar * G + rank) * kNV + v] = v < 32 ? x0 : x1;
-                }
-            }
+            const int at = (xpar * G + rank) * kNV + v;
+#pragma unroll 4
+            for (int r = 0; r < G; ++r) cluster.map_shared_rank(xch, r)[at] = x;
         } else {
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                if (lane + 32 * h < nv) sh.tot[lane + 32 * h] = x[h];
+            sh.tot[v] = x;
         }
     }
     if (G > 1) {
         cluster.sync();
-        if (threadIdx.x < kCtl) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int v = lane + 32 * h;
-                if (v >= nv) continue;
-                double x = 0.0;
-                for (int r = 0; r < G; ++r) {
-                    const double y = xch[(xpar * G + r) * kNV + v];
-                    x = (v == RV_OVL) ? fmax(x, y) : x + y;
-                }
-                sh.tot[v] = x;
+        if (own) {
+            double x = 0.0;
+#pragma unroll 4
+            for (int r = 0; r < G; ++r) {
+                const double y = xch[(xpar * G + r) * kNV + v];
+                x = flag ? fmax(x, y) : x + y;
             }
+            sh.tot[v] = x;
         }
     }
 }
