@@ -77,8 +77,9 @@ def test_real_space_tiles_with_molecules_outside_the_box(tmp_path, n_water, n_io
     assert np.abs(eng.forces()[0] - f0).max() <= 1e-12 * np.abs(f0).max()
 
 
-@pytest.mark.parametrize("m", [1023, 1024, 1057, 2001])
-def test_rdf_tiles_count_as_all_pairs(m):
+@pytest.mark.parametrize("box", [31.0, 40.0])  # rmax above and below a third of the box
+@pytest.mark.parametrize("m", [1023, 1024, 1057, 2001, 2399, 2400, 2433, 3599, 3600, 4001])
+def test_rdf_tiles_count_as_all_pairs(m, box):
     r = np.random.default_rng(m)
     x, y, z = r.uniform(-0.5, 0.5, (3, m))
     x[::7] += 1.0   # outside the unit box: counted by the single conditional wrap
@@ -86,9 +87,9 @@ def test_rdf_tiles_count_as_all_pairs(m):
     mol_type = np.where(np.arange(m) % 5 == 0, 2, 1).astype(np.int32)
     counts = np.array([(mol_type == 1).sum(), (mol_type == 2).sum()], dtype=np.int32)
     o = pyoracle.RDF(mol_type, counts, dr=0.1, rmax=12.0)
-    o.add_frame(x, y, z, 31.0)
+    o.add_frame(x, y, z, box)
     g = api.RDF(mol_type, counts, dr=0.1, rmax=12.0)
-    g.add_frame(x, y, z, 31.0)
+    g.add_frame(x, y, z, box)
     _, _, c, n = g.result()
     assert n == 1 and np.array_equal(c.ravel(), np.asarray(o.cnt4).ravel())
     assert c.sum() > 0 and math.isfinite(c.sum())

@@ -2146,14 +2146,17 @@ struct yamc_rdf {
     int tile_grid = 1, tile_split = 1;
 };
 
-// From this many centres a frame without periodic images goes over near tiles: the sort's four
-// launches and the tiles' tests cost about 15 us, which all M^2 pairs pass at about a thousand centres
-constexpr int kRdfTileMin = 1024;
+// A frame without periodic images goes over near tiles from kRdfTileMin centres where rmax <= L/3, from
+// kRdfTileMinFar where it is longer and fewer tiles are too far.  The sort's four launches and the
+// tiles' tests cost 20 us more than all M^2 pairs at 1024 centres; a frame from host centres at water's
+// density, all pairs against tiles: rmax 12 A 47 / 57 us at 1024, 58 / 66 at 2000, 98 / 73 at 3000,
+// 169 / 82 at 4252, 520 / 118 at 8000; rmax L/2 72 / 88 at 2400, 174 / 144 at 4252, 562 / 318 at 8000.
+constexpr int kRdfTileMin = 2400, kRdfTileMinFar = 3600;
 constexpr size_t kRdfTileStatic = 40 * 1024;  // k_rdf_tiles' own shared memory beside the histogram
 
 static int rdf_frame(yamc_rdf *h, double L) {
     const int nbox = h->rmax < L / 2 ? 0 : (int)((h->rmax - L / 2) / L) + 1;  // mcrdf2.f90:206-210
-    if (nbox == 0 && h->tile_path) {
+    if (nbox == 0 && h->tile_path && (3 * h->rmax <= L || h->M >= kRdfTileMinFar)) {
         if (const int r = spatial_order(h->tiles, Points{h->cx, h->cy, h->cz, 1, h->M}, h->stream)) return r;
         k_rdf_tiles<<<dim3(h->tile_grid, h->tile_split), 256, h->smem, h->stream>>>(h->cx, h->cy, h->cz, h->type, h->tiles.order, h->tiles.box,
                                                                h->tiles.ntile, tile_reach2(h->rmax / L), h->M, h->ntypes,
