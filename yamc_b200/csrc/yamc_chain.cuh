@@ -1490,7 +1490,11 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
     const long long refresh_every = MX ? D.refresh_every : 0;
     int xpar = 0;  // parity of the cluster exchange buffer, flipped after every pass
     const long long n_moves = run->n_moves;
-    long long *prof = (A.prof && rank == 0) ? A.prof : nullptr;
+    // phase cycles are counted in shared memory (a counter in global memory costs a round trip per mark)
+    __shared__ long long prof_s[PH_COUNT];
+    long long *prof = (A.prof && rank == 0) ? prof_s : nullptr;
+    if (prof && tid < PH_COUNT) prof_s[tid] = 0;
+    if (prof) __syncthreads();
     const bool pc = prof && tid == 0;
     long long t_mark = 0;
 #define YAMC_PH(ph) do { if (pc) { const long long t_now = clock64(); prof[ph] += t_now - t_mark; t_mark = t_now; } } while (0)
@@ -1871,6 +1875,10 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
     }
 #undef YAMC_PH
 
+    if (prof) {
+        __syncthreads();
+        if (tid < PH_COUNT) A.prof[tid] += prof_s[tid];
+    }
     {  // write back the register and shared state
 #pragma unroll
         for (int k = 0; k < EPT; ++k)
