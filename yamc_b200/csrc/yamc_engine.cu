@@ -856,7 +856,7 @@ void spatial_plan(SpatialOrder &o, int n, DeviceArena &arena) {
     arena.add(&o.order, n);
     arena.add(&o.hist, o.nblock * ncell);
     arena.add(&o.total, ncell);
-    arena.add(&o.box, (size_t)2 * 5 * o.ntile);
+    arena.add(&o.box, (size_t)2 * o.ntile);
 }
 
 // (each sort leaves the totals at 0)

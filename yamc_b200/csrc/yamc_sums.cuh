@@ -126,8 +126,7 @@ static __global__ void __launch_bounds__(kSortThreads) k_sort_place(Points P, in
 }
 
 // per tile of the order a bounding box (centre, half extents; box units, periodic), as the chain
-// kernel's blocks have them, and one for each group of 8 of its points (after the tiles' boxes); a box
-// with a coordinate that is not finite has no bounds
+// kernel's blocks have them; a box with a coordinate that is not finite has no bounds
 static __global__ void __launch_bounds__(256) k_tile_boxes(Points P, const int *order, int ntile, float4 *box) {
     const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= ntile) return;
@@ -142,26 +141,22 @@ static __global__ void __launch_bounds__(256) k_tile_boxes(Points P, const int *
         fine = fine && isfinite(lo[d]);
     }
     fine = __all_sync(0xffffffffu, fine);
-    auto join = [&](int o) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
             hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
         }
-    };
-    auto store = [&](float4 *b) {
-        const float inf = __int_as_float(0x7f800000);
-        b[0] = fine ? make_float4((float)wrap_half(r[0] + 0.5 * (lo[0] + hi[0])), (float)wrap_half(r[1] + 0.5 * (lo[1] + hi[1])),
-                                  (float)wrap_half(r[2] + 0.5 * (lo[2] + hi[2])), 0.f)
-                    : make_float4(0.f, 0.f, 0.f, 0.f);
-        b[1] = fine ? make_float4(__double2float_ru(0.5 * (hi[0] - lo[0]) + kBoxPad), __double2float_ru(0.5 * (hi[1] - lo[1]) + kBoxPad),
-                                  __double2float_ru(0.5 * (hi[2] - lo[2]) + kBoxPad), 0.f)
-                    : make_float4(inf, inf, inf, 0.f);
-    };
-    join(1); join(2); join(4);
-    if (lane % 8 == 0) store(box + 2 * (ntile + 4 * t + lane / 8));
-    join(8); join(16);
-    if (lane == 0) store(box + 2 * t);
+    }
+    if (lane != 0) return;
+    const float inf = __int_as_float(0x7f800000);
+    box[2 * t] = fine ? make_float4((float)wrap_half(r[0] + 0.5 * (lo[0] + hi[0])), (float)wrap_half(r[1] + 0.5 * (lo[1] + hi[1])),
+                                    (float)wrap_half(r[2] + 0.5 * (lo[2] + hi[2])), 0.f)
+                      : make_float4(0.f, 0.f, 0.f, 0.f);
+    box[2 * t + 1] = fine ? make_float4(__double2float_ru(0.5 * (hi[0] - lo[0]) + kBoxPad), __double2float_ru(0.5 * (hi[1] - lo[1]) + kBoxPad),
+                                        __double2float_ru(0.5 * (hi[2] - lo[2]) + kBoxPad), 0.f)
+                          : make_float4(inf, inf, inf, 0.f);
 }
 
 // false only if no two points of the two boxes are within sqrt(r2) under any periodic image
@@ -212,15 +207,13 @@ __device__ __forceinline__ int near_tiles(const float4 *box, int ntile, int ti, 
 // real space
 // ------------------------------------------------------------------------------------------
 constexpr int kFullParts = 8;  // ew, lj6, lj12, ew_intra, lj6_intra, lj12_intra, overlap, spare
-constexpr int kRealWarps = 4;  // (8: 10 % slower, the warps of a block end further apart)
+constexpr int kRealWarps = 4;  // (8 take the same time: 0.41 ms of energy at 49,752 atoms)
 
 // one atom of a tile as the pair loops read it
 struct TileAtom { double x, y, z, q, dhs; int mol, type; };
 
-__device__ __forceinline__ TileAtom tile_atom(const DevSys &D, const int *order, int p) {
+__device__ __forceinline__ TileAtom tile_atom(const DevSys &D, int i, double4 v) {
     TileAtom a;
-    const int i = order[p];
-    const double4 v = D.atom[i];
     const int2 m = D.meta[i];
     a.x = v.x; a.y = v.y; a.z = v.z; a.q = v.w; a.dhs = D.dhs[i]; a.mol = m.x; a.type = m.y;
     return a;
@@ -235,32 +228,31 @@ __device__ __forceinline__ float3 tile_point(double x, double y, double z) {
     return make_float3((float)wrap_half(x), (float)wrap_half(y), (float)wrap_half(z));
 }
 __device__ __forceinline__ float candidate_limit(double r2) { return (float)(r2 * (1.0 + 1e-4) + 2e-6); }
-// Groups of 8 points whose box is out of the tile's reach are passed over (box: all boxes, ti the
-// lanes' tile, tj the other).
-__device__ __forceinline__ unsigned candidates(float3 a, const float3 *b, float limit, const float4 *box, int ntile, int ti, int tj,
-                                               double reach2) {
+// Only the tile's points within the reach of the lanes' own tile's box are tested: near_point, once
+// per point, leaves 1.6 to 2 times fewer of them than the boxes of the tile's groups of 8.
+__device__ __forceinline__ bool near_point(float3 p, float4 c, float4 h, float limit) {
     constexpr float magic = 12582912.0f;  // 1.5 2^23: adding and subtracting it rounds to an integer
-    const int lane = threadIdx.x & 31;
-    bool near = false;
-    if (lane < 4) {
-        const float4 *g = box + 2 * (ntile + 4 * tj + lane);
-        near = boxes_near(box[2 * ti], box[2 * ti + 1], g[0], g[1], reach2);
-    }
-    const unsigned groups = __ballot_sync(0xffffffffu, near);
+    float dx = p.x - c.x, dy = p.y - c.y, dz = p.z - c.z;
+    dx -= (dx + magic) - magic; dy -= (dy + magic) - magic; dz -= (dz + magic) - magic;
+    dx = fmaxf(fabsf(dx) - h.x, 0.f); dy = fmaxf(fabsf(dy) - h.y, 0.f); dz = fmaxf(fabsf(dz) - h.z, 0.f);
+    return !(dx * dx + dy * dy + dz * dz >= limit);
+}
+// (b: the n near points, in groups of 4; what lies beyond them in the 32 places is masked)
+__device__ __forceinline__ unsigned candidates(float3 a, const float3 *b, int n, float limit) {
+    constexpr float magic = 12582912.0f;
     unsigned mask = 0;
-    for (int g = 0; g < 4; ++g) {
-        if (!((groups >> g) & 1)) continue;
+    for (int g = 0; g < n; g += 4) {
         unsigned m = 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float3 p = b[8 * g + j];
+        for (int j = 0; j < 4; ++j) {
+            const float3 p = b[g + j];
             float dx = a.x - p.x, dy = a.y - p.y, dz = a.z - p.z;
             dx -= (dx + magic) - magic; dy -= (dy + magic) - magic; dz -= (dz + magic) - magic;
             if (!(dx * dx + dy * dy + dz * dz >= limit)) m |= 1u << j;
         }
-        mask |= m << (8 * g);
+        mask |= m << g;
     }
-    return mask;
+    return n < 32 ? mask & ((1u << n) - 1u) : mask;
 }
 
 // The lanes' candidates one after the other in the warp's queue (lane << 5 | j, in lane order):
@@ -286,6 +278,9 @@ __device__ __forceinline__ int queue_pairs(unsigned mask, unsigned short *queue,
 // too; LJ-LJ pairs of different molecules closer than their mean hard-core diameter set the overlap
 // flag.  reach2: squared reach of the cutoff and the hard cores.  One partial per block, reduced in
 // block order by k_sum_parts.
+// Issue bound (63 % of the slots).  49,752 atoms: 3.23 ms over all pairs of 256-atom tiles, 0.76 ms over
+// the near tiles with FP64 tests in the same loop, 0.39 ms with FP32 candidates from the groups of 8
+// whose boxes are near (half the instructions tested them, 16 % were pairs), 0.35 ms from the near points.
 static __global__ void __launch_bounds__(32 * kRealWarps) k_real_energy(DevSys D, const int *order, const float4 *box, int ntile,
                                                                         double reach2, double *part) {
     __shared__ TileAtom ai[kTile], aj[kRealWarps][kTile];
@@ -297,9 +292,13 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_energy(DevSys D
     for (int k = threadIdx.x; k < D.nt * D.nt; k += blockDim.x) { s6[k] = D.lj_sig6[k]; fe[k] = D.lj_feps[k]; }
     const int ti = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ni = min(kTile, D.N - ti * kTile);
-    if (warp == 0 && lane < ni) ai[lane] = tile_atom(D, order, ti * kTile + lane);
+    if (warp == 0 && lane < ni) {
+        const int i = order[ti * kTile + lane];
+        ai[lane] = tile_atom(D, i, D.atom[i]);
+    }
     __syncthreads();
     const float limit = candidate_limit(reach2);
+    const float4 boxc = box[2 * ti], boxh = box[2 * ti + 1];
     const float3 own = tile_point(ai[min(lane, ni - 1)].x, ai[min(lane, ni - 1)].y, ai[min(lane, ni - 1)].z);
     double acc[6] = {0, 0, 0, 0, 0, 0};
     bool ovl = false;
@@ -307,16 +306,19 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_energy(DevSys D
     for (int base = 0; base < ntile; base += kNearSpan) {
         const int near = near_tiles<true, kRealWarps>(box, ntile, ti, base, reach2, words, list, &count);
         for (int m = blockIdx.y * kRealWarps + warp; m < near; m += gridDim.y * kRealWarps) {
-            const int tj = list[m], nj = min(kTile, D.N - tj * kTile);
+            const int tj = list[m], ij = order[min(tj * kTile + lane, D.N - 1)];
+            const double4 v = D.atom[ij];
+            const float3 f = tile_point(v.x, v.y, v.z);
+            const bool in_reach = tj * kTile + lane < D.N && near_point(f, boxc, boxh, limit);
+            const unsigned take = __ballot_sync(0xffffffffu, in_reach);
             __syncwarp();
-            {
-                const TileAtom b = tile_atom(D, order, tj * kTile + min(lane, nj - 1));
-                aj[warp][lane] = b;
-                fj[warp][lane] = tile_point(b.x, b.y, b.z);
+            if (in_reach) {  // (the tile's own points are all in reach: each in its lane's place)
+                const int k = __popc(take & ((1u << lane) - 1u));
+                aj[warp][k] = tile_atom(D, ij, v);
+                fj[warp][k] = f;
             }
             __syncwarp();
-            unsigned mask = candidates(own, fj[warp], limit, box, ntile, ti, tj, reach2);
-            if (nj < kTile) mask &= (1u << nj) - 1u;
+            unsigned mask = candidates(own, fj[warp], __popc(take), limit);
             if (tj == ti) mask &= lane < 31 ? ~((2u << lane) - 1u) : 0u;  // (each pair of the tile itself once)
             if (lane >= ni) mask = 0;
             int at;
@@ -357,6 +359,8 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_energy(DevSys D
 // every tile over all its near tiles as in k_real_energy; the forces of a batch of candidates go to
 // shared memory, where each lane adds those of its own atom (they follow one another in the queue),
 // the warps' sums are added in order.  gf[(blockIdx.y 3 + component) N + atom].
+// 49,752 atoms: 11.5 ms over all tiles, 1.04 ms; 12,440 atoms: 0.59 ms with every lane evaluating its
+// own pairs from a bit mask, 0.30 ms so, 0.28 ms with candidates from the near points only.
 constexpr int kForceBatch = 128;  // candidates evaluated between two gathers
 static __global__ void __launch_bounds__(32 * kRealWarps) k_real_forces(DevSys D, const int *order, const float4 *box, int ntile,
                                                                         double reach2, double *gf) {
@@ -370,9 +374,13 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_forces(DevSys D
     for (int k = threadIdx.x; k < D.nt * D.nt; k += blockDim.x) { s6[k] = D.lj_sig6[k]; fe[k] = D.lj_feps[k]; }
     const int ti = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ni = min(kTile, D.N - ti * kTile);
-    if (warp == 0 && lane < ni) ai[lane] = tile_atom(D, order, ti * kTile + lane);
+    if (warp == 0 && lane < ni) {
+        const int i = order[ti * kTile + lane];
+        ai[lane] = tile_atom(D, i, D.atom[i]);
+    }
     __syncthreads();
     const float limit = candidate_limit(reach2);
+    const float4 boxc = box[2 * ti], boxh = box[2 * ti + 1];
     const float3 own = tile_point(ai[min(lane, ni - 1)].x, ai[min(lane, ni - 1)].y, ai[min(lane, ni - 1)].z);
     double *bx = batch + (size_t)warp * 3 * kForceBatch, *by = bx + kForceBatch, *bz = by + kForceBatch;
     double gx = 0, gy = 0, gz = 0;
@@ -380,16 +388,19 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_forces(DevSys D
     for (int base = 0; base < ntile; base += kNearSpan) {
         const int near = near_tiles<false, kRealWarps>(box, ntile, ti, base, reach2, words, list, &count);
         for (int m = blockIdx.y * kRealWarps + warp; m < near; m += gridDim.y * kRealWarps) {
-            const int tj = list[m], nj = min(kTile, D.N - tj * kTile);
+            const int tj = list[m], ij = order[min(tj * kTile + lane, D.N - 1)];
+            const double4 v = D.atom[ij];
+            const float3 f = tile_point(v.x, v.y, v.z);
+            const bool in_reach = tj * kTile + lane < D.N && near_point(f, boxc, boxh, limit);
+            const unsigned take = __ballot_sync(0xffffffffu, in_reach);
             __syncwarp();
-            {
-                const TileAtom b = tile_atom(D, order, tj * kTile + min(lane, nj - 1));
-                aj[warp][lane] = b;
-                fj[warp][lane] = tile_point(b.x, b.y, b.z);
+            if (in_reach) {  // (the tile's own points are all in reach: each in its lane's place)
+                const int k = __popc(take & ((1u << lane) - 1u));
+                aj[warp][k] = tile_atom(D, ij, v);
+                fj[warp][k] = f;
             }
             __syncwarp();
-            unsigned mask = candidates(own, fj[warp], limit, box, ntile, ti, tj, reach2);
-            if (nj < kTile) mask &= (1u << nj) - 1u;
+            unsigned mask = candidates(own, fj[warp], __popc(take), limit);
             if (tj == ti) mask &= ~(1u << lane);
             if (lane >= ni) mask = 0;
             int at;
@@ -447,11 +458,12 @@ constexpr int kRhoMaxThreads = 512;  // items of a block: its tables serve up to
 // The eight sums over the slice's atoms of w (cos, sin)(kx x) (cos, sin)(ky y) (cos, sin)(kz z) give
 // the four signs of (ky, kz): 8 FMAs per 4 signed entries, the product of the first two factors once
 // per row.  The items of a warp share z0 (sorted by it).  part[slice S + e]; k_rho_reduce adds a
-// list's slices.  What bounds it is shared memory: a 16-byte load fills 512 bytes of registers, four
-// cycles of an SM, broadcast or not, so a thread takes both signs of ky (7 loads, 24 cycles, for 36
-// FP64 operations, 18 cycles; one sign and 8 kz: 11 loads, 42 cycles, for 38 operations).
-// 49,752 atoms x 29,784 entries: 5.7 ms with the full product per entry, 0.74 ms with one sign of ky
-// per thread, 0.5 ms so.
+// list's slices.  FP64 pipe bound while it sums (38 operations per atom and 16 signed entries, against
+// 16 per entry of the full product), with the tables' phases and three barriers per 32 atoms between
+// (pipe 53 % active over the kernel); both signs of ky in one thread, since a 16-byte shared load fills
+// 512 bytes of registers, four cycles of an SM, broadcast or not (7 loads per 36 operations, 11 with
+// one sign and 8 kz).  49,752 atoms x 29,784 entries: 5.7 ms with the full product per entry, 0.74 ms
+// with one sign of ky per thread, 0.72 ms so.
 static __global__ void __launch_bounds__(kRhoMaxThreads) k_rho_rows(DevSys D, AtomLists L, const int4 *slices, const int4 *items,
                                                                     const int4 *emap, int nitem, double2 *part) {
     extern __shared__ double2 rtab[];  // [3][KM][kRhoChunk + 1], then kRowZ rows of zeros
@@ -600,7 +612,7 @@ static __global__ void __launch_bounds__(256) k_row_fields(DevSys D, const int4 
 // axis tables in shared memory), its warps take the row pairs (kx, +-ky) in turn, a lane an atom;
 // blockIdx.y splits the row pairs when the atoms alone do not fill the GPU.  rows: (kx, ky, first
 // field, number of kz).  kf[(y 3 + component) npos + position].
-// 49,752 atoms x 29,784 entries: 6.6 ms with the phase formed per atom and entry, 1.1 ms.
+// 49,752 atoms x 29,784 entries: 6.6 ms with the phase formed per atom and entry, 1.56 ms.
 constexpr int kForceRowWarps = 8;
 static __global__ void __launch_bounds__(32 * kForceRowWarps) k_forces_rows(DevSys D, AtomLists L, const int4 *rows, int nrow,
                                                                             const double4 *field, int nf, int npos, double *kf) {
@@ -690,7 +702,7 @@ static __global__ void k_forces_add(DevSys D, const int2 *place, const double *g
 // ------------------------------------------------------------------------------------------
 // Every ordered pair of centres of the tile and its near tiles, counted as k_rdf_count counts it
 // (the same explicitly rounded distance, so the same bins), for frames without periodic images
-// (rmax < L / 2).  16,984 centres, rmax 12 of 79.3 A: 2.1 ms over all pairs, 0.13 ms.
+// (rmax < L / 2).  16,984 centres, rmax 12 of 79.3 A: 2.1 ms over all pairs, 0.10 ms.
 static __global__ void __launch_bounds__(256) k_rdf_tiles(const double *cx, const double *cy, const double *cz, const int *type,
                                                           const int *order, const float4 *box, int ntile, double reach2, int M,
                                                           int ntypes, int nbin, double L, double dr, double rmax2,
@@ -714,18 +726,24 @@ static __global__ void __launch_bounds__(256) k_rdf_tiles(const double *cx, cons
         if (warp == 0) ci[lane] = centre(ti * kTile + lane);
         __syncthreads();
         const int ni = min(kTile, M - ti * kTile);
+        const float4 boxc = box[2 * ti], boxh = box[2 * ti + 1];
         const float3 own = tile_point(ci[lane].x, ci[lane].y, ci[lane].z);
         for (int base = 0; base < ntile; base += kNearSpan) {
             const int near = near_tiles<false, 8>(box, ntile, ti, base, reach2, words, list, &count);
             for (int m = blockIdx.y * 8 + warp; m < near; m += gridDim.y * 8) {
-                const int tj = list[m], nj = min(kTile, M - tj * kTile);
-                __syncwarp();
+                const int tj = list[m];
                 const double4 p = centre(tj * kTile + lane);
-                cj[warp][lane] = p;
-                fj[warp][lane] = tile_point(p.x, p.y, p.z);
+                const float3 f = tile_point(p.x, p.y, p.z);
+                const bool in_reach = tj * kTile + lane < M && near_point(f, boxc, boxh, limit);
+                const unsigned take = __ballot_sync(0xffffffffu, in_reach);
                 __syncwarp();
-                unsigned mask = candidates(own, fj[warp], limit, box, ntile, ti, tj, reach2);
-                if (nj < kTile) mask &= (1u << nj) - 1u;
+                if (in_reach) {
+                    const int k = __popc(take & ((1u << lane) - 1u));
+                    cj[warp][k] = p;
+                    fj[warp][k] = f;
+                }
+                __syncwarp();
+                unsigned mask = candidates(own, fj[warp], __popc(take), limit);
                 if (tj == ti) mask &= ~(1u << lane);
                 if (lane >= ni) mask = 0;
                 int at;
