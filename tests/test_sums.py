@@ -77,6 +77,28 @@ def test_real_space_tiles_with_molecules_outside_the_box(tmp_path, n_water, n_io
     assert np.abs(eng.forces()[0] - f0).max() <= 1e-12 * np.abs(f0).max()
 
 
+@pytest.mark.parametrize("n_water,n_ion", [(2350, 3), (2355, 40)])
+def test_force_rows_of_two_atoms_per_lane(tmp_path, n_water, n_ion):
+    """Against the oracle's forces (erfc in place of erfc_Luc: 2e-4 of the force scale), and the same
+    forces for molecules listed in another order (other lanes, blocks and halves of them)."""
+    box = ((n_water + 2 * n_ion) / 0.0334) ** (1 / 3)
+    spec = systems.SystemSpec("wide", n_water, n_ion, n_ion, box, 3.2 / 9.0, 9.0, 5)
+    files = systems.write_system(spec, str(tmp_path), seed=n_water)
+    inp = api.load_inputs(files["parameters"], files["composition"], files["moltab"])
+    eng = api.Engine(inp)
+    f, mf, _ = eng.forces()
+    scale = math.sqrt((mf ** 2).sum(1).mean())
+    o = pyoracle.Oracle(files)
+    for imol in (1, 2, n_water // 2, n_water, n_water + 1, n_water + n_ion, n_water + 2 * n_ion):
+        assert np.all(np.abs(o.move_old(imol)[0] - mf[imol - 1]) <= 2e-4 * scale)
+    x = np.stack([inp.x, inp.y, inp.z], 1)
+    perm = np.arange(len(x))
+    perm[:3 * n_water] = perm[:3 * n_water].reshape(-1, 3)[::-1].ravel()
+    perm[3 * n_water:3 * n_water + n_ion] = perm[3 * n_water:3 * n_water + n_ion][::-1]
+    eng.set_positions(*(np.ascontiguousarray(v) for v in x[perm].T))
+    assert np.abs(eng.forces()[0] - f[perm]).max() <= 1e-12 * np.abs(f).max()
+
+
 @pytest.mark.parametrize("box", [31.0, 40.0])  # rmax above and below a third of the box
 @pytest.mark.parametrize("m", [1023, 1024, 1057, 2001, 2399, 2400, 2433, 3599, 3600, 4001])
 def test_rdf_tiles_count_as_all_pairs(m, box):

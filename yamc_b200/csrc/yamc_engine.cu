@@ -1122,8 +1122,14 @@ int ensure_cfg(yamc_ctx *c) {
 template <int NT>
 int launch_forces(yamc_ctx *c) {
     const HostSystem &H = c->H;
-    const size_t sm = sizeof(double2) * 32 * 3 * (H.kmax + 1), smr = sizeof(double) * kRealWarps * 3 * kForceBatch;
-    const int nblk = c->k_npos / 32, shares = tile_shares(c->tiles.ntile, c->nsm);
+    const size_t smr = sizeof(double) * kRealWarps * 3 * kForceBatch;
+    const int shares = tile_shares(c->tiles.ntile, c->nsm);
+    // two atoms per lane of k_forces_rows where two blocks' tables still fit an SM and the halved blocks
+    // fill the GPU without a split of the rows
+    const int atoms = 2 * (sizeof(double2) * 64 * 3 * (H.kmax + 1)) <= 200 * 1024 && c->k_npos / 32 >= 2 * c->nsm ? 2 : 1;
+    const size_t sm = sizeof(double2) * 32 * atoms * 3 * (H.kmax + 1);
+    int nblk = 0;
+    for (int l = 0; l < kMaxLists; ++l) nblk += (c->k_lbeg[l + 1] - c->k_lbeg[l] + 32 * atoms - 1) / (32 * atoms);
     // the row pairs split over blockIdx.y until the blocks fill the GPU about four times
     const int nsplit = std::max(1, std::min((4 * c->nsm + nblk - 1) / nblk, (c->k_nfrow + kForceRowWarps - 1) / kForceRowWarps));
     int r;
@@ -1136,9 +1142,10 @@ int launch_forces(yamc_ctx *c) {
     CUDA_TRY(cudaGetLastError());
     k_row_fields<NT><<<dim3((c->k_nf + 255) / 256, 1 + NT), 256, 0, c->stream>>>(c->hsys, c->k_fmap, c->k_nf, c->d_field);
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaFuncSetAttribute(k_forces_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_forces_rows<<<dim3(nblk, nsplit), 32 * kForceRowWarps, sm, c->stream>>>(c->hsys, atom_lists(c), c->k_frows, c->k_nfrow,
-                                                                              c->d_field, c->k_nf, c->k_npos, c->d_kf);
+    auto *rows = atoms == 2 ? k_forces_rows<2> : k_forces_rows<1>;
+    CUDA_TRY(cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    rows<<<dim3(nblk, nsplit), 32 * kForceRowWarps, sm, c->stream>>>(c->hsys, atom_lists(c), c->k_frows, c->k_nfrow, c->d_field,
+                                                                     c->k_nf, c->k_npos, c->d_kf);
     CUDA_TRY(cudaGetLastError());
     k_forces_add<<<(H.N + 255) / 256, 256, 0, c->stream>>>(c->hsys, c->k_place, c->d_gf, shares, c->d_kf, c->k_npos, nsplit,
                                                            c->d_hpos);

@@ -359,7 +359,7 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_energy(DevSys D
 // every tile over all its near tiles as in k_real_energy; the forces of a batch of candidates go to
 // shared memory, where each lane adds those of its own atom (they follow one another in the queue),
 // the warps' sums are added in order.  gf[(blockIdx.y 3 + component) N + atom].
-// 49,752 atoms: 11.5 ms over all tiles, 1.04 ms; 12,440 atoms: 0.59 ms with every lane evaluating its
+// 49,752 atoms: 11.5 ms over all tiles, 0.93 ms; 12,440 atoms: 0.59 ms with every lane evaluating its
 // own pairs from a bit mask, 0.30 ms so, 0.28 ms with candidates from the near points only.
 constexpr int kForceBatch = 128;  // candidates evaluated between two gathers
 static __global__ void __launch_bounds__(32 * kRealWarps) k_real_forces(DevSys D, const int *order, const float4 *box, int ntile,
@@ -608,70 +608,93 @@ static __global__ void __launch_bounds__(256) k_row_fields(DevSys D, const int4 
 // k-space forces (ForceKSpace_coulomb / _LJ, ForceKSpace.f90:59-302): for an atom the weight of a
 // signed k vector is w = G.re sin - G.im cos of its phase; with A = X^kx Y^ky the sums over kz of a
 // row give w = A.im R1 + A.re R2 (and the kz-weighted sums the z component), 4 FMAs per signed k
-// vector, the phase of a single k vector never formed.  A block holds 32 atoms of one list (their
-// axis tables in shared memory), its warps take the row pairs (kx, +-ky) in turn, a lane an atom;
+// vector, the phase of a single k vector never formed.  A block holds 32 A atoms of one list (their
+// axis tables in shared memory), its warps take the row pairs (kx, +-ky) in turn, a lane A atoms;
 // blockIdx.y splits the row pairs when the atoms alone do not fill the GPU.  rows: (kx, ky, first
 // field, number of kz).  kf[(y 3 + component) npos + position].
-// 49,752 atoms x 29,784 entries: 6.6 ms with the phase formed per atom and entry, 1.56 ms.
+// With one atom per lane the loads bind: 4 uniform 16-byte loads and one of the lane's table per 18 FP64
+// operations, 20 cycles of an SM against 9.  Two atoms share the uniform loads (24 against 18).
+// 49,752 atoms x 29,784 entries: 6.6 ms with the phase formed per atom and entry, 1.56 ms with one
+// atom per lane, 1.23 ms with two.
 constexpr int kForceRowWarps = 8;
+template <int A>
 static __global__ void __launch_bounds__(32 * kForceRowWarps) k_forces_rows(DevSys D, AtomLists L, const int4 *rows, int nrow,
                                                                             const double4 *field, int nf, int npos, double *kf) {
-    extern __shared__ double2 ftab[];  // [3][KM][32]
-    __shared__ double red[kForceRowWarps][3][32];
+    constexpr int W = 32 * A;
+    extern __shared__ double2 ftab[];  // [3][KM][W]
+    __shared__ double red[kForceRowWarps][3][W];
     const int KM = D.kmax + 1;
-    const int p0 = blockIdx.x * 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int l = 0;
-    while (p0 >= L.lbeg[l + 1]) ++l;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int l = 0, b = blockIdx.x;
+    for (int n; b >= (n = (L.lbeg[l + 1] - L.lbeg[l] + W - 1) / W); ++l) b -= n;
+    const int p0 = L.lbeg[l] + W * b, pe = L.lbeg[l + 1];
     const double4 *F = field + (size_t)l * nf * 2;
-    for (int idx = threadIdx.x; idx < 32 * 3 * KM; idx += blockDim.x) {
-        const int r = idx / 32, d = r / KM, m = r % KM, i = L.alist[p0 + idx % 32];
+    for (int idx = threadIdx.x; idx < W * 3 * KM; idx += blockDim.x) {
+        const int r = idx / W, d = r / KM, m = r % KM, p = p0 + idx % W, i = p < pe ? L.alist[p] : -1;
         double s = 0.0, c = 0.0;
         if (i >= 0) {
-            const double4 p = D.atom[i];
-            const double u = d == 0 ? p.x : (d == 1 ? p.y : p.z);
+            const double4 v = D.atom[i];
+            const double u = d == 0 ? v.x : (d == 1 ? v.y : v.z);
             sincospi(2.0 * (double)m * u, &s, &c);
             if (m == 0) { s = 0.0; c = 1.0; }
         }
         ftab[idx] = make_double2(c, s);
     }
     __syncthreads();
-    double gx = 0, gy = 0, gz = 0;
+    double gx[A] = {}, gy[A] = {}, gz[A] = {};
     for (int r = blockIdx.y * kForceRowWarps + warp; r < nrow; r += gridDim.y * kForceRowWarps) {
         const int4 row = rows[r];
-        const double2 *tz = ftab + 2 * KM * 32 + lane;
+        const double2 *tz = ftab + 2 * KM * W + lane;
         const double4 *f = F + 2 * (size_t)row.z;
-        double r1[2] = {0, 0}, r2[2] = {0, 0}, z1[2] = {0, 0}, z2[2] = {0, 0};
-#pragma unroll 4
+        double r1[A][2] = {}, r2[A][2] = {}, z1[A][2] = {}, z2[A][2] = {};
+#pragma unroll (4 / A)
         for (int k = 0; k < row.w; ++k) {
-            const double2 Z = tz[k * 32];
-            const double kc = (double)k * Z.x, ks = (double)k * Z.y;
+            double2 Z[A];
+            double kc[A], ks[A];
+#pragma unroll
+            for (int a = 0; a < A; ++a) {
+                Z[a] = tz[k * W + 32 * a];
+                kc[a] = (double)k * Z[a].x; ks[a] = (double)k * Z[a].y;
+            }
 #pragma unroll
             for (int y = 0; y < 2; ++y) {
                 const double2 ab = __ldg(reinterpret_cast<const double2 *>(f + 2 * k + y));
                 const double2 cd = __ldg(reinterpret_cast<const double2 *>(f + 2 * k + y) + 1);
-                r1[y] += ab.x * Z.x; r1[y] += cd.y * Z.y;
-                r2[y] += ab.y * Z.y; r2[y] -= cd.x * Z.x;
-                z1[y] += ab.y * kc; z1[y] += cd.x * ks;
-                z2[y] += ab.x * ks; z2[y] -= cd.y * kc;
+#pragma unroll
+                for (int a = 0; a < A; ++a) {
+                    r1[a][y] += ab.x * Z[a].x; r1[a][y] += cd.y * Z[a].y;
+                    r2[a][y] += ab.y * Z[a].y; r2[a][y] -= cd.x * Z[a].x;
+                    z1[a][y] += ab.y * kc[a]; z1[a][y] += cd.x * ks[a];
+                    z2[a][y] += ab.x * ks[a]; z2[a][y] -= cd.y * kc[a];
+                }
             }
         }
-        const double2 X = ftab[row.x * 32 + lane], Y = ftab[(KM + row.y) * 32 + lane];
 #pragma unroll
-        for (int y = 0; y < 2; ++y) {
-            const double sy = y ? -Y.y : Y.y;
-            const double ar = X.x * Y.x - X.y * sy, ai = X.y * Y.x + X.x * sy;
-            const double w = ai * r1[y] + ar * r2[y];
-            gx += (double)row.x * w;
-            gy += (double)(y ? -row.y : row.y) * w;
-            gz += ai * z1[y] + ar * z2[y];
+        for (int a = 0; a < A; ++a) {
+            const double2 X = ftab[row.x * W + 32 * a + lane], Y = ftab[(KM + row.y) * W + 32 * a + lane];
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                const double sy = y ? -Y.y : Y.y;
+                const double ar = X.x * Y.x - X.y * sy, ai = X.y * Y.x + X.x * sy;
+                const double w = ai * r1[a][y] + ar * r2[a][y];
+                gx[a] += (double)row.x * w;
+                gy[a] += (double)(y ? -row.y : row.y) * w;
+                gz[a] += ai * z1[a][y] + ar * z2[a][y];
+            }
         }
     }
-    red[warp][0][lane] = gx; red[warp][1][lane] = gy; red[warp][2][lane] = gz;
+#pragma unroll
+    for (int a = 0; a < A; ++a) {
+        red[warp][0][32 * a + lane] = gx[a]; red[warp][1][32 * a + lane] = gy[a]; red[warp][2][32 * a + lane] = gz[a];
+    }
     __syncthreads();
     if (warp < 3) {
-        double x = 0;
-        for (int w = 0; w < kForceRowWarps; ++w) x += red[w][warp][lane];
-        kf[((size_t)blockIdx.y * 3 + warp) * npos + p0 + lane] = x;
+#pragma unroll
+        for (int a = 0; a < A; ++a) {
+            double x = 0;
+            for (int w = 0; w < kForceRowWarps; ++w) x += red[w][warp][32 * a + lane];
+            if (p0 + 32 * a < pe) kf[((size_t)blockIdx.y * 3 + warp) * npos + p0 + 32 * a + lane] = x;
+        }
     }
 }
 
