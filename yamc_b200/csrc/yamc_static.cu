@@ -10,13 +10,12 @@
 // inputs and outputs is the per-block partial-sum buffer below, a fixed file-scope
 // __device__ array.
 //
-// The kernel is a variant of the engine's k_realspace_full (the full real-space Ewald sum
-// of EwaldSumRealSpace_calc, EwaldSumRealSpace.f90:233-500, with j0 = i+1): the same pair
-// arithmetic, the same tile order and the same deterministic block reduction, but it reads
+// The kernel is the full real-space Ewald sum over all pairs (EwaldSumRealSpace_calc,
+// EwaldSumRealSpace.f90:233-500, with j0 = i+1) with the engine's pair arithmetic; it reads
 // the reference's structure-of-arrays atom data directly instead of the engine's packed
 // double4 layout, and a second one-block kernel adds the block partials in block order on
-// the device.  The engine's own full sum splits the pairs differently (blocks over pairs of
-// atom tiles), so the totals agree with yamc_full_sums to rounding, not bit for bit.
+// the device.  The engine's own full sum goes over near tiles of spatially ordered atoms
+// (k_real_energy), so the totals agree with yamc_full_sums to rounding, not bit for bit.
 #include <cuda_runtime.h>
 
 #include <cstdint>

@@ -7,7 +7,7 @@ warm-up and then REPEATS more times (default 3), timing each call on the host (t
 synchronises), then VOLUME_STEPS volume steps through yamc_volume_eval/_commit (default 0)
 and FORCES calls of the adjoint yamc_forces (default 0).
 Capture one kernel of the second call at a time, e.g.
-``ncu --clock-control none -k regex:k_realspace_full -s 1 -c 1`` (``--clock-control none`` leaves
+``ncu --clock-control none -k regex:k_real_energy -s 1 -c 1`` (``--clock-control none`` leaves
 the GPU's clocks as they are).
 """
 from __future__ import annotations
