@@ -267,6 +267,7 @@ struct ChainShared {
     int icur;             // buffer of the move being evaluated
     int spec[3];          // buffers of the candidates: after an overlap / after a draw / accepted same molecule
     int abort, accepted, overlap, last_mol, spec_ok;
+    int prop_out;         // the stream ran out in the proposal (a word of its own: see there)
     long long cursor;     // stream position after the last completed move
     long long icycle, mic;
     double eold[3];
@@ -1595,9 +1596,9 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
                         __syncwarp();
                     }
                     if (lane == 0) {
+                        sh.prop_out = out;
                         if (out) {
                             C.valid = 0;
-                            sh.abort = kAbortStream;
                         } else {
                             // old positions from slots [na0, 2 na0), new ones into [0, na0): no overlap
                             const Slot *os = C.slot + na0;
@@ -1613,10 +1614,16 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
                 RngReader rng = make_reader(X, sh, C.cur_prop);
                 propose(D, C, rng);
                 C.cur_prop = rng.cur();
-                if (rng.out) { C.valid = 0; sh.abort = kAbortStream; }
+                // (not into sh.abort: a warp that has yet to read it after the choice above would
+                // leave the loop alone, and the others wait for it at the next barrier)
+                sh.prop_out = rng.out;
+                if (rng.out) C.valid = 0;
             }
             __syncthreads();
-            if (sh.abort) break;
+            if (sh.prop_out) {
+                if (tid == 0) sh.abort = kAbortStream;
+                break;
+            }
             YAMC_PH(PH_PROPOSE);
         }
         const int na = sh.cand[sh.icur].na;
