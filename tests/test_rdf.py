@@ -94,3 +94,22 @@ def test_rdf_from_engine_matches_oracle(nacl_files):
     # water O-O peak near 2.8 A
     k = int(np.argmax(g[0, 0]))
     assert 2.5 < r[k] < 3.2, r[k]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,box", [(200, 30.0), (2500, 40.0), (4000, 30.0), (200, 9.0)])  # all pairs, tiles, tiles, images
+def test_rdf_centres_that_are_not_numbers_are_in_no_pair(m, box):
+    """Their distances are NaN, which is in no bin: the counts are those of the other centres."""
+    from yamc_b200 import api
+    r = np.random.default_rng(m)
+    x, y, z = r.uniform(-0.5, 0.5, (3, m))
+    x[3::97], y[5::101], z[7::89] = np.nan, np.nan, np.inf
+    mol_type = np.where(np.arange(m) % 3 == 0, 2, 1).astype(np.int32)
+    counts = np.array([(mol_type == 1).sum(), (mol_type == 2).sum()], dtype=np.int32)
+    keep = np.isfinite(x) & np.isfinite(y) & np.isfinite(z)
+    o = pyoracle.RDF(mol_type[keep], np.array([(mol_type[keep] == t).sum() for t in (1, 2)], dtype=np.int32), dr=0.1, rmax=12.0)
+    o.add_frame(x[keep], y[keep], z[keep], box)
+    gpu = api.RDF(mol_type, counts, dr=0.1, rmax=12.0)
+    gpu.add_frame(x, y, z, box)
+    _, _, c, nf = gpu.result()
+    assert nf == 1 and keep.sum() < m and np.array_equal(c, o.cnt4.reshape(c.shape))

@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256) k_rdf_count(const double *cx, const doubl
                     const double dy = __dmul_rn(__dadd_rn(__dsub_rn(y1, y2), (double)ny), L);
                     const double dz = __dmul_rn(__dadd_rn(__dsub_rn(z1, z2), (double)nz), L);
                     const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-                    if (r2 > __dsub_rn(rmax2, 1e-10)) continue;
+                    if (!(r2 <= __dsub_rn(rmax2, 1e-10))) continue;  // (a NaN, whose bin would be no index, too)
                     const int b = (int)__ddiv_rn(__dsqrt_rn(r2), dr);
                     atomicAdd(&hs[npair * nbin + off], 1u);
                     if (b < nbin) atomicAdd(&hs[off * nbin + b], 1u);

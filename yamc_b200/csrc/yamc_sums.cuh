@@ -784,7 +784,7 @@ static __global__ void __launch_bounds__(256) k_rdf_tiles(const double *cx, cons
                     const double dx = __dmul_rn(__dsub_rn(a.x, x2), L), dy = __dmul_rn(__dsub_rn(a.y, y2), L),
                                  dz = __dmul_rn(__dsub_rn(a.z, z2), L);
                     const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-                    if (r2 > __dsub_rn(rmax2, 1e-10)) continue;
+                    if (!(r2 <= __dsub_rn(rmax2, 1e-10))) continue;  // (a NaN, whose bin would be no index, too)
                     const int t1 = (int)a.w, t2 = (int)b.w, off = t1 < t2 ? t1 * ntypes + t2 : t2 * ntypes + t1;
                     const int bin = (int)__ddiv_rn(__dsqrt_rn(r2), dr);
                     atomicAdd(&hs[npair * nbin + off], 1u);
