@@ -1,0 +1,35 @@
+"""Systems whose atoms fill a CTA's shared memory to the last bytes: the launch picker takes the
+larger cluster exactly where the smaller one no longer fits beside the chain kernel's static part, so
+every size in a range around that limit builds and runs.  Energies of the moved configuration against
+its full recomputation, 1e-9 relative."""
+import numpy as np
+import pytest
+
+from yamc_b200 import api, rng as grng, systems
+
+pytestmark = pytest.mark.gpu
+
+
+def _water(n, directory, kmax=10):
+    box = (n / 0.015) ** (1 / 3)
+    spec = systems.SystemSpec("water", n, 0, 0, box, 3.0 / 9.0, 9.0, kmax)
+    f = systems.write_system(spec, directory, seed=3)
+    return api.load_inputs(f["parameters"], f["composition"], f["moltab"])
+
+
+# one atom more is 40 bytes and a block of 32 atoms another 32, so the waters of the range step over
+# the limit in parts of 120 bytes
+@pytest.mark.parametrize("cluster,waters", [(1, range(1660, 1700)), (2, range(3330, 3390, 2))])
+def test_every_size_around_the_shared_memory_limit_runs(tmp_path, cluster, waters):
+    seen = set()
+    moves = 6
+    stream = grng.gfortran_stream(5, 60 * moves)
+    for n in waters:
+        b = api.Batch([_water(n, str(tmp_path / str(n)))])
+        _, _, done, st, s = b.run([stream], moves)
+        assert s == 0 and st[0] == 0 and done[0] == moves, n
+        view = b.replica(0)
+        assert np.all(np.abs(view.energies() - view.full_sums()) <= 1e-9 * np.maximum(np.abs(view.full_sums()), 1.0)), n
+        seen.add(b.launch["cluster_blocks"])
+        b.close()
+    assert seen == {cluster, cluster + 1}

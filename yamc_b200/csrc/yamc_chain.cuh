@@ -293,6 +293,18 @@ struct ChainShared {
     int wnext;
 };
 
+// All static shared memory of the chain kernel: one object, so the host that plans the dynamic part
+// (pick_launch_for) knows its size.
+struct __align__(16) ChainStatic {
+    ChainShared sh;
+    float rwin[2][kWin];  // the windows of the random stream
+    // the system's parameters and array pointers: every thread reads them from here (a per-thread
+    // copy would live in local memory, which the staged atoms leave little L1 for)
+    DevSys sys;
+    // phase cycles (a counter in global memory costs a round trip per mark)
+    long long prof[PH_COUNT];
+};
+
 // why a chain stops before its last move (ChainShared::abort)
 constexpr int kAbortStream = 1;     // the random stream ran out (YAMC_ERNG_EXHAUSTED, resumable)
 constexpr int kAbortNonFinite = 2;  // a non-finite energy change or bias force (YAMC_ENAN)
@@ -1359,23 +1371,21 @@ __device__ __noinline__ void refresh_in_chain(const DevSys &D, double2 *scr, int
 template <int NT, int EPT, bool SPLIT, bool MX>
 __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThreads, 1) k_chain(ChainArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ ChainShared sh;
-    __shared__ float rwin[2][kWin];
+    __shared__ ChainStatic st;
+    ChainShared &sh = st.sh;
+    float(&rwin)[2][kWin] = st.rwin;
 
     cg::cluster_group cluster = cg::this_cluster();
     const int G = A.G;
     const int rank = G > 1 ? (int)cluster.block_rank() : 0;
     const int rep = blockIdx.x / G;
-    // the system's parameters and array pointers in shared memory: every thread reads them from
-    // there (a per-thread copy would live in local memory, which the staged atoms leave little L1 for)
-    __shared__ DevSys D_s;
     {
         const int *src = reinterpret_cast<const int *>(A.sys + rep);
-        int *dst = reinterpret_cast<int *>(&D_s);
+        int *dst = reinterpret_cast<int *>(&st.sys);
         for (int i = threadIdx.x; i < (int)(sizeof(DevSys) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
         __syncthreads();
     }
-    const DevSys &D = D_s;
+    const DevSys &D = st.sys;
     RunSlot *run = A.run + rep;
     const int B = blockDim.x;
     const int tid = threadIdx.x;
@@ -1491,10 +1501,8 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
     const long long refresh_every = MX ? D.refresh_every : 0;
     int xpar = 0;  // parity of the cluster exchange buffer, flipped after every pass
     const long long n_moves = run->n_moves;
-    // phase cycles are counted in shared memory (a counter in global memory costs a round trip per mark)
-    __shared__ long long prof_s[PH_COUNT];
-    long long *prof = (A.prof && rank == 0) ? prof_s : nullptr;
-    if (prof && tid < PH_COUNT) prof_s[tid] = 0;
+    long long *prof = (A.prof && rank == 0) ? st.prof : nullptr;
+    if (prof && tid < PH_COUNT) prof[tid] = 0;
     if (prof) __syncthreads();
     const bool pc = prof && tid == 0;
     long long t_mark = 0;
@@ -1884,7 +1892,7 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
 
     if (prof) {
         __syncthreads();
-        if (tid < PH_COUNT) A.prof[tid] += prof_s[tid];
+        if (tid < PH_COUNT) A.prof[tid] += prof[tid];
     }
     {  // write back the register and shared state
 #pragma unroll

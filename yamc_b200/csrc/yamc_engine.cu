@@ -699,15 +699,15 @@ struct yamc_ctx {
 namespace {
 
 // The first (G, B) that fits every system of hosts: each worker thread holds at most 2 signed
-// entries, the CTA's atoms and the pair queue fit in shared memory.  G (1..16 CTAs per cluster)
+// entries, the CTA's atoms and the warps' buffers fit in shared memory.  G (1..16 CTAs per cluster)
 // from large to small when large_first (the shortest move for a lone chain), else from small to
 // large; B from 256 to 128 threads; force_G / force_B pin either (0 = free).
 int pick_launch_for(const std::vector<const HostSystem *> &hosts, int device, int force_G, int force_B, int layout,
                     bool mx, LaunchCfg *out, bool large_first = true) {
     cudaDeviceProp prop;
     CUDA_TRY(cudaGetDeviceProperties(&prop, device));
-    // the kernel's static shared memory (ChainShared and the two random-stream windows) comes first
-    const size_t smem_max = prop.sharedMemPerBlockOptin - sizeof(ChainShared) - sizeof(float) * 2 * kWin - 256;
+    // what the kernel's static shared memory leaves of a block's
+    const size_t smem_max = prop.sharedMemPerBlockOptin - sizeof(ChainStatic);
     int Smax = 0, Nmax = 0, Nmin = 1 << 30, kmax = 0, nt = 0;
     for (const HostSystem *h : hosts) {
         Smax = std::max(Smax, h->S); Nmax = std::max(Nmax, h->N); Nmin = std::min(Nmin, h->N);
