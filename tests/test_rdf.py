@@ -113,3 +113,24 @@ def test_rdf_centres_that_are_not_numbers_are_in_no_pair(m, box):
     gpu.add_frame(x, y, z, box)
     _, _, c, nf = gpu.result()
     assert nf == 1 and keep.sum() < m and np.array_equal(c, o.cnt4.reshape(c.shape))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [300, 2500])  # all pairs, tiles
+def test_rdf_handles_of_different_sizes_side_by_side(m):
+    """A handle made later, with fewer bins or one species, takes nothing from one with more: a block's
+    shared memory limit belongs to the kernel, not to the handle."""
+    from yamc_b200 import api
+    r = np.random.default_rng(m)
+    x, y, z = r.uniform(-0.5, 0.5, (3, m))
+    mol_type = np.where(np.arange(m) % 3 == 0, 2, 1).astype(np.int32)
+    counts = np.array([(mol_type == 1).sum(), (mol_type == 2).sum()], dtype=np.int32)
+    shapes = [(mol_type, counts, 0.001), (np.ones(m, dtype=np.int32), np.array([m], dtype=np.int32), 0.1), (mol_type, counts, 0.01)]
+    gpu = [api.RDF(t, c, dr=dr, rmax=10.0) for t, c, dr in shapes]
+    for k in (0, 1, 2, 0):
+        t, c, dr = shapes[k]
+        o = pyoracle.RDF(t, c, dr=dr, rmax=10.0)
+        before = gpu[k].result()[2]
+        gpu[k].add_frame(x, y, z, 40.0)
+        o.add_frame(x, y, z, 40.0)
+        assert np.array_equal(gpu[k].result()[2] - before, o.cnt4.reshape(before.shape))

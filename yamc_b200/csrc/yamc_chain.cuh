@@ -7,6 +7,7 @@
 #include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 #include <type_traits>
 
@@ -29,6 +30,25 @@
 namespace yamc {
 
 namespace cg = cooperative_groups;
+
+// Lets blocks of `kernel` have `bytes` of dynamic shared memory.  The limit belongs to the kernel
+// on the device, for the whole process: it is only ever raised, and to all that a block can have, so
+// no handle or thread takes back what another has planned with.  Kernels start with 48 KB, their
+// static part included, of which none here takes more than 36 (k_rdf_tiles: 33): small requests need
+// no query, which takes 0.6 us (a host-driven move makes two).
+template <class Kernel>
+int grant_smem(Kernel *kernel, size_t bytes) {
+    if (bytes <= 12 * 1024) return YAMC_OK;
+    cudaFuncAttributes a;
+    CUDA_TRY(cudaFuncGetAttributes(&a, kernel));
+    if ((long long)bytes <= (long long)a.maxDynamicSharedSizeBytes - (long long)a.sharedSizeBytes) return YAMC_OK;
+    int device, optin;
+    CUDA_TRY(cudaGetDevice(&device));
+    CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  std::max((int)bytes, optin - (int)a.sharedSizeBytes)));
+    return YAMC_OK;
+}
 
 struct LaunchCfg {
     int G = 0, B = 0, EPT = 0;  // EPT: entries per worker in registers; 0 streamed; -1 streamed, wide CTAs
@@ -1922,7 +1942,7 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
 template <int NT, int EPT, bool SPLIT, bool MX>
 int launch_chain_t(const LaunchCfg &L, cudaStream_t stream, int nrep, const ChainArgs &args) {
     auto kfn = k_chain<NT, EPT, SPLIT, MX>;
-    CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
+    if (const int r = grant_smem(kfn, L.smem)) return r;
     if (L.G > 8) CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(L.G * nrep, 1, 1);
@@ -1944,7 +1964,7 @@ int launch_chain_t(const LaunchCfg &L, cudaStream_t stream, int nrep, const Chai
 template <int NT, int EPT, bool SPLIT, bool MX>
 int max_clusters_t(const LaunchCfg &L, int *out) {
     auto kfn = k_chain<NT, EPT, SPLIT, MX>;
-    CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
+    if (const int r = grant_smem(kfn, L.smem)) return r;
     if (L.G > 8) CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(L.G, 1, 1);

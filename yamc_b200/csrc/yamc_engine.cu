@@ -805,8 +805,8 @@ int pick_launch(yamc_ctx *c, LaunchCfg *out) {
 // the spatial staging order of every CTA of nrep chains (k_stage_order), ahead of their launch
 int launch_stage_order(const LaunchCfg &L, cudaStream_t stream, int nrep, const DevSys *d_sys) {
     const size_t smem = sizeof(int) * ((size_t)kStageMaxCells + L.nown_max);
-    if (smem > 48 * 1024)
-        CUDA_TRY(cudaFuncSetAttribute(k_stage_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024)  // (no static part)
+        if (const int r = grant_smem(k_stage_order, smem)) return r;
     k_stage_order<<<L.G * nrep, kStageThreads, smem, stream>>>(d_sys, L.G);
     CUDA_TRY(cudaGetLastError());
     return YAMC_OK;
@@ -869,8 +869,8 @@ int spatial_reset(const SpatialOrder &o, cudaStream_t stream) {
 int spatial_order(const SpatialOrder &o, const Points &P, cudaStream_t stream) {
     const int ncell = o.nc * o.nc * o.nc;
     const size_t smem = sizeof(int) * ((size_t)ncell + o.chunk);
-    if (smem > 48 * 1024)
-        CUDA_TRY(cudaFuncSetAttribute(k_sort_place, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024)  // (no static part)
+        if (const int r = grant_smem(k_sort_place, smem)) return r;
     k_sort_count<<<o.nblock, kSortThreads, 0, stream>>>(P, o.nc, o.chunk, o.hist, o.total);
     k_sort_scan<<<(ncell + 255) / 256, 256, 0, stream>>>(o.total, o.hist, o.nblock, ncell);
     k_sort_place<<<o.nblock, kSortThreads, smem, stream>>>(P, o.nc, o.chunk, o.hist, o.total, o.order);
@@ -901,7 +901,7 @@ AtomLists atom_lists(const yamc_ctx *c) {
 int launch_rho(yamc_ctx *c) {
     const HostSystem &H = c->H;
     const size_t sm = sizeof(double2) * (3 * (H.kmax + 1) + kRowZ) * (kRhoChunk + 1);
-    CUDA_TRY(cudaFuncSetAttribute(k_rho_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (const int r = grant_smem(k_rho_rows, sm)) return r;
     const dim3 grid((c->k_nitem + c->k_threads - 1) / c->k_threads, c->k_nslice);
     k_rho_rows<<<grid, c->k_threads, sm, c->stream>>>(c->hsys, atom_lists(c), c->k_slices, c->k_items, c->k_emap, c->k_nitem,
                                                       c->rho_part);
@@ -1136,14 +1136,14 @@ int launch_forces(yamc_ctx *c) {
     if (!c->d_field && ((r = dalloc(&c->d_gf, (size_t)3 * shares * H.N)) || (r = dalloc(&c->d_kf, (size_t)3 * nsplit * c->k_npos)) ||
                         (r = dalloc(&c->d_field, (size_t)2 * (1 + NT) * c->k_nf))))
         return r;
-    CUDA_TRY(cudaFuncSetAttribute(k_real_forces, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smr));
+    if ((r = grant_smem(k_real_forces, smr))) return r;
     k_real_forces<<<dim3(c->tiles.ntile, shares), 32 * kRealWarps, smr, c->stream>>>(
         c->hsys, c->tiles.order, c->tiles.box, c->tiles.ntile, tile_reach2(std::sqrt(c->hsys.rmax2)), c->d_gf);
     CUDA_TRY(cudaGetLastError());
     k_row_fields<NT><<<dim3((c->k_nf + 255) / 256, 1 + NT), 256, 0, c->stream>>>(c->hsys, c->k_fmap, c->k_nf, c->d_field);
     CUDA_TRY(cudaGetLastError());
     auto *rows = atoms == 2 ? k_forces_rows<2> : k_forces_rows<1>;
-    CUDA_TRY(cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if ((r = grant_smem(rows, sm))) return r;
     rows<<<dim3(nblk, nsplit), 32 * kForceRowWarps, sm, c->stream>>>(c->hsys, atom_lists(c), c->k_frows, c->k_nfrow, c->d_field,
                                                                      c->k_nf, c->k_npos, c->d_kf);
     CUDA_TRY(cudaGetLastError());
@@ -2007,13 +2007,13 @@ static int xchange_eval(yamc_ctx *c, int imol1, int imol2, double du[4], int *ov
     const size_t sm = sizeof(double2) * (size_t)(n1 + n2) * 2 * 3 * (H.kmax + 1);
     const int nbk = (H.S + 255) / 256;
     switch (H.nt) {
-        case 1: CUDA_TRY(cudaFuncSetAttribute(k_xchg_kspace<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        case 1: if (const int r = grant_smem(k_xchg_kspace<1>, sm)) return r;
                 k_xchg_kspace<1><<<nbk, 256, sm, c->stream>>>(c->hsys, in, c->scratch, c->part); break;
-        case 2: CUDA_TRY(cudaFuncSetAttribute(k_xchg_kspace<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        case 2: if (const int r = grant_smem(k_xchg_kspace<2>, sm)) return r;
                 k_xchg_kspace<2><<<nbk, 256, sm, c->stream>>>(c->hsys, in, c->scratch, c->part); break;
-        case 3: CUDA_TRY(cudaFuncSetAttribute(k_xchg_kspace<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        case 3: if (const int r = grant_smem(k_xchg_kspace<3>, sm)) return r;
                 k_xchg_kspace<3><<<nbk, 256, sm, c->stream>>>(c->hsys, in, c->scratch, c->part); break;
-        default: CUDA_TRY(cudaFuncSetAttribute(k_xchg_kspace<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        default: if (const int r = grant_smem(k_xchg_kspace<4>, sm)) return r;
                  k_xchg_kspace<4><<<nbk, 256, sm, c->stream>>>(c->hsys, in, c->scratch, c->part); break;
     }
     CUDA_TRY(cudaGetLastError());
@@ -2205,10 +2205,10 @@ static int rdf_create_impl(yamc_rdf *h, int32_t nmol, const int32_t *mol_type, i
     cudaDeviceProp prop;
     CUDA_TRY(cudaGetDeviceProperties(&prop, device));
     if (h->smem > prop.sharedMemPerBlockOptin) { set_error("too many RDF bins x species pairs for one block's histogram"); return YAMC_ELIMITS; }
-    CUDA_TRY(cudaFuncSetAttribute(k_rdf_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem));
+    if (const int r = grant_smem(k_rdf_count, h->smem)) return r;
     h->tile_path = nmol >= kRdfTileMin && h->smem + kRdfTileStatic <= prop.sharedMemPerBlockOptin;
     if (h->tile_path) {
-        CUDA_TRY(cudaFuncSetAttribute(k_rdf_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem));
+        if (const int r = grant_smem(k_rdf_tiles, h->smem)) return r;
         DeviceArena arena;
         spatial_plan(h->tiles, nmol, arena);
         if (const int r = arena.commit(&h->tiles.base)) return r;
