@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 def _water(n, directory, kmax=10):
     box = (n / 0.015) ** (1 / 3)
-    spec = systems.SystemSpec("water", n, 0, 0, box, 3.0 / 9.0, 9.0, kmax)
+    rc = min(9.0, 0.48 * box)
+    spec = systems.SystemSpec("water", n, 0, 0, box, 3.0 / rc, rc, kmax)
     f = systems.write_system(spec, directory, seed=3)
     return api.load_inputs(f["parameters"], f["composition"], f["moltab"])
 
@@ -33,3 +34,20 @@ def test_every_size_around_the_shared_memory_limit_runs(tmp_path, cluster, water
         seen.add(b.launch["cluster_blocks"])
         b.close()
     assert seen == {cluster, cluster + 1}
+
+
+@pytest.mark.parametrize("kmax", [108, 110, 112, 127])  # phase tables of 46, 47 and 48 KB, and the largest
+def test_per_move_calls_at_large_kmax(tmp_path, kmax):
+    """The per-move pass's tables beside its static shared memory, around the 48 KB that need no leave:
+    its energy change against that of the full sums, 1e-10 of the energies' scale."""
+    inp = _water(12, str(tmp_path), kmax)
+    eng = api.Engine(inp)
+    e0 = eng.energies()
+    eng.move_old(5)
+    a, b = inp.first_atom[4] - 1, inp.last_atom[4]
+    new = [v[a:b] + 0.004 for v in (inp.x, inp.y, inp.z)]
+    du, overlap, _, _ = eng.move_eval(5, *new)
+    assert not overlap
+    eng.move_commit(True)
+    assert np.all(np.abs(eng.energies() - eng.full_sums()) <= 1e-10 * np.abs(e0).max())
+    assert abs(du[1] - (eng.energies()[6] - e0[6])) <= 1e-10 * np.abs(e0).max()

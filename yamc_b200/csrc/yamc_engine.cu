@@ -749,7 +749,7 @@ bool is_mixed(const yamc_ctx *c) { return c->H.p.precision == YAMC_MIXED; }
 template <int NT, bool MX>
 int launch_move_pass_t(yamc_ctx *c, const MoveIn &in, bool eval, size_t smem) {
     auto kfn = eval ? k_move_pass<NT, MX, true> : k_move_pass<NT, MX, false>;
-    if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (const int r = grant_smem(kfn, smem)) return r;
     kfn<<<c->mblocks, kMoveThreads, smem, c->stream>>>(c->hsys, in, c->d_mpart, c->d_mcount, c->d_hout);
     CUDA_TRY(cudaGetLastError());
     return YAMC_OK;
