@@ -5,7 +5,7 @@ its full recomputation, 1e-9 relative."""
 import numpy as np
 import pytest
 
-from yamc_b200 import api, rng as grng, systems
+from yamc_b200 import _lib, api, rng as grng, systems
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +51,15 @@ def test_per_move_calls_at_large_kmax(tmp_path, kmax):
     eng.move_commit(True)
     assert np.all(np.abs(eng.energies() - eng.full_sums()) <= 1e-10 * np.abs(e0).max())
     assert abs(du[1] - (eng.energies()[6] - e0[6])) <= 1e-10 * np.abs(e0).max()
+
+
+def test_a_refused_call_leaves_no_error_behind(tmp_path):
+    """The runtime keeps the last error of a call until it is asked for: the calls after one that was
+    refused must not report it."""
+    inp = _water(12, str(tmp_path), 6)
+    ok = api.Engine(inp)
+    for _ in range(2):
+        with pytest.raises(_lib.YamcError):
+            api.Engine(inp, device=999)
+        assert np.array_equal(ok.set_positions(inp.x, inp.y, inp.z), ok.full_sums())
+        api.Engine(inp).close()

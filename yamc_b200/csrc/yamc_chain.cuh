@@ -18,6 +18,7 @@
     do {                                                                                      \
         cudaError_t _e = (expr);                                                              \
         if (_e != cudaSuccess) {                                                              \
+            (void)cudaGetLastError(); /* the next call must not meet it */                    \
             yamc::set_error(std::string(#expr) + ": " + cudaGetErrorString(_e));              \
             return YAMC_ECUDA;                                                                \
         }                                                                                     \

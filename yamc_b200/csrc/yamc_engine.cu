@@ -1270,6 +1270,7 @@ int batch_build_graph(yamc_batch *b) {
     const cudaError_t ee = cudaStreamEndCapture(b->stream, &graph);
     if (r) {
         if (graph) cudaGraphDestroy(graph);
+        (void)cudaGetLastError();
         if (r == YAMC_ECUDA) set_error("capturing the batch step failed");
         return r;
     }
@@ -1530,6 +1531,7 @@ int yamc_destroy(yamc_ctx *c) {
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
+    (void)cudaGetLastError();  // (what a half-made object could not give back)
     return YAMC_OK;
 }
 
@@ -2188,6 +2190,7 @@ int yamc_rdf_destroy(yamc_rdf *h) {
     if (h->tiles.base) cudaFree(h->tiles.base);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
+    (void)cudaGetLastError();  // (what a half-made object could not give back)
     return YAMC_OK;
 }
 
@@ -2640,6 +2643,7 @@ int yamc_batch_destroy(yamc_batch *b) {
     if (b->fork) cudaEventDestroy(b->fork);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
+    (void)cudaGetLastError();  // (what a half-made object could not give back)
     return YAMC_OK;
 }
 
