@@ -134,3 +134,19 @@ def test_rdf_handles_of_different_sizes_side_by_side(m):
         gpu[k].add_frame(x, y, z, 40.0)
         o.add_frame(x, y, z, 40.0)
         assert np.array_equal(gpu[k].result()[2] - before, o.cnt4.reshape(before.shape))
+
+
+@pytest.mark.gpu
+def test_rdf_of_a_frame_of_three_and_a_half_million_centres():
+    """More centres than 64 blocks of the sort hold: the known answer of the simple cubic lattice."""
+    from yamc_b200 import api
+    n = 152  # 1 A apart
+    x, y, z = _lattice(n)
+    M = x.size
+    gpu = api.RDF(np.ones(M, dtype=np.int32), np.array([M], dtype=np.int32), dr=0.19, rmax=1.9)
+    gpu.add_frame(x, y, z, float(n))
+    _, _, c, nf = gpu.result()
+    assert nf == 1
+    for r, k in ((1.0, 6), (np.sqrt(2.0), 12), (np.sqrt(3.0), 8)):
+        assert c[0, 0, int(r / 0.19)] == k * M
+    assert c.sum() == 26 * M

@@ -849,7 +849,7 @@ int launch_chain(yamc_ctx *c, const ChainArgs &args) {
 void spatial_plan(SpatialOrder &o, int n, DeviceArena &arena) {
     o.n = n;
     o.nc = sort_cells(n);
-    o.chunk = std::max(kSortChunk, (((n + kSortBlocks - 1) / kSortBlocks) + 31) / 32 * 32);
+    o.chunk = std::clamp((((n + kSortBlocks - 1) / kSortBlocks) + 31) / 32 * 32, kSortChunk, kSortMaxChunk);
     o.nblock = (n + o.chunk - 1) / o.chunk;
     o.ntile = (n + kTile - 1) / kTile;
     const size_t ncell = (size_t)o.nc * o.nc * o.nc;
@@ -869,8 +869,7 @@ int spatial_reset(const SpatialOrder &o, cudaStream_t stream) {
 int spatial_order(const SpatialOrder &o, const Points &P, cudaStream_t stream) {
     const int ncell = o.nc * o.nc * o.nc;
     const size_t smem = sizeof(int) * ((size_t)ncell + o.chunk);
-    if (smem > 48 * 1024)  // (no static part)
-        if (const int r = grant_smem(k_sort_place, smem)) return r;
+    static_assert(sizeof(int) * (kSortMaxCells + kSortMaxChunk) <= 48 * 1024, "k_sort_place's shared memory");
     k_sort_count<<<o.nblock, kSortThreads, 0, stream>>>(P, o.nc, o.chunk, o.hist, o.total);
     k_sort_scan<<<(ncell + 255) / 256, 256, 0, stream>>>(o.total, o.hist, o.nblock, ncell);
     k_sort_place<<<o.nblock, kSortThreads, smem, stream>>>(P, o.nc, o.chunk, o.hist, o.total, o.order);

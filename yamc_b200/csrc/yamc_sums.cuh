@@ -21,7 +21,10 @@ namespace yamc {
 // spatial order
 // ------------------------------------------------------------------------------------------
 constexpr int kTile = 32;          // points per tile: one warp's lanes
-constexpr int kSortChunk = 256;    // points per block of the counting sort, at least (at most kSortBlocks blocks)
+// Points per block of the counting sort: at least kSortChunk, and as many as make kSortBlocks blocks,
+// up to kSortMaxChunk, whose cells beside those of the grid fill the 48 KB that a block has without
+// asking (from there on there are more blocks).
+constexpr int kSortChunk = 256, kSortMaxChunk = 8192;
 constexpr int kSortBlocks = 64;
 constexpr int kSortMaxCells = 4096;
 constexpr int kSortThreads = 256;
