@@ -17,6 +17,7 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 
 from yamc_b200 import _lib, build
@@ -86,3 +87,34 @@ def test_checked_library_runs_chains_in_bounds():
     res = subprocess.run([sys.executable, "-c", f"ROOT = {ROOT!r}\n" + CHILD], env=env, capture_output=True,
                          text=True, timeout=600)
     assert res.returncode == 0 and "checked chains ok" in res.stdout, res.stdout[-2000:] + res.stderr[-4000:]
+
+
+CHILD_SUMS = r'''
+import sys, tempfile
+import numpy as np
+sys.path.insert(0, ROOT)
+from yamc_b200 import api, systems
+out = {}
+for n, ions in ((11, 0), (171, 1), (2400, 9)):  # a part of a tile, tiles and a rest, two atoms per lane of the force rows
+    with tempfile.TemporaryDirectory() as d:
+        box = ((n + 2 * ions) / 0.015) ** (1 / 3)
+        rc = min(9.0, 0.48 * box)
+        f = systems.write_system(systems.SystemSpec("s", n, ions, ions, box, 3.0 / rc, rc, 6), d, seed=n)
+        eng = api.Engine.from_files(f)
+        out[f"e{n}"] = eng.full_sums()
+        out[f"f{n}"] = eng.forces()[0]
+np.savez(OUT, **out)
+'''
+
+
+def test_checked_library_sums_in_bounds(tmp_path):
+    res = []
+    for lib in (build.LIB_CHECKED, build.LIB):
+        out = str(tmp_path / (os.path.basename(lib) + ".npz"))
+        run = subprocess.run([sys.executable, "-c", f"ROOT = {ROOT!r}\nOUT = {out!r}\n" + CHILD_SUMS],
+                             env=dict(os.environ, YAMC_LIBRARY=lib), capture_output=True, text=True, timeout=600)
+        assert run.returncode == 0, run.stdout[-2000:] + run.stderr[-4000:]
+        res.append(np.load(out))
+    for k in res[0].files:  # the same sums, to the rounding of differently contracted operations
+        scale = np.abs(res[1][k]).max()
+        assert np.all(np.abs(res[0][k] - res[1][k]) <= 1e-12 * scale), k

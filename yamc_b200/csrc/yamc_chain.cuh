@@ -962,7 +962,7 @@ __device__ __forceinline__ void real_part(const DevSys &D, ChainShared &sh, bool
                 bool near[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    jl[u] = i0 + u < nmine ? blocks[i0 + u] * kBlk + lane : nown;
+                    jl[u] = i0 + u < nmine ? blocks[YAMC_IX(i0 + u, kBlkList)] * kBlk + lane : nown;
                     const int j = jl[u] < nown ? jl[u] : 0;
                     const double4 pj = atom_s[YAMC_IX(j, nown)];
                     const double dx = min_image(qx - pj.x), dy = min_image(qy - pj.y), dz = min_image(qz - pj.z);
@@ -984,7 +984,7 @@ __device__ __forceinline__ void real_part(const DevSys &D, ChainShared &sh, bool
             do {
                 // slot tests of 32 gathered atoms
                 const bool valid = k0 + lane < nnear;
-                const int jl = valid ? nb[k0 + lane] : 0;
+                const int jl = valid ? nb[YAMC_IX(k0 + lane, kNear)] : 0;
                 const double4 pj = atom_s[YAMC_IX(jl, nown)];
                 const int tj = meta_s[YAMC_IX(jl, nown)].y;
                 // hard-core diameter: by LJ type when every atom of a type has the same one (a
@@ -1019,7 +1019,7 @@ __device__ __forceinline__ void real_part(const DevSys &D, ChainShared &sh, bool
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
                         const int q = q0 + 32 * u;
-                        const int item = queue[q < n ? q : q0];
+                        const int item = queue[YAMC_IX(q < n ? q : q0, kPairs)];
                         const int ji = item & 8191, s = item >> 13;
                         const Slot &sl = m.slot[s];
                         const double4 pi = atom_s[YAMC_IX(ji, nown)];
@@ -1051,7 +1051,8 @@ __device__ __forceinline__ void real_part(const DevSys &D, ChainShared &sh, bool
                 }
                 if (n > 0) {
                     __syncwarp();
-                    const unsigned short r0 = n + lane < npair ? queue[n + lane] : 0, r1 = n + 32 + lane < npair ? queue[n + 32 + lane] : 0;
+                    const unsigned short r0 = n + lane < npair ? queue[YAMC_IX(n + lane, kPairs)] : 0,
+                                         r1 = n + 32 + lane < npair ? queue[YAMC_IX(n + 32 + lane, kPairs)] : 0;
                     __syncwarp();
                     queue[lane] = r0; queue[32 + lane] = r1;
                     npair -= n;

@@ -52,7 +52,8 @@ struct DevSys {
 
 // Bounds-checked builds (-DYAMC_CHECKED, libyamc_b200_checked.so): YAMC_IX(i, n) checks every
 // index the chain kernel computes into its atom, staging, k-entry, scratch, pair-queue, near-atom
-// and table arrays.  An index outside [0, n) records the source line in *D.check (the first one
+// and near-block arrays, and those of the whole-configuration sums of a context into their orders,
+// lists, queues, entry maps and fields.  An index outside [0, n) records the source line in *D.check (the first one
 // wins) and is replaced by 0, so the access stays inside the array: no trap, no fault; the host
 // returns YAMC_EBOUNDS after the launch.  In normal builds YAMC_IX(i, n) is i.
 __device__ __forceinline__ long long checked_ix(long long i, long long n, int line, int *check) {
@@ -61,8 +62,10 @@ __device__ __forceinline__ long long checked_ix(long long i, long long n, int li
     return 0;
 }
 #ifdef YAMC_CHECKED
-#define YAMC_IX(i, n) ::yamc::checked_ix((long long)(i), (long long)(n), __LINE__, D.check)
+#define YAMC_IXC(i, n, check) ::yamc::checked_ix((long long)(i), (long long)(n), __LINE__, check)
+#define YAMC_IX(i, n) YAMC_IXC(i, n, D.check)
 #else
+#define YAMC_IXC(i, n, check) (i)
 #define YAMC_IX(i, n) (i)
 #endif
 

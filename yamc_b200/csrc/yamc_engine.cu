@@ -1039,6 +1039,25 @@ int pull_state(yamc_ctx *c) {
     return YAMC_OK;
 }
 
+// Bounds-checked builds: the index check word of a context after its kernels ran (YAMC_EBOUNDS
+// with the source line when an index was out of bounds; the word is cleared).  Normal builds
+// compile the checks out and return `status`.
+int bounds_status(yamc_ctx *c, int status) {
+#ifdef YAMC_CHECKED
+    int line = 0;
+    CUDA_TRY(cudaMemcpyAsync(&line, c->d_check, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if (line) {
+        CUDA_TRY(cudaMemsetAsync(c->d_check, 0, sizeof(int), c->stream));
+        set_error("index out of bounds in a kernel, at line " + std::to_string(line) + " of yamc_chain.cuh or yamc_sums.cuh");
+        return YAMC_EBOUNDS;
+    }
+#else
+    (void)c;
+#endif
+    return status;
+}
+
 // what a chain's run slot brings back
 void take_state(yamc_ctx *c, const RunSlot &rs) {
     std::copy(rs.sc, rs.sc + SC_COUNT, c->sc);
@@ -1089,6 +1108,7 @@ int full_sums(yamc_ctx *c, int *overlap = nullptr) {
     double ek[2];
     CUDA_TRY(cudaMemcpyAsync(ek, c->sums + kFullParts, sizeof(ek), cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if ((r = bounds_status(c, YAMC_OK))) return r;
     const double ekc = ek[0], ekl = ek[1];
     if (!std::isfinite(ekc) || !std::isfinite(ekl)) { set_error("non-finite k-space sum"); return YAMC_ENAN; }
     // EwaldSumExternal_calc_mu over all atoms, in atom order (EwaldSumExternal.f90:34-52)
@@ -1281,25 +1301,6 @@ int batch_build_graph(yamc_batch *b) {
 }
 
 // one step of every replica: replica i's stream holds positions [rng_off[i], n_rng[i]) at rng[i]
-// Bounds-checked builds: the index check word of a context after its kernels ran (YAMC_EBOUNDS
-// with the source line when an index was out of bounds; the word is cleared).  Normal builds
-// compile the checks out and return `status`.
-static int bounds_status(yamc_ctx *c, int status) {
-#ifdef YAMC_CHECKED
-    int line = 0;
-    CUDA_TRY(cudaMemcpyAsync(&line, c->d_check, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CUDA_TRY(cudaStreamSynchronize(c->stream));
-    if (line) {
-        CUDA_TRY(cudaMemsetAsync(c->d_check, 0, sizeof(int), c->stream));
-        set_error("index out of bounds in the chain kernel at yamc_chain.cuh line " + std::to_string(line));
-        return YAMC_EBOUNDS;
-    }
-#else
-    (void)c;
-#endif
-    return status;
-}
-
 int batch_step(yamc_batch *b, const float *const *rng, const int64_t *rng_off, const int64_t *n_rng,
                int64_t *cursors, int64_t n_moves, int64_t *moves_done, int32_t *status, yamc_move_record *d_log,
                int only_group = -1) {
@@ -2972,6 +2973,7 @@ int yamc_forces(yamc_ctx *c, double *fx, double *fy, double *fz, double *mol_f, 
     }
     if (r) return r;
     CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if ((r = bounds_status(c, YAMC_OK))) return r;
     double *gx = c->h_pos, *gy = gx + N, *gz = gy + N;  // (k_forces_add writes to the mapped pinned memory)
     // external term: F = -2 kext q mu (EwaldSumExternal.f90:84-102)
     const double mx = c->sc[SC_MU_X], my = c->sc[SC_MU_Y], mz = c->sc[SC_MU_Z], m2k = H.p.minus_two_kext;

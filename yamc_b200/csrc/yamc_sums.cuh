@@ -171,13 +171,13 @@ __device__ __forceinline__ bool boxes_near(float4 ca, float4 ha, float4 cb, floa
 }
 
 // The near tiles of tile ti among [base, base + kNearSpan), in increasing order, into list (shared);
-// returns their number.  All threads of a block of NW warps; HALF: each unordered pair of tiles
+// returns their number (check: the index check word, or null).  All threads of a block of NW warps; HALF: each unordered pair of tiles
 // belongs to one of the two (by the parity of their sum, so the tiles' shares are even), the tile
 // itself included.
 constexpr int kNearSpan = 1024;
 template <bool HALF, int NW>
 __device__ __forceinline__ int near_tiles(const float4 *box, int ntile, int ti, int base, double r2, unsigned *words, int *list,
-                                          int *count) {
+                                          int *count, int *check) {
     const float4 c = box[2 * ti], h = box[2 * ti + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -199,7 +199,7 @@ __device__ __forceinline__ int near_tiles(const float4 *box, int ntile, int ti, 
             const int y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
         }
-        for (int at = x - n; b; b &= b - 1) list[at++] = base + lane * 32 + __ffs(b) - 1;
+        for (int at = x - n; b; b &= b - 1, ++at) list[YAMC_IXC(at, kNearSpan, check)] = base + lane * 32 + __ffs(b) - 1;
         if (lane == 31) *count = x;
     }
     __syncthreads();
@@ -260,7 +260,7 @@ __device__ __forceinline__ unsigned candidates(float3 a, const float3 *b, int n,
 
 // The lanes' candidates one after the other in the warp's queue (lane << 5 | j, in lane order):
 // returns their number; *at: where the lane's own begin.
-__device__ __forceinline__ int queue_pairs(unsigned mask, unsigned short *queue, int *at) {
+__device__ __forceinline__ int queue_pairs(unsigned mask, unsigned short *queue, int *at, int *check) {
     const int lane = threadIdx.x & 31, n = __popc(mask);
     int x = n;
 #pragma unroll
@@ -269,7 +269,7 @@ __device__ __forceinline__ int queue_pairs(unsigned mask, unsigned short *queue,
         if (lane >= o) x += y;
     }
     *at = x - n;
-    for (int k = x - n; mask; mask &= mask - 1) queue[k++] = (unsigned short)(lane << 5 | (__ffs(mask) - 1));
+    for (int k = x - n; mask; mask &= mask - 1, ++k) queue[YAMC_IXC(k, kTile * kTile, check)] = (unsigned short)(lane << 5 | (__ffs(mask) - 1));
     return __shfl_sync(0xffffffffu, x, 31);
 }
 
@@ -296,7 +296,7 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_energy(DevSys D
     const int ti = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ni = min(kTile, D.N - ti * kTile);
     if (warp == 0 && lane < ni) {
-        const int i = order[ti * kTile + lane];
+        const int i = (int)YAMC_IX(order[YAMC_IX(ti * kTile + lane, D.N)], D.N);
         ai[lane] = tile_atom(D, i, D.atom[i]);
     }
     __syncthreads();
@@ -307,9 +307,9 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_energy(DevSys D
     bool ovl = false;
     const int nt = D.nt;
     for (int base = 0; base < ntile; base += kNearSpan) {
-        const int near = near_tiles<true, kRealWarps>(box, ntile, ti, base, reach2, words, list, &count);
+        const int near = near_tiles<true, kRealWarps>(box, ntile, ti, base, reach2, words, list, &count, D.check);
         for (int m = blockIdx.y * kRealWarps + warp; m < near; m += gridDim.y * kRealWarps) {
-            const int tj = list[m], ij = order[min(tj * kTile + lane, D.N - 1)];
+            const int tj = list[YAMC_IX(m, kNearSpan)], ij = (int)YAMC_IX(order[YAMC_IX(min(tj * kTile + lane, D.N - 1), D.N)], D.N);
             const double4 v = D.atom[ij];
             const float3 f = tile_point(v.x, v.y, v.z);
             const bool in_reach = tj * kTile + lane < D.N && near_point(f, boxc, boxh, limit);
@@ -325,10 +325,11 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_energy(DevSys D
             if (tj == ti) mask &= lane < 31 ? ~((2u << lane) - 1u) : 0u;  // (each pair of the tile itself once)
             if (lane >= ni) mask = 0;
             int at;
-            const int total = queue_pairs(mask, queue[warp], &at);
+            const int total = queue_pairs(mask, queue[warp], &at, D.check);
             __syncwarp();
             for (int q = lane; q < total; q += 32) {
-                const TileAtom &a = ai[queue[warp][q] >> 5], &b = aj[warp][queue[warp][q] & 31];
+                const int pair = queue[warp][YAMC_IX(q, kTile * kTile)];
+                const TileAtom &a = ai[pair >> 5], &b = aj[warp][pair & 31];
                 const double dx = min_image(a.x - b.x), dy = min_image(a.y - b.y), dz = min_image(a.z - b.z);
                 const double r2 = dx * dx + dy * dy + dz * dz;
                 const bool lj = a.type > 0 && b.type > 0, same = a.mol == b.mol;
@@ -378,7 +379,7 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_forces(DevSys D
     const int ti = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ni = min(kTile, D.N - ti * kTile);
     if (warp == 0 && lane < ni) {
-        const int i = order[ti * kTile + lane];
+        const int i = (int)YAMC_IX(order[YAMC_IX(ti * kTile + lane, D.N)], D.N);
         ai[lane] = tile_atom(D, i, D.atom[i]);
     }
     __syncthreads();
@@ -389,9 +390,9 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_forces(DevSys D
     double gx = 0, gy = 0, gz = 0;
     const int nt = D.nt;
     for (int base = 0; base < ntile; base += kNearSpan) {
-        const int near = near_tiles<false, kRealWarps>(box, ntile, ti, base, reach2, words, list, &count);
+        const int near = near_tiles<false, kRealWarps>(box, ntile, ti, base, reach2, words, list, &count, D.check);
         for (int m = blockIdx.y * kRealWarps + warp; m < near; m += gridDim.y * kRealWarps) {
-            const int tj = list[m], ij = order[min(tj * kTile + lane, D.N - 1)];
+            const int tj = list[YAMC_IX(m, kNearSpan)], ij = (int)YAMC_IX(order[YAMC_IX(min(tj * kTile + lane, D.N - 1), D.N)], D.N);
             const double4 v = D.atom[ij];
             const float3 f = tile_point(v.x, v.y, v.z);
             const bool in_reach = tj * kTile + lane < D.N && near_point(f, boxc, boxh, limit);
@@ -407,12 +408,13 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_forces(DevSys D
             if (tj == ti) mask &= ~(1u << lane);
             if (lane >= ni) mask = 0;
             int at;
-            const int mine = __popc(mask), total = queue_pairs(mask, queue[warp], &at);
+            const int mine = __popc(mask), total = queue_pairs(mask, queue[warp], &at, D.check);
             __syncwarp();
             for (int q0 = 0; q0 < total; q0 += kForceBatch) {
                 const int q1 = min(total, q0 + kForceBatch);
                 for (int q = q0 + lane; q < q1; q += 32) {
-                    const TileAtom &a = ai[queue[warp][q] >> 5], &b = aj[warp][queue[warp][q] & 31];
+                    const int pair = queue[warp][YAMC_IX(q, kTile * kTile)];
+                    const TileAtom &a = ai[pair >> 5], &b = aj[warp][pair & 31];
                     const double dx = min_image(a.x - b.x), dy = min_image(a.y - b.y), dz = min_image(a.z - b.z);
                     const double r2 = dx * dx + dy * dy + dz * dz;
                     double FR = 0.0;
@@ -437,7 +439,7 @@ static __global__ void __launch_bounds__(32 * kRealWarps) k_real_forces(DevSys D
     if (warp < 3 && lane < ni) {
         double x = 0;
         for (int w = 0; w < kRealWarps; ++w) x += batch[((size_t)w * 3 + warp) * kForceBatch + lane];
-        gf[((size_t)blockIdx.y * 3 + warp) * D.N + order[ti * kTile + lane]] = x;
+        gf[((size_t)blockIdx.y * 3 + warp) * D.N + YAMC_IX(order[YAMC_IX(ti * kTile + lane, D.N)], D.N)] = x;
     }
 }
 
@@ -485,9 +487,9 @@ static __global__ void __launch_bounds__(kRhoMaxThreads) k_rho_rows(DevSys D, At
     for (int j = 0; j < kRowZ; ++j) cc[j] = ss[j] = sc[j] = cs[j] = make_double2(0.0, 0.0);
     // (the next chunk's atoms are on their way while this one is summed)
     auto fetch = [&](int p) {
-        const int i = p < sl.z ? L.alist[p] : -1;
+        const int i = p < sl.z ? L.alist[YAMC_IX(p, L.lbeg[kMaxLists])] : -1;
         double4 v = make_double4(0.0, 0.0, 0.0, 0.0);
-        if (i >= 0) { v = D.atom[i]; if (sl.x > 0) v.w = 1.0; }
+        if (i >= 0) { v = D.atom[YAMC_IX(i, D.N)]; if (sl.x > 0) v.w = 1.0; }
         return v;
     };
     for (int k = threadIdx.x; k < kRowZ * P; k += blockDim.x) rtab[3 * KM * P + k] = make_double2(0.0, 0.0);
@@ -545,8 +547,8 @@ static __global__ void __launch_bounds__(kRhoMaxThreads) k_rho_rows(DevSys D, At
                 const double rc = y ? cc[j].x + ss[j].x : cc[j].x - ss[j].x, is = y ? sc[j].y - cs[j].y : sc[j].y + cs[j].y;
                 const double rs = y ? cc[j].y + ss[j].y : cc[j].y - ss[j].y, ic = y ? sc[j].x - cs[j].x : sc[j].x + cs[j].x;
                 const int ep = y ? e.z : e.x, em = y ? e.w : e.y;
-                if (ep >= 0) out[ep] = make_double2(rc - is, rs + ic);
-                if (em >= 0) out[em] = make_double2(rc + is, ic - rs);
+                if (ep >= 0) out[YAMC_IX(ep, D.S)] = make_double2(rc - is, rs + ic);
+                if (em >= 0) out[YAMC_IX(em, D.S)] = make_double2(rc + is, ic - rs);
             }
         }
     }
@@ -583,12 +585,13 @@ static __global__ void __launch_bounds__(256) k_row_fields(DevSys D, const int4 
     const int f = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y;
     if (f >= nf) return;
     const int4 m = fmap[f];
-    const int e[4] = {m.x, m.y, m.z, m.w};
+    int e[4] = {m.x, m.y, m.z, m.w};
     double2 g[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         g[k] = make_double2(0.0, 0.0);
         if (e[k] < 0) continue;
+        e[k] = (int)YAMC_IX(e[k], D.S);
         if (l == 0) {
             const double2 r = D.rho[e[k]];
             const double b = D.ebeta[e[k]];
@@ -633,10 +636,10 @@ static __global__ void __launch_bounds__(32 * kForceRowWarps) k_forces_rows(DevS
     const int p0 = L.lbeg[l] + W * b, pe = L.lbeg[l + 1];
     const double4 *F = field + (size_t)l * nf * 2;
     for (int idx = threadIdx.x; idx < W * 3 * KM; idx += blockDim.x) {
-        const int r = idx / W, d = r / KM, m = r % KM, p = p0 + idx % W, i = p < pe ? L.alist[p] : -1;
+        const int r = idx / W, d = r / KM, m = r % KM, p = p0 + idx % W, i = p < pe ? L.alist[YAMC_IX(p, L.lbeg[kMaxLists])] : -1;
         double s = 0.0, c = 0.0;
         if (i >= 0) {
-            const double4 v = D.atom[i];
+            const double4 v = D.atom[YAMC_IX(i, D.N)];
             const double u = d == 0 ? v.x : (d == 1 ? v.y : v.z);
             sincospi(2.0 * (double)m * u, &s, &c);
             if (m == 0) { s = 0.0; c = 1.0; }
@@ -648,7 +651,7 @@ static __global__ void __launch_bounds__(32 * kForceRowWarps) k_forces_rows(DevS
     for (int r = blockIdx.y * kForceRowWarps + warp; r < nrow; r += gridDim.y * kForceRowWarps) {
         const int4 row = rows[r];
         const double2 *tz = ftab + 2 * KM * W + lane;
-        const double4 *f = F + 2 * (size_t)row.z;
+        const double4 *f = F + 2 * (size_t)YAMC_IX(row.z, nf - row.w + 1);
         double r1[A][2] = {}, r2[A][2] = {}, z1[A][2] = {}, z2[A][2] = {};
 #pragma unroll (4 / A)
         for (int k = 0; k < row.w; ++k) {
@@ -716,8 +719,8 @@ static __global__ void k_forces_add(DevSys D, const int2 *place, const double *g
         for (int s = 0; s < nreal; ++s) g += gf[((size_t)s * 3 + c) * D.N + i];
         for (int s = 0; s < nsplit; ++s) {
             const double *v = kf + ((size_t)s * 3 + c) * npos;
-            if (p.x >= 0) a += v[p.x];
-            if (p.y >= 0) b += v[p.y];
+            if (p.x >= 0) a += v[YAMC_IX(p.x, npos)];
+            if (p.y >= 0) b += v[YAMC_IX(p.y, npos)];
         }
         f[(size_t)c * D.N + i] = g + kFourPi * (q * a + b);
     }
@@ -755,7 +758,7 @@ static __global__ void __launch_bounds__(256) k_rdf_tiles(const double *cx, cons
         const float4 boxc = box[2 * ti], boxh = box[2 * ti + 1];
         const float3 own = tile_point(ci[lane].x, ci[lane].y, ci[lane].z);
         for (int base = 0; base < ntile; base += kNearSpan) {
-            const int near = near_tiles<false, 8>(box, ntile, ti, base, reach2, words, list, &count);
+            const int near = near_tiles<false, 8>(box, ntile, ti, base, reach2, words, list, &count, nullptr);
             for (int m = blockIdx.y * 8 + warp; m < near; m += gridDim.y * 8) {
                 const int tj = list[m];
                 const double4 p = centre(tj * kTile + lane);
@@ -773,7 +776,7 @@ static __global__ void __launch_bounds__(256) k_rdf_tiles(const double *cx, cons
                 if (tj == ti) mask &= ~(1u << lane);
                 if (lane >= ni) mask = 0;
                 int at;
-                const int total = queue_pairs(mask, queue[warp], &at);
+                const int total = queue_pairs(mask, queue[warp], &at, nullptr);
                 __syncwarp();
                 for (int q = lane; q < total; q += 32) {
                     const double4 a = ci[queue[warp][q] >> 5], b = cj[warp][queue[warp][q] & 31];
