@@ -314,18 +314,6 @@ struct ChainShared {
     int wnext;
 };
 
-// All static shared memory of the chain kernel: one object, so the host that plans the dynamic part
-// (pick_launch_for) knows its size.
-struct __align__(16) ChainStatic {
-    ChainShared sh;
-    float rwin[2][kWin];  // the windows of the random stream
-    // the system's parameters and array pointers: every thread reads them from here (a per-thread
-    // copy would live in local memory, which the staged atoms leave little L1 for)
-    DevSys sys;
-    // phase cycles (a counter in global memory costs a round trip per mark)
-    long long prof[PH_COUNT];
-};
-
 // why a chain stops before its last move (ChainShared::abort)
 constexpr int kAbortStream = 1;     // the random stream ran out (YAMC_ERNG_EXHAUSTED, resumable)
 constexpr int kAbortNonFinite = 2;  // a non-finite energy change or bias force (YAMC_ENAN)
@@ -1388,26 +1376,35 @@ __device__ __noinline__ void refresh_in_chain(const DevSys &D, double2 *scr, int
     __syncthreads();
 }
 
+// The static shared memory of k_chain: its __shared__ variables, each on its own 16 bytes.  (As members of
+// one object, whose size would say it without this list, they cost the FP64 streamed variant 5 % of its
+// time in spills: nacl1m on 3 x 256 threads 21.5 -> 22.5 us a move.)
+constexpr size_t pad16(size_t bytes) { return (bytes + 15) / 16 * 16; }
+constexpr size_t kChainStaticBytes = pad16(sizeof(ChainShared)) + pad16(sizeof(float) * 2 * kWin) + pad16(sizeof(DevSys)) +
+                                     pad16(sizeof(long long) * PH_COUNT);
+
 // SPLIT = false: unbiased device-resident chain only (one fused pass per move, speculation);
 // SPLIT = true: force-biased moves (old pass + new pass with forces).
 template <int NT, int EPT, bool SPLIT, bool MX>
 __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThreads, 1) k_chain(ChainArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ ChainStatic st;
-    ChainShared &sh = st.sh;
-    float(&rwin)[2][kWin] = st.rwin;
+    __shared__ ChainShared sh;
+    __shared__ float rwin[2][kWin];
 
     cg::cluster_group cluster = cg::this_cluster();
     const int G = A.G;
     const int rank = G > 1 ? (int)cluster.block_rank() : 0;
     const int rep = blockIdx.x / G;
+    // the system's parameters and array pointers in shared memory: every thread reads them from
+    // there (a per-thread copy would live in local memory, which the staged atoms leave little L1 for)
+    __shared__ DevSys D_s;
     {
         const int *src = reinterpret_cast<const int *>(A.sys + rep);
-        int *dst = reinterpret_cast<int *>(&st.sys);
+        int *dst = reinterpret_cast<int *>(&D_s);
         for (int i = threadIdx.x; i < (int)(sizeof(DevSys) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
         __syncthreads();
     }
-    const DevSys &D = st.sys;
+    const DevSys &D = D_s;
     RunSlot *run = A.run + rep;
     const int B = blockDim.x;
     const int tid = threadIdx.x;
@@ -1523,8 +1520,10 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
     const long long refresh_every = MX ? D.refresh_every : 0;
     int xpar = 0;  // parity of the cluster exchange buffer, flipped after every pass
     const long long n_moves = run->n_moves;
-    long long *prof = (A.prof && rank == 0) ? st.prof : nullptr;
-    if (prof && tid < PH_COUNT) prof[tid] = 0;
+    // phase cycles are counted in shared memory (a counter in global memory costs a round trip per mark)
+    __shared__ long long prof_s[PH_COUNT];
+    long long *prof = (A.prof && rank == 0) ? prof_s : nullptr;
+    if (prof && tid < PH_COUNT) prof_s[tid] = 0;
     if (prof) __syncthreads();
     const bool pc = prof && tid == 0;
     long long t_mark = 0;
@@ -1914,7 +1913,7 @@ __global__ void __launch_bounds__(EPT < 0 ? kChainMaxThreadsWide : kChainMaxThre
 
     if (prof) {
         __syncthreads();
-        if (tid < PH_COUNT) A.prof[tid] += prof[tid];
+        if (tid < PH_COUNT) A.prof[tid] += prof_s[tid];
     }
     {  // write back the register and shared state
 #pragma unroll

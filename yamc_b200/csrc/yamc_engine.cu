@@ -707,7 +707,7 @@ int pick_launch_for(const std::vector<const HostSystem *> &hosts, int device, in
     cudaDeviceProp prop;
     CUDA_TRY(cudaGetDeviceProperties(&prop, device));
     // what the kernel's static shared memory leaves of a block's
-    const size_t smem_max = prop.sharedMemPerBlockOptin - sizeof(ChainStatic);
+    const size_t smem_max = prop.sharedMemPerBlockOptin - kChainStaticBytes;
     int Smax = 0, Nmax = 0, Nmin = 1 << 30, kmax = 0, nt = 0;
     for (const HostSystem *h : hosts) {
         Smax = std::max(Smax, h->S); Nmax = std::max(Nmax, h->N); Nmin = std::min(Nmin, h->N);
