@@ -1297,6 +1297,12 @@ __device__ __noinline__ void refresh_in_chain(const DevSys &D, double2 *scr, int
 #pragma unroll
             for (int t = 0; t <= NT; ++t) acc[j][t] = make_double2(0.0, 0.0);
         }
+        // the entries of the batch that the warp has: its first lane's (a lane's one past its last has
+        // k = 0, and its sums go nowhere)
+        int nent = 0;
+#pragma unroll
+        for (int j = 0; j < EB; ++j) nent += ent[j] >= 0;
+        nent = __shfl_sync(0xffffffffu, nent, 0);
         for (int a0 = 0; a0 < N; a0 += CH) {
             const int na = min(CH, N - a0);
             for (int idx = tid; idx < na * 3 * KM; idx += B) {
@@ -1311,28 +1317,49 @@ __device__ __noinline__ void refresh_in_chain(const DevSys &D, double2 *scr, int
             for (int a = tid; a < na; a += B) { sq[a] = D.atom[a0 + a].w; st[a] = D.meta[a0 + a].y; }
             __syncthreads();
             if (!ctl) {
-                for (int a = 0; a < na; ++a) {
-                    const double2 *T = tabs + (size_t)a * 3 * KM;
-                    const double q = sq[a];
-                    const int ty = st[a];
+                // Two entries side by side, with no branch between them or before their phases: latency binds
+                // (7 or 11 worker warps a CTA).  A branch per entry and atom took 10.3 ms a refresh of 12,440
+                // atoms on 16 CTAs and 137 ms of 49,752, this 7.8 and 100; four side by side 5.6 and 77, but
+                // their registers cost every move of the streamed mixed form up to 8 %.
+                auto sum = [&](auto jc, auto nc) {
+                    constexpr int j0 = decltype(jc)::value, n = decltype(nc)::value;
+#pragma unroll 1
+                    for (int a = 0; a < na; ++a) {
+                        const double2 *T = tabs + (size_t)a * 3 * KM;
+                        const double q = sq[a], w = q != 0.0 ? q : 1.0;
+                        const int ty = st[a];
+                        double c[n], s[n];
 #pragma unroll
-                    for (int j = 0; j < EB; ++j) {
-                        if (ent[j] < 0) continue;
-                        double c = 0, s = 0;
+                        for (int j = 0; j < n; ++j)
+                            entry_phase<double, double2>(T, T + KM, T + 2 * KM, kv[j0 + j].x, kv[j0 + j].y, kv[j0 + j].z, w,
+                                                         c[j], s[j]);
                         if (q != 0.0) {
-                            entry_phase<double, double2>(T, T + KM, T + 2 * KM, kv[j].x, kv[j].y, kv[j].z, q, c, s);
-                            acc[j][0].x = acc[j][0].x + c; acc[j][0].y = acc[j][0].y + s;
+#pragma unroll
+                            for (int j = 0; j < n; ++j) {
+                                double2 &A = acc[j0 + j][0];
+                                A.x = A.x + c[j]; A.y = A.y + s[j];
+                            }
                         }
                         if (ty > 0) {
-                            double cl, sl;
-                            if (q != 0.0) { const double iq = 1.0 / q; cl = c * iq; sl = s * iq; }
-                            else entry_phase<double, double2>(T, T + KM, T + 2 * KM, kv[j].x, kv[j].y, kv[j].z, 1.0, cl, sl);
+                            const double iw = 1.0 / w;
 #pragma unroll
                             for (int t = 0; t < NT; ++t)
-                                if (t == ty - 1) { acc[j][1 + t].x = acc[j][1 + t].x + cl; acc[j][1 + t].y = acc[j][1 + t].y + sl; }
+                                if (t == ty - 1) {
+#pragma unroll
+                                    for (int j = 0; j < n; ++j) {
+                                        double2 &A = acc[j0 + j][1 + t];
+                                        A.x = A.x + c[j] * iw; A.y = A.y + s[j] * iw;
+                                    }
+                                }
                         }
                     }
-                }
+                };
+                static_for<0, (EB + 1) / 2>([&](auto hc) {
+                    constexpr int j0 = 2 * decltype(hc)::value;
+                    if (nent == j0 + 1) sum(IntC<j0>{}, IntC<1>{});
+                    if constexpr (j0 + 1 < EB)
+                        if (nent > j0 + 1) sum(IntC<j0>{}, IntC<2>{});
+                });
             }
             __syncthreads();
         }
