@@ -115,3 +115,24 @@ def test_rdf_tiles_count_as_all_pairs(m, box):
     _, _, c, n = g.result()
     assert n == 1 and np.array_equal(c.ravel(), np.asarray(o.cnt4).ravel())
     assert c.sum() > 0 and math.isfinite(c.sum())
+
+
+# remainders of a tile of 1, 31 and 0 above both thresholds of the tiles, and more tiles than one span of
+# the near lists takes (1024)
+@pytest.mark.parametrize("m,box", [(2401, 40.0), (2431, 40.0), (2432, 40.0), (3617, 31.0), (3647, 31.0), (3648, 31.0), (33001, 60.0)])
+def test_rdf_tiles_count_as_all_pairs_at_their_edges(m, box):
+    test_rdf_tiles_count_as_all_pairs(m, box)
+
+
+def test_forces_over_more_than_one_span_of_tiles(nacl16k_files):
+    """49,752 atoms, 1,555 tiles: against the oracle's forces as in the test above (2e-4 of the force
+    scale), and the sum of all real-space and k-space pair forces, which is 0 but for rounding: 1e-9 of
+    the sum of magnitudes (the sums of 1e5 terms of an atom are good to 1e-12 of theirs)."""
+    inp = api.load_inputs(nacl16k_files["parameters"], nacl16k_files["composition"], nacl16k_files["moltab"])
+    eng = api.Engine(inp)
+    f, mf, _ = eng.forces()
+    scale = math.sqrt((mf ** 2).sum(1).mean())
+    o = pyoracle.Oracle(nacl16k_files)
+    for imol in (1, 5461, 12000, 16384, 16385, 16684, 16984):
+        assert np.all(np.abs(o.move_old(imol)[0] - mf[imol - 1]) <= 2e-4 * scale)
+    assert np.all(np.abs(f.sum(0)) <= 1e-9 * np.abs(f).sum(0))
