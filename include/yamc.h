@@ -47,9 +47,9 @@ extern "C" {
 #define YAMC_ENAN (-13)
 #define YAMC_EOVERLAP_INIT (-14)
 /* YAMC_EBOUNDS: bounds-checked builds only (libyamc_b200_checked.so, compiled with
-   -DYAMC_CHECKED): an index the chain kernel computed fell outside its array.  The kernel
-   replaced it by 0 (no fault) and the call returns this code; yamc_last_error_detail names the
-   source line.  The state of the context is then unreliable. */
+   -DYAMC_CHECKED): an index that the chain kernel or the whole-configuration sums computed fell
+   outside its array.  The kernel replaced it by 0 (no fault) and the call returns this code;
+   yamc_last_error_detail names the source line.  The state of the context is then unreliable. */
 #define YAMC_EBOUNDS (-15)
 
 /* precision of the device arithmetic */
@@ -288,7 +288,8 @@ int yamc_rdf_create(int32_t nmol, const int32_t *mol_type, int32_t ntypes, const
                     double dr, double rmax, int32_t device, yamc_rdf **out);
 int yamc_rdf_destroy(yamc_rdf *h);
 int yamc_rdf_nbin(yamc_rdf *h, int32_t *nbin);
-/* centres in box units (HOST arrays, nmol each), box length in Angstrom */
+/* centres in box units (HOST arrays, nmol each), box length in Angstrom; a centre with a coordinate that
+   is not finite is in no pair */
 int yamc_rdf_add_frame(yamc_rdf *h, const double *x, const double *y, const double *z, double box_length);
 /* the context's current configuration: centres of mass (center_of_mass, geometry.f90:170-201)
    computed on the device from its positions; the context must be on the RDF's device */

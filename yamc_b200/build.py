@@ -3,8 +3,8 @@
 ``python -m yamc_b200.build`` compiles ``csrc/`` into ``yamc_b200/libyamc_b200.so``
 in-tree, so the shared object travels with the source tree; ``--checked`` builds the
 bounds-checked variant ``yamc_b200/libyamc_b200_checked.so`` (``-DYAMC_CHECKED``: every index the
-chain kernel computes is checked, an out-of-bounds one is recorded and replaced by 0, and the call
-returns YAMC_EBOUNDS).
+chain kernel and the whole-configuration sums compute is checked, an out-of-bounds one is recorded and
+replaced by 0, and the call returns YAMC_EBOUNDS).
 """
 from __future__ import annotations
 

@@ -65,10 +65,10 @@ struct LaunchCfg {
 // (redundantly in every CTA, on identical data, so the CTAs agree without talking).  The
 // other warps are workers: they run the fused real-space + k-space pass of the current move
 // over the CTA's atoms and k-vector entries.  For unbiased moves the control warp prepares
-// the next move while the workers run the current pass: the next move starts either where the
-// current one ends after a hard-core overlap (no acceptance draw) or one draw later, and when
-// the next molecule is the one being moved its old positions depend on the decision, so lanes
-// 0-2 prepare the (at most) three candidates and the decision picks one.
+// the next move while the workers run the current pass: after the acceptance draw, and as the next
+// molecule's old positions depend on the decision when it is the one being moved, lanes 1 and 2
+// prepare two candidates and the decision picks one.  After a hard-core overlap (no acceptance draw)
+// the next move starts one number earlier: it is rare, and not prepared.
 
 // per-replica run control, in device memory
 struct RunSlot {
@@ -103,7 +103,6 @@ enum Phase { PH_CHOOSE = 0, PH_SPECULATE, PH_PROPOSE, PH_TABLES, PH_KSPACE, PH_F
 // flag and per-atom forces
 constexpr int RV_EW = 0, RV_LJ6 = 1, RV_LJ12 = 2, RV_DUC = 3, RV_DUL = 4, RV_OVL = 5, RV_F = 6;
 constexpr int kNV = 6 + 3 * kMaxA;
-constexpr int kNVP = kNV;
 
 enum PassKind { PASS_OLD = 0, PASS_NEW = 1, PASS_BOTH = 2 };
 
@@ -286,7 +285,7 @@ struct ChainShared {
     StageView view;
     Cand cand[4];         // the move being evaluated (cand[icur]) and up to three prepared next moves
     int icur;             // buffer of the move being evaluated
-    int spec[3];          // buffers of the candidates: after an overlap / after a draw / accepted same molecule
+    int spec[3];          // buffers of the candidates: after an overlap (never valid) / after a draw / accepted same molecule
     int abort, accepted, overlap, last_mol, spec_ok;
     int prop_out;         // the stream ran out in the proposal (a word of its own: see there)
     long long cursor;     // stream position after the last completed move
@@ -376,7 +375,7 @@ __host__ __device__ __forceinline__ typename Prec<MX>::R2 *scratch_buf(double2 *
 // Per-thread partial sums of a pass: FP64; in the mixed form FP64 for the pair terms (which
 // reach tens of kT) and FP32 with two-sum compensation (the running sum and its rounding
 // error, added in FP64 when the warp reduces) for the FP32 k-space terms.
-template <bool MX, int N = kNVP>
+template <bool MX, int N = kNV>
 struct Acc {
     double v[N];
     __device__ __forceinline__ void zero() {

@@ -75,7 +75,7 @@ __device__ inline void block_sum(double *vals, int nv, double *sh) {
 constexpr int kSumThreads = 1024;  // up to 16 values
 __global__ void __launch_bounds__(kSumThreads) k_sum_parts(const double *part, int nb, int nv, int vmax, double *out) {
     __shared__ double half[16];
-    const int v = threadIdx.x >> 6, t = threadIdx.x & 63, lane = threadIdx.x & 31;
+    const int v = threadIdx.x >> 6, t = threadIdx.x & 63;
     const bool flag = v == vmax;
     double x = 0;
     if (v < nv) {
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_parts(const double *part, i
 }
 
 // EwaldSumKSpace_calc_coulomb_energy / _calc_LJ_energy (EwaldSumKSpace.f90:389-526) per entry,
-// reduced per block (host adds the blocks in order).
+// reduced per block (k_sum_parts adds the blocks in order).
 template <int NT>
 __global__ void __launch_bounds__(256) k_kspace_energy(DevSys D, const double2 *rho, double *part) {
     __shared__ double red[(256 / 32 + 1) * 2];
@@ -2160,6 +2160,9 @@ struct yamc_rdf {
 // tiles' tests cost 20 us more than all M^2 pairs at 1024 centres; a frame from host centres at water's
 // density, all pairs against tiles: rmax 12 A 47 / 57 us at 1024, 58 / 66 at 2000, 98 / 73 at 3000,
 // 169 / 82 at 4252, 520 / 118 at 8000; rmax L/2 72 / 88 at 2400, 174 / 144 at 4252, 562 / 318 at 8000.
+// (For evenly spread centres the near tiles follow from rmax / L and the number of centres alone.  Where they
+// crowd the tiles gain later: a Gaussian blob of 0.1 L, rmax L/3, 101 / 134 at 2400, 132 / 149 at 3600, 173 / 177
+// at 4252, 320 / 300 at 6000.)
 constexpr int kRdfTileMin = 2400, kRdfTileMinFar = 3600;
 constexpr size_t kRdfTileStatic = 40 * 1024;  // k_rdf_tiles' own shared memory beside the histogram
 

@@ -619,7 +619,8 @@ static __global__ void __launch_bounds__(256) k_row_fields(DevSys D, const int4 
 // blockIdx.y splits the row pairs when the atoms alone do not fill the GPU.  rows: (kx, ky, first
 // field, number of kz).  kf[(y 3 + component) npos + position].
 // With one atom per lane the loads bind: 4 uniform 16-byte loads and one of the lane's table per 18 FP64
-// operations, 20 cycles of an SM against 9.  Two atoms share the uniform loads (24 against 18).
+// operations, 20 cycles of an SM against 9.  Two atoms share the uniform loads (24 against 18); the wait for
+// the fields' loads leads then (2.9 of 9 cycles per instruction; load pipe 65 %, FP64 pipe 57 %).
 // 49,752 atoms x 29,784 entries: 6.6 ms with the phase formed per atom and entry, 1.56 ms with one
 // atom per lane, 1.23 ms with two.
 constexpr int kForceRowWarps = 8;
@@ -731,7 +732,8 @@ static __global__ void k_forces_add(DevSys D, const int2 *place, const double *g
 // ------------------------------------------------------------------------------------------
 // Every ordered pair of centres of the tile and its near tiles, counted as k_rdf_count counts it
 // (the same explicitly rounded distance, so the same bins), for frames without periodic images
-// (rmax < L / 2).  16,984 centres, rmax 12 of 79.3 A: 2.1 ms over all pairs, 0.10 ms.
+// (rmax < L / 2).  16,984 centres, rmax 12 of 79.3 A: 2.1 ms over all pairs, 0.10 ms; the barriers around
+// each tile's near list bind (4.9 of 13 cycles per instruction; load pipe 50 %).
 static __global__ void __launch_bounds__(256) k_rdf_tiles(const double *cx, const double *cy, const double *cz, const int *type,
                                                           const int *order, const float4 *box, int ntile, double reach2, int M,
                                                           int ntypes, int nbin, double L, double dr, double rmax2,
